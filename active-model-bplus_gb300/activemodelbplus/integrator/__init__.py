@@ -176,7 +176,8 @@ class Integrator:
         seed: 64-bit key of the Philox noise; ``None`` draws one from the OS,
             like the reference's non-deterministic seed.
         device: CUDA device (default: current).
-        kernel: "auto", "tile" or "sliding" (FP32 kernel choice; FP64 always runs the tile kernel).
+        kernel: "auto", "tile" or "sliding" (FP32 kernel choice; FP64 runs the three-phase kernel, or
+            the tile kernel with kernel="tile" or where its workspace does not fit).
         autotune: with kernel="auto" and FP32 storage, time the candidate kernels and
             launch shapes for this grid once per process (``amb_autotune_f32``) and use
             the fastest; otherwise a shape heuristic decides. The FP32 kernels give
@@ -218,6 +219,13 @@ class Integrator:
         self._residual = (torch.zeros((self._ny, self._nx), dtype=torch.int16, device=self._device)
                           if precision == "f32c" else None)
         self._flag = torch.zeros(1, dtype=torch.int32, device=self._device)
+        self._workspace = None  # planes of the three-phase FP64 kernel
+        if precision == "f64" and kernel != "tile":
+            try:
+                self._workspace = torch.empty(lib.amb_step_workspace_bytes(N.AMB_F64, self._ny, self._nx),
+                                              dtype=torch.uint8, device=self._device)
+            except torch.cuda.OutOfMemoryError:
+                pass  # the tile kernel needs none
         self._timestep = 0
         self._terms_step = None
         self._terms_dev = None
@@ -318,7 +326,12 @@ class Integrator:
             cur, other = self._buf[self._cur], self._buf[1 - self._cur]
             if self._events is not None:
                 self._events[0].record()
-            if self._precision == "f64":
+            if self._workspace is not None:
+                rc = lib.amb_step_f64_ws(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
+                                         cur.data_ptr(), other.data_ptr(), self._timestep, nsteps, None,
+                                         self._workspace.data_ptr(), self._workspace.numel(), stream,
+                                         ctypes.byref(in_spare))
+            elif self._precision == "f64":
                 rc = lib.amb_step_f64_ex(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny,
                                          self._nx, cur.data_ptr(), other.data_ptr(), self._timestep, nsteps, None,
                                          ctypes.byref(self._launch_cfg) if self._launch_cfg is not None else None,

@@ -73,6 +73,8 @@ SIGNATURES = {
     "amb_step_f64": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _I64, _I, _VP, _VP, _IP]),
     "amb_step_f64_ex": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _I64, _I, _VP, ctypes.POINTER(amb_kernel_config),
                              _VP, _IP]),
+    "amb_step_workspace_bytes": (ctypes.c_size_t, [_I, _I, _I]),
+    "amb_step_f64_ws": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _I64, _I, _VP, _VP, ctypes.c_size_t, _VP, _IP]),
     "amb_step_f32": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _VP, _I64, _I, _VP, _I, _VP, _IP]),
     "amb_step_f32_ex": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _VP, _I64, _I, _VP, ctypes.POINTER(amb_kernel_config),
                              _VP, _IP]),

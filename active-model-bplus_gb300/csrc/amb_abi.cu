@@ -163,6 +163,34 @@ extern "C" int amb_step_f64(const amb_stencil* stencil, const amb_model* model, 
                            stream, result_in_spare);
 }
 
+extern "C" size_t amb_step_workspace_bytes(int precision, int nrows, int ncols)
+{
+    if (precision != AMB_F64 || nrows < 1 || ncols < 1 || nrows > kMaxDim || ncols > kMaxDim) return 0;
+    return amb::step_phase_workspace(nrows, ncols);
+}
+
+extern "C" int amb_step_f64_ws(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
+                               double* field, double* spare, int64_t step0, int nsteps, const double* injected_noise,
+                               void* workspace, size_t workspace_bytes, void* stream, int* result_in_spare)
+{
+    if (int rc = check_shape(nrows, ncols)) return rc;
+    if (int rc = check_params(stencil, model)) return rc;
+    if (!field || !spare || field == spare) return fail(AMB_ERR_INVALID, "field and spare must be distinct device buffers");
+    if (nsteps < 0) return fail(AMB_ERR_INVALID, "nsteps must be >= 0");
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15)
+        || workspace_bytes < amb_step_workspace_bytes(AMB_F64, nrows, ncols))
+        return fail(AMB_ERR_INVALID, "amb_step_f64_ws: workspace NULL, unaligned or smaller than amb_step_workspace_bytes");
+    if (nsteps == 0 || capturing(as_stream(stream)))
+        return amb_step_f64(stencil, model, seed, nrows, ncols, field, spare, step0, nsteps, injected_noise, stream,
+                            result_in_spare);
+    const amb::StepParams p = make_params(stencil, model, seed, nrows, ncols, step0);
+    cudaError_t e = amb::launch_steps_phase(field, spare, p, noise_mode_for(model, injected_noise), injected_noise,
+                                            nsteps, workspace, as_stream(stream));
+    if (e != cudaSuccess) return cuda_fail(e, "amb_step_f64_ws");
+    if (result_in_spare) *result_in_spare = nsteps & 1;
+    return AMB_OK;
+}
+
 namespace
 {
     bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
@@ -326,6 +354,8 @@ struct amb_integrator
     void* buf[2] = {nullptr, nullptr};  // field ping-pong
     int cur = 0;
     uint16_t* residual = nullptr;
+    void* workspace = nullptr;  // step workspace (FP64), allocated at the first run if there is room
+    bool workspace_tried = false;
     double* stage = nullptr;  // float64 staging plane for FP32 fields, allocated on first transfer
     double* terms = nullptr;  // AMB_NTERMS planes, allocated on first getter call
     int* flag = nullptr;
@@ -344,6 +374,7 @@ namespace
         cudaFree(h->buf[0]);
         cudaFree(h->buf[1]);
         cudaFree(h->residual);
+        cudaFree(h->workspace);
         cudaFree(h->stage);
         cudaFree(h->terms);
         cudaFree(h->flag);
@@ -450,7 +481,21 @@ extern "C" int amb_integrator_run(amb_integrator* h, int nsteps)
         int in_spare = 0;
         int rc;
         void* other = h->buf[1 - h->cur];
-        if (h->precision == AMB_F64)
+        const size_t ws_bytes = amb_step_workspace_bytes(h->precision, h->nrows, h->ncols);
+        if (ws_bytes && !h->workspace_tried)
+        {
+            h->workspace_tried = true;
+            if (cudaMalloc(&h->workspace, ws_bytes) != cudaSuccess)
+            {
+                h->workspace = nullptr;  // no room: the tile kernel needs none
+                cudaGetLastError();
+            }
+        }
+        if (h->precision == AMB_F64 && h->workspace)
+            rc = amb_step_f64_ws(&h->stencil, &h->model, h->seed, h->nrows, h->ncols,
+                                 static_cast<double*>(h->buf[h->cur]), static_cast<double*>(other), h->timestep, nsteps,
+                                 nullptr, h->workspace, ws_bytes, h->stream, &in_spare);
+        else if (h->precision == AMB_F64)
             rc = amb_step_f64(&h->stencil, &h->model, h->seed, h->nrows, h->ncols, static_cast<double*>(h->buf[h->cur]),
                               static_cast<double*>(other), h->timestep, nsteps, nullptr, h->stream, &in_spare);
         else

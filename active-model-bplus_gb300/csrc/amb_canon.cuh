@@ -103,6 +103,15 @@ namespace amb
         }
     };
 
+    // The rounded operations as a coefficient block K provides them. Canon's are the plain ones; a
+    // kernel may evaluate the same values in another instruction form (amb_step_phase.cuh).
+    template <typename Real>
+    __device__ __forceinline__ Real kadd(Real a, Real b, const Canon<Real>&) { return radd(a, b); }
+    template <typename Real>
+    __device__ __forceinline__ Real ksub(Real a, Real b, const Canon<Real>&) { return rsub(a, b); }
+    template <typename Real>
+    __device__ __forceinline__ Real kmul(Real a, Real b, const Canon<Real>&) { return rmul(a, b); }
+
     // Stage A at one site from its 3x3 box: rows u (above), m (centre), d (below), each at
     // columns -1, 0, +1 (pointers to the centre column).
     template <typename Real>
@@ -111,92 +120,98 @@ namespace amb
         Real f, mup, mua, jcy, jcx;
     };
 
-    template <typename Real>
-    __device__ __forceinline__ SiteA<Real> canon_stage_a(const Real* u, const Real* m, const Real* d,
-                                                         const Canon<Real>& k)
+    // From the centre column (u above, f, d below) and the sums A and differences D of the left and
+    // right columns of the three rows (a kernel that walks down rows forms each row's once).
+    template <typename Real, typename K>
+    __device__ __forceinline__ SiteA<Real> canon_site_a(Real u, Real f, Real d, Real Am, Real A0, Real Ap, Real Dm,
+                                                        Real D0, Real Dp, const K& k)
     {
-        const Real Am = radd(u[-1], u[1]), Dm = rsub(u[1], u[-1]);
-        const Real A0 = radd(m[-1], m[1]), D0 = rsub(m[1], m[-1]);
-        const Real Ap = radd(d[-1], d[1]), Dp = rsub(d[1], d[-1]);
-        const Real f = m[0];
-        Real l = rmul(k.lA, radd(Am, Ap));
-        l = rfma(k.lB, radd(u[0], d[0]), l);
+        Real l = kmul(k.lA, kadd(Am, Ap, k), k);
+        l = rfma(k.lB, kadd(u, d, k), l);
         l = rfma(k.lC, A0, l);
         const Real lap = rfma(k.lD, f, l);
-        const Real gx = rfma(k.gxb, D0, rmul(k.gxa, radd(Dm, Dp)));
-        const Real gy = rfma(k.gyb, rsub(d[0], u[0]), rmul(k.gya, rsub(Ap, Am)));
+        const Real gx = rfma(k.gxb, D0, kmul(k.gxa, kadd(Dm, Dp, k), k));
+        const Real gy = rfma(k.gyb, ksub(d, u, k), kmul(k.gya, ksub(Ap, Am, k), k));
         SiteA<Real> s;
         s.f = f;
-        s.mup = rfma(k.nkappa, lap, rmul(rfma(rfma(k.c, f, k.b), f, k.a), f));
-        s.mua = rmul(k.lambda, rfma(gy, gy, rmul(gx, gx)));
-        const Real zl = rmul(k.zeta, lap);
-        s.jcy = rmul(zl, gy);
-        s.jcx = rmul(zl, gx);
+        s.mup = rfma(k.nkappa, lap, kmul(rfma(rfma(k.c, f, k.b), f, k.a), f, k));
+        s.mua = kmul(k.lambda, rfma(gy, gy, kmul(gx, gx, k)), k);
+        const Real zl = kmul(k.zeta, lap, k);
+        s.jcy = kmul(zl, gy, k);
+        s.jcx = kmul(zl, gx, k);
         return s;
     }
 
-    // mu_p alone at one site (the same operations as canon_stage_a's mu_p).
-    template <typename Real>
-    __device__ __forceinline__ Real canon_mu_p(const Real* u, const Real* m, const Real* d, const Canon<Real>& k)
+    template <typename Real, typename K>
+    __device__ __forceinline__ SiteA<Real> canon_stage_a(const Real* u, const Real* m, const Real* d,
+                                                         const K& k)
     {
-        const Real Am = radd(u[-1], u[1]);
-        const Real A0 = radd(m[-1], m[1]);
-        const Real Ap = radd(d[-1], d[1]);
+        return canon_site_a(u[0], m[0], d[0], kadd(u[-1], u[1], k), kadd(m[-1], m[1], k), kadd(d[-1], d[1], k),
+                            ksub(u[1], u[-1], k), ksub(m[1], m[-1], k), ksub(d[1], d[-1], k), k);
+    }
+
+    // mu_p alone at one site (the same operations as canon_stage_a's mu_p).
+    template <typename Real, typename K>
+    __device__ __forceinline__ Real canon_mu_p(const Real* u, const Real* m, const Real* d, const K& k)
+    {
+        const Real Am = kadd(u[-1], u[1], k);
+        const Real A0 = kadd(m[-1], m[1], k);
+        const Real Ap = kadd(d[-1], d[1], k);
         const Real f = m[0];
-        Real l = rmul(k.lA, radd(Am, Ap));
-        l = rfma(k.lB, radd(u[0], d[0]), l);
+        Real l = kmul(k.lA, kadd(Am, Ap, k), k);
+        l = rfma(k.lB, kadd(u[0], d[0], k), l);
         l = rfma(k.lC, A0, l);
         const Real lap = rfma(k.lD, f, l);
-        return rfma(k.nkappa, lap, rmul(rfma(rfma(k.c, f, k.b), f, k.a), f));
+        return rfma(k.nkappa, lap, kmul(rfma(rfma(k.c, f, k.b), f, k.a), f, k));
     }
 
     // sum_j c_j (g[+j] - g[-j]), j = 1..4, in that order (first a product, then fused).
-    template <typename Real>
+    template <typename Real, typename K>
     __device__ __forceinline__ Real canon_d8(const Real (&c)[4], Real m1, Real p1, Real m2, Real p2, Real m3, Real p3,
-                                             Real m4, Real p4)
+                                             Real m4, Real p4, const K& k)
     {
-        Real s = rmul(c[0], rsub(p1, m1));
-        s = rfma(c[1], rsub(p2, m2), s);
-        s = rfma(c[2], rsub(p3, m3), s);
-        return rfma(c[3], rsub(p4, m4), s);
+        Real s = kmul(c[0], ksub(p1, m1, k), k);
+        s = rfma(c[1], ksub(p2, m2, k), s);
+        s = rfma(c[2], ksub(p3, m3, k), s);
+        return rfma(c[3], ksub(p4, m4, k), s);
     }
 
     // 0.1 (left + right) + 0.3 centre (fused).
-    template <typename Real>
-    __device__ __forceinline__ Real canon_smooth(Real l, Real c, Real r, const Canon<Real>& k)
+    template <typename Real, typename K>
+    __device__ __forceinline__ Real canon_smooth(Real l, Real c, Real r, const K& k)
     {
-        return rfma(k.p1, radd(l, r), rmul(k.p3, c));
+        return rfma(k.p1, kadd(l, r, k), kmul(k.p3, c, k));
     }
 
     // J2_y and J2_x at row r from the x-smoothed (sx) and x-differenced (dx) mu_a rows r-1, r, r+1.
-    template <typename Real>
-    __device__ __forceinline__ Real canon_j2y(Real sx_m, Real sx_p, Real jcy, const Canon<Real>& k)
+    template <typename Real, typename K>
+    __device__ __forceinline__ Real canon_j2y(Real sx_m, Real sx_p, Real jcy, const K& k)
     {
-        return rfma(k.ndy, rsub(sx_p, sx_m), jcy);
+        return rfma(k.ndy, ksub(sx_p, sx_m, k), jcy);
     }
 
-    template <typename Real>
-    __device__ __forceinline__ Real canon_j2x(Real dx_m, Real dx_0, Real dx_p, Real jcx, const Canon<Real>& k)
+    template <typename Real, typename K>
+    __device__ __forceinline__ Real canon_j2x(Real dx_m, Real dx_0, Real dx_p, Real jcx, const K& k)
     {
-        return rfma(k.jx3, dx_0, rfma(k.jx1, radd(dx_p, dx_m), jcx));
+        return rfma(k.jx3, dx_0, rfma(k.jx1, kadd(dx_p, dx_m, k), jcx));
     }
 
     // Tjhung divergence of J2 at row r from sxj (x-smoothed J2_y) and dxj (x-differenced J2_x)
     // of rows r-1, r, r+1.
-    template <typename Real>
+    template <typename Real, typename K>
     __device__ __forceinline__ Real canon_divtj(Real sxj_m, Real sxj_p, Real dxj_m, Real dxj_0, Real dxj_p,
-                                                const Canon<Real>& k)
+                                                const K& k)
     {
-        Real v = rmul(k.tx1, radd(dxj_m, dxj_p));
+        Real v = kmul(k.tx1, kadd(dxj_m, dxj_p, k), k);
         v = rfma(k.tx3, dxj_0, v);
-        return rfma(k.dyInv, rsub(sxj_p, sxj_m), v);
+        return rfma(k.dyInv, ksub(sxj_p, sxj_m, k), v);
     }
 
     // The update of one site: plain, or compensated with residual r (in/out).
-    template <typename Real>
-    __device__ __forceinline__ Real canon_update(Real f, Real dx8, Real divtj, Real dy8, const Canon<Real>& k)
+    template <typename Real, typename K>
+    __device__ __forceinline__ Real canon_update(Real f, Real dx8, Real divtj, Real dy8, const K& k)
     {
-        const Real div = radd(dx8, radd(divtj, dy8));
+        const Real div = kadd(dx8, kadd(divtj, dy8, k), k);
         return rfma(k.ndt, div, f);
     }
 

@@ -24,6 +24,12 @@ namespace amb
                                              const StepParams& p, int noise_mode, const Real* injected, int nsteps,
                                              int groups, bool rows28, cudaStream_t stream);
 
+    // FP64 steps in three grid-wide phases, all steps of a call in one cooperative launch (or several,
+    // for long calls); the planes between the phases live in `workspace` (amb_step_phase.cuh).
+    size_t step_phase_workspace(int ny, int nx);
+    cudaError_t launch_steps_phase(double* a, double* b, const StepParams& p, int noise_mode, const double* injected,
+                                   int nsteps, void* workspace, cudaStream_t stream);
+
     // Register-sliding FP32 kernel (amb_step_f32.cu). Returns cudaErrorNotSupported
     // when the grid shape is outside its fast-path constraints.
     cudaError_t launch_step_f32_sliding(const float* phi_in, float* phi_out, __nv_bfloat16* comp, int comp_mode,

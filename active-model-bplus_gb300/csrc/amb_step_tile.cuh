@@ -148,11 +148,11 @@ namespace amb
             const Real* c = MUP + (i + 8) * G::MX + (j + 8);
             constexpr int L = G::MX;
             return rfma(k.mag, xi, canon_d8(k.ny8, c[-L], c[L], c[-2 * L], c[2 * L], c[-3 * L], c[3 * L], c[-4 * L],
-                                            c[4 * L]));
+                                            c[4 * L], k));
         };
         const auto j1x_at = [&](int i, int j, Real xi) {  // row i in [0, TY), column j in [-4, TX+4)
             const Real* c = MUP + (i + 8) * G::MX + (j + 8);
-            return rfma(k.mag, xi, canon_d8(k.nx8, c[-1], c[1], c[-2], c[2], c[-3], c[3], c[-4], c[4]));
+            return rfma(k.mag, xi, canon_d8(k.nx8, c[-1], c[1], c[-2], c[2], c[-3], c[3], c[-4], c[4], k));
         };
         if (noise_mode == NOISE_PHILOX && nx % 4 == 0)
         {
@@ -222,9 +222,9 @@ namespace amb
                                            rsub(x0[1], x0[-1]), rsub(x1[1], x1[-1]), rsub(x2[1], x2[-1]), k);
             const Real* cy = J1Y + (i + 4) * TX + j;
             const Real dy8 = canon_d8(k.py8, cy[-TX], cy[TX], cy[-2 * TX], cy[2 * TX], cy[-3 * TX], cy[3 * TX],
-                                      cy[-4 * TX], cy[4 * TX]);
+                                      cy[-4 * TX], cy[4 * TX], k);
             const Real* cx = J1X + i * G::QX + j + 4;
-            const Real dx8 = canon_d8(k.px8, cx[-1], cx[1], cx[-2], cx[2], cx[-3], cx[3], cx[-4], cx[4]);
+            const Real dx8 = canon_d8(k.px8, cx[-1], cx[1], cx[-2], cx[2], cx[-3], cx[3], cx[-4], cx[4], k);
             const Real f = PHI[(i + G::H) * G::LX + (j + G::H)];
             const size_t gi = (size_t)gr * nx + gc;
             if constexpr (COMP == COMP_BF16)

@@ -166,6 +166,16 @@ int amb_step_f64(const amb_stencil* stencil, const amb_model* model, uint64_t se
 int amb_step_f64_ex(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
                     double* field, double* spare, int64_t step0, int nsteps, const double* injected_noise,
                     const amb_kernel_config* config, void* stream, int* result_in_spare);
+/* amb_step_f64 with a workspace for the planes of the three-phase kernel, the fastest FP64 form
+ * (every step of the call in one cooperative launch, no FP64 operation recomputed in halos):
+ * amb_step_workspace_bytes(AMB_F64, nrows, ncols) bytes of device memory, 16-byte aligned, whose
+ * content need not be kept between calls but which calls that may overlap must not share. At most
+ * 256 MiB (more only for rows of over 87000 columns). The results are bitwise those of
+ * amb_step_f64. While the stream is being captured the call runs as amb_step_f64. */
+size_t amb_step_workspace_bytes(int precision, int nrows, int ncols);
+int amb_step_f64_ws(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
+                    double* field, double* spare, int64_t step0, int nsteps, const double* injected_noise,
+                    void* workspace, size_t workspace_bytes, void* stream, int* result_in_spare);
 /* FP32 storage. residual: NULL for plain FP32 (AMB_F32), else a device plane of
  * nrows*ncols bf16 words updated in place (AMB_F32C; zero it before the first step).
  * kernel: AMB_KERNEL_*. */
