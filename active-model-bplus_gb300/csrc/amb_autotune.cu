@@ -4,8 +4,8 @@
 // Candidates: the tile kernel with 256, 512 or 1024 threads per CTA, 32 x 32 or 28 x 32 output
 // tiles, launched once per step or once for all steps (persistent, grid barrier between steps),
 // and the warp-pair sliding
-// kernel with 1, 2 or 4 pairs per CTA (or, fused, 1, 2 or 4 single warps per CTA) and row-segment
-// heights from 2 rows up to the whole grid (plus the occupancy model's own choice). All candidates
+// kernel with 1, 2 or 4 pairs per CTA (or, fused, one single warp per CTA) and the row-segment
+// heights that put a whole number of tasks on each SM (plus the occupancy model's own choice). All candidates
 // give bitwise the same field. Each is timed with CUDA events over a few steps on
 // scratch buffers of the same shape; the fastest few are timed again and the best
 // is kept in a process-wide cache keyed by (device, nrows, ncols, compensated,
@@ -106,13 +106,27 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
         for (int flags : {0, AMB_FLAG_PERSISTENT, AMB_FLAG_TILE_ROWS_28, AMB_FLAG_PERSISTENT | AMB_FLAG_TILE_ROWS_28})
             cands.push_back({AMB_KERNEL_TILE, 0, groups, flags});
     if (ncols >= 112 && ncols % 4 == 0)
-        for (int pairs : {1, 2, 4})
-            for (int flags : {0, AMB_FLAG_FUSED})
-            {
-                cands.push_back({AMB_KERNEL_SLIDING, 0, pairs, flags});
-                for (int seg = 2; seg < 2 * nrows && seg <= 4096; seg *= 2)
-                    cands.push_back({AMB_KERNEL_SLIDING, std::min(seg, nrows), pairs, flags});
-            }
+    {
+        // Segment heights that put m tasks on each SM: a task costs its rows plus about eight rows of
+        // pipeline fill, so the best height is one whose task count just fills the SMs, with as many
+        // resident tasks as pay for their fill (1536^2: 24 rows, 30.8 us; 16 and 32 rows 37).
+        int sms = 152, dev = key_device();
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int strips = (ncols + 111) / 112;
+        const auto rows_for = [&](int m) {
+            const int segs = std::max(1, std::min(nrows, sms * m / strips));
+            return (nrows + segs - 1) / segs;
+        };
+        const auto add = [&](std::initializer_list<int> ms, int pairs, int flags) {
+            std::vector<int> rows{0};
+            for (int m : ms) rows.push_back(rows_for(m));
+            std::sort(rows.begin(), rows.end());
+            rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
+            for (int h : rows) cands.push_back({AMB_KERNEL_SLIDING, h, pairs, flags});
+        };
+        for (int pairs : {1, 2, 4}) add({2, 3, 4, 5, 6, 7, 8, 16}, pairs, 0);
+        add({6, 8, 10, 12}, 1, AMB_FLAG_FUSED);
+    }
 
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);

@@ -1,0 +1,57 @@
+// Four adjacent columns of one row as two packed FP32 pairs, and the canonical operations on them
+// (amb_canon.cuh): a packed instruction rounds each half as the scalar one, so the bits are the same
+// in half the issue slots.
+#pragma once
+
+#include "amb_canon.cuh"
+
+namespace amb
+{
+    struct Quad
+    {
+        float2 a, b;
+    };
+
+    __device__ __forceinline__ float2 sub2(float2 x, float2 y) { return __fadd2_rn(x, make_float2(-y.x, -y.y)); }
+    __device__ __forceinline__ Quad operator+(Quad x, Quad y) { return {__fadd2_rn(x.a, y.a), __fadd2_rn(x.b, y.b)}; }
+    __device__ __forceinline__ Quad operator-(Quad x, Quad y) { return {sub2(x.a, y.a), sub2(x.b, y.b)}; }
+    __device__ __forceinline__ Quad operator*(Quad x, Quad y) { return {__fmul2_rn(x.a, y.a), __fmul2_rn(x.b, y.b)}; }
+    __device__ __forceinline__ Quad operator*(float2 c, Quad x) { return {__fmul2_rn(c, x.a), __fmul2_rn(c, x.b)}; }
+    __device__ __forceinline__ Quad fma4(float2 c, Quad x, Quad y) { return {__ffma2_rn(c, x.a, y.a), __ffma2_rn(c, x.b, y.b)}; }
+    __device__ __forceinline__ Quad fma4(float2 c, Quad x, float2 y) { return {__ffma2_rn(c, x.a, y), __ffma2_rn(c, x.b, y)}; }
+    __device__ __forceinline__ Quad fma4(Quad x, Quad y, Quad z) { return {__ffma2_rn(x.a, y.a, z.a), __ffma2_rn(x.b, y.b, z.b)}; }
+    __device__ __forceinline__ Quad fma4(Quad x, Quad y, float2 z) { return {__ffma2_rn(x.a, y.a, z), __ffma2_rn(x.b, y.b, z)}; }
+    __device__ __forceinline__ Quad quad(float4 v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+    __device__ __forceinline__ float4 vec(Quad v) { return make_float4(v.a.x, v.a.y, v.b.x, v.b.y); }
+    __device__ __forceinline__ Quad zero_quad() { return {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+    __device__ __forceinline__ Quad load_quad(const float* p) { return quad(*reinterpret_cast<const float4*>(p)); }
+    __device__ __forceinline__ void store_quad(float* p, Quad v) { *reinterpret_cast<float4*>(p) = vec(v); }
+
+    // left + right and right - left neighbours of four columns, l to their left and r to their right
+    __device__ __forceinline__ Quad nsum(float l, Quad v, float r)
+    {
+        return {make_float2(__fadd_rn(l, v.a.y), __fadd_rn(v.a.x, v.b.x)),
+                make_float2(__fadd_rn(v.a.y, v.b.y), __fadd_rn(v.b.x, r))};
+    }
+    __device__ __forceinline__ Quad ndiff(float l, Quad v, float r)
+    {
+        return {make_float2(__fsub_rn(v.a.y, l), __fsub_rn(v.b.x, v.a.x)),
+                make_float2(__fsub_rn(v.b.y, v.a.y), __fsub_rn(r, v.b.x))};
+    }
+
+    // sum_j c_j (g[+j] - g[-j]) along x at the columns of c, from the quads l and r beside it: the even
+    // offsets are aligned pairs, the odd ones are formed as scalars
+    __device__ __forceinline__ Quad d8x(const float2 (&k)[4], Quad l, Quad c, Quad r)
+    {
+        const Quad d1{make_float2(__fsub_rn(c.a.y, l.b.y), __fsub_rn(c.b.x, c.a.x)),
+                      make_float2(__fsub_rn(c.b.y, c.a.y), __fsub_rn(r.a.x, c.b.x))};
+        const Quad d2{sub2(c.b, l.b), sub2(r.a, c.a)};
+        const Quad d3{make_float2(__fsub_rn(c.b.y, l.a.y), __fsub_rn(r.a.x, l.b.x)),
+                      make_float2(__fsub_rn(r.a.y, l.b.y), __fsub_rn(r.b.x, c.a.x))};
+        const Quad d4{sub2(r.a, l.a), sub2(r.b, l.b)};
+        Quad s = k[0] * d1;
+        s = fma4(k[1], d2, s);
+        s = fma4(k[2], d3, s);
+        return fma4(k[3], d4, s);
+    }
+}
