@@ -187,7 +187,8 @@ class Integrator:
             "pairs_per_cta": p, "fused": bool (one warp per strip runs every stage; p then counts
             warps)}; for kernel="tile" {"pairs_per_cta": g (256-thread groups per CTA),
             "persistent": bool (all steps of a run() in one launch), "tile_rows": 32 or 28
-            (output tile height)}; e.g. a configuration the autotuner reported.
+            (output tile height), and for FP32 storage "seg_rows": 1 to 64 (output tile height, 0:
+            tile_rows) and "tile_cols": 32 or 64}; e.g. a configuration the autotuner reported.
     """
 
     def __init__(self, field, stencil, model, *, precision: str = "f64", seed: int | None = None,
@@ -219,10 +220,10 @@ class Integrator:
         self._residual = (torch.zeros((self._ny, self._nx), dtype=torch.int16, device=self._device)
                           if precision == "f32c" else None)
         self._flag = torch.zeros(1, dtype=torch.int32, device=self._device)
-        self._workspace = None  # planes of the three-phase FP64 kernel
-        if precision == "f64" and kernel != "tile":
+        self._workspace = None  # planes of the three-phase FP64 kernel; FP32: the grid barrier's counter
+        if precision != "f64" or kernel != "tile":
             try:
-                self._workspace = torch.empty(lib.amb_step_workspace_bytes(N.AMB_F64, self._ny, self._nx),
+                self._workspace = torch.empty(lib.amb_step_workspace_bytes(_PRECISIONS[precision], self._ny, self._nx),
                                               dtype=torch.uint8, device=self._device)
             except torch.cuda.OutOfMemoryError:
                 pass  # the tile kernel needs none
@@ -242,7 +243,8 @@ class Integrator:
                 raise ValueError("tile_rows must be 32 or 28")
             flags = ((N.AMB_FLAG_PERSISTENT if launch.get("persistent", False) else 0)
                      | (N.AMB_FLAG_FUSED if launch.get("fused", False) else 0)
-                     | (N.AMB_FLAG_TILE_ROWS_28 if int(launch.get("tile_rows", 32)) == 28 else 0))
+                     | (N.AMB_FLAG_TILE_ROWS_28 if int(launch.get("tile_rows", 32)) == 28 else 0)
+                     | (N.AMB_FLAG_TILE_COLS_64 if int(launch.get("tile_cols", 32)) == 64 else 0))
             self._launch_cfg = N.amb_kernel_config(_KERNELS[kernel], int(launch.get("seg_rows", 0)),
                                                    int(launch.get("pairs_per_cta", 0)), flags)
         self._tuned = None
@@ -256,7 +258,8 @@ class Integrator:
                            "pairs_per_cta": cfg.pairs_per_cta,
                            "persistent": bool(cfg.flags & N.AMB_FLAG_PERSISTENT),
                            "fused": bool(cfg.flags & N.AMB_FLAG_FUSED),
-                           "tile_rows": 28 if cfg.flags & N.AMB_FLAG_TILE_ROWS_28 else 32, "us_per_step": us.value}
+                           "tile_rows": 28 if cfg.flags & N.AMB_FLAG_TILE_ROWS_28 else 32,
+                           "tile_cols": 64 if cfg.flags & N.AMB_FLAG_TILE_COLS_64 else 32, "us_per_step": us.value}
         del lib
 
     # -------------------------------------------------------------- plumbing
@@ -326,7 +329,7 @@ class Integrator:
             cur, other = self._buf[self._cur], self._buf[1 - self._cur]
             if self._events is not None:
                 self._events[0].record()
-            if self._workspace is not None:
+            if self._precision == "f64" and self._workspace is not None:
                 rc = lib.amb_step_f64_ws(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
                                          cur.data_ptr(), other.data_ptr(), self._timestep, nsteps, None,
                                          self._workspace.data_ptr(), self._workspace.numel(), stream,
@@ -338,14 +341,16 @@ class Integrator:
                                          stream, ctypes.byref(in_spare))
             else:
                 res = self._residual.data_ptr() if self._residual is not None else None
-                if self._launch_cfg is not None:
-                    rc = lib.amb_step_f32_ex(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny,
-                                             self._nx, cur.data_ptr(), other.data_ptr(), res, self._timestep, nsteps,
-                                             None, ctypes.byref(self._launch_cfg), stream, ctypes.byref(in_spare))
+                cfg = self._launch_cfg
+                if cfg is None:
+                    cfg = N.amb_kernel_config(_KERNELS[self._kernel], 0, 0, 0)
+                args = (ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx, cur.data_ptr(),
+                        other.data_ptr(), res, self._timestep, nsteps, None, ctypes.byref(cfg))
+                if self._workspace is not None:
+                    rc = lib.amb_step_f32_ws(*args, self._workspace.data_ptr(), self._workspace.numel(), stream,
+                                             ctypes.byref(in_spare))
                 else:
-                    rc = lib.amb_step_f32(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny,
-                                          self._nx, cur.data_ptr(), other.data_ptr(), res, self._timestep, nsteps,
-                                          None, _KERNELS[self._kernel], stream, ctypes.byref(in_spare))
+                    rc = lib.amb_step_f32_ex(*args, stream, ctypes.byref(in_spare))
             if self._events is not None:
                 self._events[1].record()
             _check(rc)

@@ -43,6 +43,7 @@ class amb_kernel_config(ctypes.Structure):
 AMB_FLAG_PERSISTENT = 1
 AMB_FLAG_FUSED = 2
 AMB_FLAG_TILE_ROWS_28 = 4
+AMB_FLAG_TILE_COLS_64 = 8
 
 
 _VP = ctypes.c_void_p
@@ -78,6 +79,8 @@ SIGNATURES = {
     "amb_step_f32": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _VP, _I64, _I, _VP, _I, _VP, _IP]),
     "amb_step_f32_ex": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _VP, _I64, _I, _VP, ctypes.POINTER(amb_kernel_config),
                              _VP, _IP]),
+    "amb_step_f32_ws": (_I, [_SP, _MP, _U64, _I, _I, _VP, _VP, _VP, _I64, _I, _VP, ctypes.POINTER(amb_kernel_config),
+                             _VP, ctypes.c_size_t, _VP, _IP]),
     "amb_autotune_f32": (_I, [_SP, _MP, _I, _I, _I, _I, _VP, ctypes.POINTER(amb_kernel_config),
                               ctypes.POINTER(ctypes.c_double)]),
     "amb_terms_f64": (_I, [_SP, _MP, _U64, _I, _I, _VP, _I64, _VP, _VP, _VP]),

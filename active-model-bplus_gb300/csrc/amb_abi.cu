@@ -92,39 +92,68 @@ namespace
         return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
     }
 
-    // Steps of the tile kernel: one launch per step, or all of them in one persistent launch.
-    template <typename Real>
+    // Steps of the FP64 tile kernel: one launch per step, or all of them in one persistent launch.
     int tile_steps(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
-                   Real* field, Real* spare, __nv_bfloat16* res, int comp, int64_t step0, int nsteps,
-                   const Real* injected_noise, const amb_kernel_config& cfg, cudaStream_t stream,
+                   double* field, double* spare, int64_t step0, int nsteps,
+                   const double* injected_noise, const amb_kernel_config& cfg, cudaStream_t stream,
                    int* result_in_spare, const char* name)
     {
         const size_t n = size_t(nrows) * ncols;
         const int mode = noise_mode_for(model, injected_noise);
-        // default CTA width: 512 threads (measured fastest for FP64 at 1024^2-4096^2 and for FP32
-        // small grids; the FP32 autotuner names its own)
+        // default CTA width: 512 threads (measured fastest at 1024^2-4096^2)
         const int groups = cfg.pairs_per_cta == 0 ? 2 : cfg.pairs_per_cta;
         const bool rows28 = (cfg.flags & AMB_FLAG_TILE_ROWS_28) != 0;
         if ((cfg.flags & AMB_FLAG_PERSISTENT) && nsteps > 1 && !capturing(stream))
         {
             amb::StepParams p = make_params(stencil, model, seed, nrows, ncols, step0);
-            cudaError_t e = amb::launch_steps_tile_persistent<Real>(field, spare, res, comp, p, mode, injected_noise,
+            cudaError_t e = amb::launch_steps_tile_persistent(field, spare, p, mode, injected_noise,
                                                                     nsteps, groups, rows28, stream);
             if (e != cudaSuccess) return cuda_fail(e, name);
             if (result_in_spare) *result_in_spare = nsteps & 1;
             return AMB_OK;
         }
-        Real* cur = field;
-        Real* nxt = spare;
+        double* cur = field;
+        double* nxt = spare;
         for (int s = 0; s < nsteps; ++s)
         {
             amb::StepParams p = make_params(stencil, model, seed, nrows, ncols, step0 + s);
-            const Real* inj = injected_noise ? injected_noise + size_t(s) * 2 * n : nullptr;
-            cudaError_t e = amb::launch_step_tile<Real>(cur, nxt, res, comp, p, mode, inj, groups, rows28, stream);
+            const double* inj = injected_noise ? injected_noise + size_t(s) * 2 * n : nullptr;
+            cudaError_t e = amb::launch_step_tile(cur, nxt, p, mode, inj, groups, rows28, stream);
             if (e != cudaSuccess) return cuda_fail(e, name);
             std::swap(cur, nxt);
         }
         if (result_in_spare) *result_in_spare = (cur == spare) ? 1 : 0;
+        return AMB_OK;
+    }
+
+    // Steps of the FP32 quad tile kernel. Without a workspace the persistent form's barrier counter comes
+    // from the stream-ordered allocator.
+    int quad_steps(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols, float* field,
+                   float* spare, __nv_bfloat16* res, int64_t step0, int nsteps, const float* injected_noise,
+                   const amb_kernel_config& cfg, void* workspace, cudaStream_t stream, int* result_in_spare)
+    {
+        const amb::StepParams p = make_params(stencil, model, seed, nrows, ncols, step0);
+        const int mode = noise_mode_for(model, injected_noise);
+        const amb::QuadTile tile{cfg.seg_rows > 0 ? cfg.seg_rows : (cfg.flags & AMB_FLAG_TILE_ROWS_28) ? 28 : 32,
+                                 cfg.pairs_per_cta == 1 ? 256 : 512, (cfg.flags & AMB_FLAG_TILE_COLS_64) != 0};
+        void* count = nullptr;
+        cudaError_t e = cudaSuccess;
+        const bool persistent = (cfg.flags & AMB_FLAG_PERSISTENT) && nsteps > 1 && !capturing(stream);
+        if (persistent)
+        {
+            count = workspace;
+            if (!count) e = cudaMallocAsync(&count, sizeof(unsigned), stream);
+        }
+        if (e == cudaSuccess)
+            e = amb::launch_step_quad(field, spare, res, p, mode, injected_noise, nsteps, tile,
+                                      static_cast<unsigned*>(count), stream);
+        if (count && !workspace)
+        {
+            const cudaError_t ef = cudaFreeAsync(count, stream);
+            if (e == cudaSuccess) e = ef;
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "amb_step_f32");
+        if (result_in_spare) *result_in_spare = nsteps & 1;
         return AMB_OK;
     }
 
@@ -133,7 +162,7 @@ namespace
         if (cfg.kernel < AMB_KERNEL_AUTO || cfg.kernel > max_kernel) return fail(AMB_ERR_INVALID, "unknown kernel selector");
         if (cfg.seg_rows < 0 || cfg.pairs_per_cta < 0 || cfg.pairs_per_cta > 4 || cfg.pairs_per_cta == 3)
             return fail(AMB_ERR_INVALID, "kernel config: seg_rows >= 0, pairs_per_cta in {0, 1, 2, 4}");
-        if (cfg.flags & ~(AMB_FLAG_PERSISTENT | AMB_FLAG_FUSED | AMB_FLAG_TILE_ROWS_28))
+        if (cfg.flags & ~(AMB_FLAG_PERSISTENT | AMB_FLAG_FUSED | AMB_FLAG_TILE_ROWS_28 | AMB_FLAG_TILE_COLS_64))
             return fail(AMB_ERR_INVALID, "kernel config: unknown flags");
         return AMB_OK;
     }
@@ -151,8 +180,7 @@ extern "C" int amb_step_f64_ex(const amb_stencil* stencil, const amb_model* mode
     amb_kernel_config cfg{AMB_KERNEL_AUTO, 0, 0, 0};
     if (config) cfg = *config;
     if (int rc = check_config(cfg, AMB_KERNEL_TILE)) return rc;
-    return tile_steps<double>(stencil, model, seed, nrows, ncols, field, spare, nullptr, amb::COMP_NONE, step0, nsteps,
-                              injected_noise, cfg, as_stream(stream), result_in_spare, "amb_step_f64");
+    return tile_steps(stencil, model, seed, nrows, ncols, field, spare, step0, nsteps, injected_noise, cfg, as_stream(stream), result_in_spare, "amb_step_f64");
 }
 
 extern "C" int amb_step_f64(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
@@ -165,8 +193,9 @@ extern "C" int amb_step_f64(const amb_stencil* stencil, const amb_model* model, 
 
 extern "C" size_t amb_step_workspace_bytes(int precision, int nrows, int ncols)
 {
-    if (precision != AMB_F64 || nrows < 1 || ncols < 1 || nrows > kMaxDim || ncols > kMaxDim) return 0;
-    return amb::step_phase_workspace(nrows, ncols);
+    if (nrows < 1 || ncols < 1 || nrows > kMaxDim || ncols > kMaxDim) return 0;
+    if (precision == AMB_F32 || precision == AMB_F32C) return 256;  // the persistent tile kernel's barrier counter
+    return precision == AMB_F64 ? amb::step_phase_workspace(nrows, ncols) : 0;
 }
 
 extern "C" int amb_step_f64_ws(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
@@ -196,10 +225,9 @@ namespace
     bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 }
 
-extern "C" int amb_step_f32_ex(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows,
-                               int ncols, float* field, float* spare, uint16_t* residual, int64_t step0, int nsteps,
-                               const float* injected_noise, const amb_kernel_config* config, void* stream,
-                               int* result_in_spare)
+static int step_f32(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols, float* field,
+                    float* spare, uint16_t* residual, int64_t step0, int nsteps, const float* injected_noise,
+                    const amb_kernel_config* config, void* workspace, void* stream, int* result_in_spare)
 {
     if (int rc = check_shape(nrows, ncols)) return rc;
     if (int rc = check_params(stencil, model)) return rc;
@@ -233,8 +261,8 @@ extern "C" int amb_step_f32_ex(const amb_stencil* stencil, const amb_model* mode
     else if (cfg.kernel == AMB_KERNEL_AUTO)
         sliding = fits;
     if (!sliding)
-        return tile_steps<float>(stencil, model, seed, nrows, ncols, field, spare, res, comp, step0, nsteps,
-                                 injected_noise, cfg, as_stream(stream), result_in_spare, "amb_step_f32");
+        return quad_steps(stencil, model, seed, nrows, ncols, field, spare, res, step0, nsteps, injected_noise, cfg,
+                          workspace, as_stream(stream), result_in_spare);
     const int pairs_code = cfg.pairs_per_cta == 1 ? 1 : cfg.pairs_per_cta == 4 ? 3 : cfg.pairs_per_cta == 2 ? 2 : 0;
     const int variant = (cfg.seg_rows << 4) | ((cfg.flags & AMB_FLAG_FUSED) ? 8 : 0) | pairs_code;
     float* cur = field;
@@ -249,6 +277,27 @@ extern "C" int amb_step_f32_ex(const amb_stencil* stencil, const amb_model* mode
     }
     if (result_in_spare) *result_in_spare = (cur == spare) ? 1 : 0;
     return AMB_OK;
+}
+
+extern "C" int amb_step_f32_ex(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows,
+                               int ncols, float* field, float* spare, uint16_t* residual, int64_t step0, int nsteps,
+                               const float* injected_noise, const amb_kernel_config* config, void* stream,
+                               int* result_in_spare)
+{
+    return step_f32(stencil, model, seed, nrows, ncols, field, spare, residual, step0, nsteps, injected_noise, config,
+                    nullptr, stream, result_in_spare);
+}
+
+extern "C" int amb_step_f32_ws(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows,
+                               int ncols, float* field, float* spare, uint16_t* residual, int64_t step0, int nsteps,
+                               const float* injected_noise, const amb_kernel_config* config, void* workspace,
+                               size_t workspace_bytes, void* stream, int* result_in_spare)
+{
+    if (int rc = check_shape(nrows, ncols)) return rc;
+    if (!workspace || !aligned(workspace, 16) || workspace_bytes < amb_step_workspace_bytes(AMB_F32, nrows, ncols))
+        return fail(AMB_ERR_INVALID, "amb_step_f32_ws: workspace NULL, unaligned or smaller than amb_step_workspace_bytes");
+    return step_f32(stencil, model, seed, nrows, ncols, field, spare, residual, step0, nsteps, injected_noise, config,
+                    workspace, stream, result_in_spare);
 }
 
 extern "C" int amb_step_f32(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
@@ -354,7 +403,7 @@ struct amb_integrator
     void* buf[2] = {nullptr, nullptr};  // field ping-pong
     int cur = 0;
     uint16_t* residual = nullptr;
-    void* workspace = nullptr;  // step workspace (FP64), allocated at the first run if there is room
+    void* workspace = nullptr;  // step workspace, allocated at the first run if there is room
     bool workspace_tried = false;
     double* stage = nullptr;  // float64 staging plane for FP32 fields, allocated on first transfer
     double* terms = nullptr;  // AMB_NTERMS planes, allocated on first getter call
@@ -498,6 +547,10 @@ extern "C" int amb_integrator_run(amb_integrator* h, int nsteps)
         else if (h->precision == AMB_F64)
             rc = amb_step_f64(&h->stencil, &h->model, h->seed, h->nrows, h->ncols, static_cast<double*>(h->buf[h->cur]),
                               static_cast<double*>(other), h->timestep, nsteps, nullptr, h->stream, &in_spare);
+        else if (h->workspace)
+            rc = amb_step_f32_ws(&h->stencil, &h->model, h->seed, h->nrows, h->ncols,
+                                 static_cast<float*>(h->buf[h->cur]), static_cast<float*>(other), h->residual,
+                                 h->timestep, nsteps, nullptr, nullptr, h->workspace, ws_bytes, h->stream, &in_spare);
         else
             rc = amb_step_f32(&h->stencil, &h->model, h->seed, h->nrows, h->ncols, static_cast<float*>(h->buf[h->cur]),
                               static_cast<float*>(other), h->residual, h->timestep, nsteps, nullptr, AMB_KERNEL_AUTO,

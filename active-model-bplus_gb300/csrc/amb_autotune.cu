@@ -1,9 +1,9 @@
 // Measured choice of the FP32 step kernel and its launch shape for one grid shape
 // (no reference counterpart; the reference launches fixed 8 x 8 blocks).
 //
-// Candidates: the tile kernel with 256, 512 or 1024 threads per CTA, 32 x 32 or 28 x 32 output
-// tiles, launched once per step or once for all steps (persistent, grid barrier between steps),
-// and the warp-pair sliding
+// Candidates: the tile kernel with 256 or 512 threads per CTA, 32 or 64 output columns and the
+// heights that put a whole number of tiles on each SM, launched once per step or once for all steps
+// (persistent, grid barrier between steps), and the warp-pair sliding
 // kernel with 1, 2 or 4 pairs per CTA (or, fused, one single warp per CTA) and the row-segment
 // heights that put a whole number of tasks on each SM (plus the occupancy model's own choice). All candidates
 // give bitwise the same field. Each is timed with CUDA events over a few steps on
@@ -39,8 +39,10 @@ namespace
         float* a = nullptr;
         float* b = nullptr;
         uint16_t* r = nullptr;
+        void* ws = nullptr;
         ~Scratch()
         {
+            if (ws) cudaFree(ws);
             if (a) cudaFree(a);
             if (b) cudaFree(b);
             if (r) cudaFree(r);
@@ -93,6 +95,8 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
     cudaError_t e = cudaMalloc(&s.a, n * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&s.b, n * sizeof(float));
     if (e == cudaSuccess && compensated) e = cudaMalloc(&s.r, n * sizeof(uint16_t));
+    const size_t ws_bytes = amb_step_workspace_bytes(AMB_F32, nrows, ncols);
+    if (e == cudaSuccess) e = cudaMalloc(&s.ws, ws_bytes);
     if (e == cudaSuccess) e = cudaMemset(s.a, 0, n * sizeof(float));
     if (e == cudaSuccess && compensated) e = cudaMemset(s.r, 0, n * sizeof(uint16_t));
     if (e != cudaSuccess)
@@ -102,16 +106,30 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
     }
 
     std::vector<amb_kernel_config> cands;
-    for (int groups : {1, 2, 4})
-        for (int flags : {0, AMB_FLAG_PERSISTENT, AMB_FLAG_TILE_ROWS_28, AMB_FLAG_PERSISTENT | AMB_FLAG_TILE_ROWS_28})
-            cands.push_back({AMB_KERNEL_TILE, 0, groups, flags});
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, key_device());
+    // Tile heights that put m tiles on each SM (and the default 32 rows), for both tile widths.
+    for (int cols : {32, 64})
+    {
+        const int across = (ncols + cols - 1) / cols, wide = cols == 64 ? AMB_FLAG_TILE_COLS_64 : 0;
+        std::vector<int> rows{std::min(32, nrows)};
+        for (int m : {1, 2, 3, 4, 6})
+        {
+            const int down = std::max(1, std::min(nrows, sms * m / across));
+            const int h = (nrows + down - 1) / down;
+            if (h <= 64) rows.push_back(h);
+        }
+        std::sort(rows.begin(), rows.end());
+        rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
+        for (int h : rows)
+            for (int groups : {1, 2})
+                for (int flags : {0, AMB_FLAG_PERSISTENT}) cands.push_back({AMB_KERNEL_TILE, h, groups, flags | wide});
+    }
     if (ncols >= 112 && ncols % 4 == 0)
     {
         // Segment heights that put m tasks on each SM: a task costs its rows plus about eight rows of
         // pipeline fill, so the best height is one whose task count just fills the SMs, with as many
         // resident tasks as pay for their fill (1536^2: 24 rows, 30.8 us; 16 and 32 rows 37).
-        int sms = 152, dev = key_device();
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int strips = (ncols + 111) / 112;
         const auto rows_for = [&](int m) {
             const int segs = std::max(1, std::min(nrows, sms * m / strips));
@@ -133,11 +151,12 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
     cudaEventCreate(&t1);
     auto time_one = [&](const amb_kernel_config& c, float* ms) -> int {
         int in_spare = 0;
-        int rc = amb_step_f32_ex(stencil, model, 1, nrows, ncols, s.a, s.b, s.r, 0, 2, nullptr, &c, stream, &in_spare);
+        int rc = amb_step_f32_ws(stencil, model, 1, nrows, ncols, s.a, s.b, s.r, 0, 2, nullptr, &c, s.ws, ws_bytes, stream,
+                                 &in_spare);
         if (rc) return rc;
         cudaEventRecord(t0, static_cast<cudaStream_t>(stream));
-        rc = amb_step_f32_ex(stencil, model, 1, nrows, ncols, s.a, s.b, s.r, 2, probe_steps, nullptr, &c, stream,
-                             &in_spare);
+        rc = amb_step_f32_ws(stencil, model, 1, nrows, ncols, s.a, s.b, s.r, 2, probe_steps, nullptr, &c, s.ws, ws_bytes,
+                             stream, &in_spare);
         if (rc) return rc;
         cudaEventRecord(t1, static_cast<cudaStream_t>(stream));
         if (cudaEventSynchronize(t1) != cudaSuccess) return AMB_ERR_CUDA;

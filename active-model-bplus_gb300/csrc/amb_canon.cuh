@@ -207,21 +207,11 @@ namespace amb
         return rfma(k.dyInv, ksub(sxj_p, sxj_m, k), v);
     }
 
-    // The update of one site: plain, or compensated with residual r (in/out).
+    // The plain update of one site.
     template <typename Real, typename K>
     __device__ __forceinline__ Real canon_update(Real f, Real dx8, Real divtj, Real dy8, const K& k)
     {
         const Real div = kadd(dx8, kadd(divtj, dy8, k), k);
         return rfma(k.ndt, div, f);
-    }
-
-    __device__ __forceinline__ float canon_update_comp(float f, float dx8, float divtj, float dy8, float& r,
-                                                       const Canon<float>& k)
-    {
-        const float div = radd(dx8, radd(divtj, dy8));
-        const float F = rfma(k.dt, div, r);
-        const float nf = rsub(f, F);
-        r = radd(rsub(nf, f), F);
-        return nf;
     }
 }

@@ -11,18 +11,27 @@
 
 namespace amb
 {
-    // Fused single-step tile kernel (amb_step_tile.cuh), one launch = one step; groups x 256
+    // Fused single-step FP64 tile kernel (amb_step_tile.cuh), one launch = one step; groups x 256
     // threads per CTA (groups in {1, 2, 4}); 32 x 32 output tiles, or 28 x 32 with rows28.
-    template <typename Real>
-    cudaError_t launch_step_tile(const Real* phi_in, Real* phi_out, __nv_bfloat16* comp, int comp_mode,
-                                 const StepParams& p, int noise_mode, const Real* injected, int groups, bool rows28,
-                                 cudaStream_t stream);
-    // nsteps steps of the tile kernel in one cooperative launch (grid barrier between steps); the
+    cudaError_t launch_step_tile(const double* phi_in, double* phi_out, const StepParams& p, int noise_mode,
+                                 const double* injected, int groups, bool rows28, cudaStream_t stream);
+    // nsteps steps of the FP64 tile kernel in one cooperative launch (grid barrier between steps); the
     // result is in a when nsteps is even, in b when odd. injected: nsteps * 2 planes or nullptr.
-    template <typename Real>
-    cudaError_t launch_steps_tile_persistent(Real* a, Real* b, __nv_bfloat16* comp, int comp_mode,
-                                             const StepParams& p, int noise_mode, const Real* injected, int nsteps,
-                                             int groups, bool rows28, cudaStream_t stream);
+    cudaError_t launch_steps_tile_persistent(double* a, double* b, const StepParams& p, int noise_mode,
+                                             const double* injected, int nsteps, int groups, bool rows28,
+                                             cudaStream_t stream);
+
+    // FP32 steps of the quad tile kernel (amb_step_quad.cuh): one launch per step, or, with a barrier
+    // counter (one word of device memory), one cooperative launch. The result is in a when nsteps is even.
+    struct QuadTile
+    {
+        int rows;      // output rows of a tile, 1 .. 64
+        int threads;   // 256 or 512
+        bool cols64;   // output columns 64 instead of 32
+    };
+    cudaError_t launch_step_quad(float* a, float* b, __nv_bfloat16* comp, const StepParams& p, int noise_mode,
+                                 const float* injected, int nsteps, const QuadTile& tile, unsigned* count,
+                                 cudaStream_t stream);
 
     // FP64 steps in three grid-wide phases, all steps of a call in one cooperative launch (or several,
     // for long calls); the planes between the phases live in `workspace` (amb_step_phase.cuh).

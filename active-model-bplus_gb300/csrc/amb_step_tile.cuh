@@ -7,10 +7,9 @@
 // 112-176, 178-262) run out of shared memory in one launch, so HBM sees one read
 // and one write of phi per site-update instead of ~280 B.
 //
-// This is the general form: any grid size >= 1 (periodic wrap by index
-// arithmetic on the halo load), FP64 or FP32 storage, Philox or injected noise.
-// It is the correctness vehicle and the FP64 path; the FP32 headline path is the
-// register-sliding kernel in amb_step_f32.cu.
+// Any grid size >= 1 (periodic wrap by index arithmetic on the halo load), Philox or injected noise.
+// It runs FP64 calls that bring no workspace for the three-phase kernel (amb_step_phase.cuh), and
+// calls under stream capture.
 #pragma once
 
 #include "amb_canon.cuh"
@@ -70,9 +69,8 @@ namespace amb
     }
 
     // One step of one TY x TX output tile (origin r0, c0): the whole body of the tile kernel.
-    template <typename Real, int TY, int TX, int COMP, bool COHERENT, int NT>
+    template <typename Real, int TY, int TX, bool COHERENT, int NT>
     __device__ __forceinline__ void tile_step(const Real* __restrict__ phi_in, Real* __restrict__ phi_out,
-                                              const __nv_bfloat16* comp_in, __nv_bfloat16* comp_out,
                                               const StepParams& p, const Canon<Real>& k, int noise_mode,
                                               const Real* __restrict__ injected, int r0, int c0,
                                               unsigned char* smem_raw)
@@ -227,29 +225,19 @@ namespace amb
             const Real dx8 = canon_d8(k.px8, cx[-1], cx[1], cx[-2], cx[2], cx[-3], cx[3], cx[-4], cx[4], k);
             const Real f = PHI[(i + G::H) * G::LX + (j + G::H)];
             const size_t gi = (size_t)gr * nx + gc;
-            if constexpr (COMP == COMP_BF16)
-            {
-                float r = __bfloat162float(load_field<__nv_bfloat16, COHERENT>(comp_in + gi));
-                phi_out[gi] = canon_update_comp(f, dx8, divtj, dy8, r, k);
-                comp_out[gi] = __float2bfloat16_rn(r);
-            }
-            else
-            {
-                phi_out[gi] = canon_update(f, dx8, divtj, dy8, k);
-            }
+            phi_out[gi] = canon_update(f, dx8, divtj, dy8, k);
         });
     }
 
     // One step, one tile per CTA (grid = tiles). Both tile kernels are built for 1024 threads per
     // SM (at most 64 registers per thread).
-    template <typename Real, int TY, int TX, int COMP, int NT>
+    template <typename Real, int TY, int TX, int NT>
     __global__ void __launch_bounds__(NT, 1024 / NT)
     step_tile_kernel(const Real* __restrict__ phi_in, Real* __restrict__ phi_out,
-                     const __nv_bfloat16* comp_in, __nv_bfloat16* comp_out,  // may alias: each site reads/writes only its own
                      StepParams p, const Canon<Real> k, int noise_mode, const Real* __restrict__ injected)
     {
         extern __shared__ __align__(16) unsigned char smem_raw[];
-        tile_step<Real, TY, TX, COMP, false, NT>(phi_in, phi_out, comp_in, comp_out, p, k, noise_mode, injected,
+        tile_step<Real, TY, TX, false, NT>(phi_in, phi_out, p, k, noise_mode, injected,
                                              blockIdx.y * TY, blockIdx.x * TX, smem_raw);
     }
 
@@ -287,9 +275,9 @@ namespace amb
     // and writes buf[(s + 1) % 2]. The per-site arithmetic is the tile kernel's (tile_step), so
     // the result is bitwise that of nsteps single-step launches. If a barrier gives up, the CTA
     // fills its tiles of both buffers with NaN (caught by the finite check) and leaves.
-    template <typename Real, int TY, int TX, int COMP, int NT>
+    template <typename Real, int TY, int TX, int NT>
     __global__ void __launch_bounds__(NT, 1024 / NT)
-    step_tile_persistent_kernel(Real* buf0, Real* buf1, __nv_bfloat16* comp, StepParams p, const Canon<Real> k,
+    step_tile_persistent_kernel(Real* buf0, Real* buf1, StepParams p, const Canon<Real> k,
                                 int noise_mode, const Real* __restrict__ injected, int nsteps, unsigned* count,
                                 int* error)
     {
@@ -307,7 +295,7 @@ namespace amb
             const Real* inj = injected ? injected + (size_t)s * 2 * plane : nullptr;
             for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
             {
-                tile_step<Real, TY, TX, COMP, true, NT>(in, out, comp, comp, p, k, noise_mode, inj, (tile / tx) * TY,
+                tile_step<Real, TY, TX, true, NT>(in, out, p, k, noise_mode, inj, (tile / tx) * TY,
                                                     (tile % tx) * TX, smem_raw);
                 __syncthreads();
             }

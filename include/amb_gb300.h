@@ -81,9 +81,10 @@ typedef struct amb_model
 #define AMB_KERNEL_SLIDING 2 /* warp-pair sliding FP32 kernel (ncols % 4 == 0, ncols >= 112, 16-byte aligned) */
 
 /* Explicit kernel configuration for amb_step_f32_ex / amb_step_f64_ex (zeros mean defaults).
- * seg_rows: rows per warp-pair task of the sliding kernel.
+ * seg_rows: rows per warp-pair task of the sliding kernel; output rows per tile of the FP32 tile
+ *   kernel (1 to 64; 0: 32, or 28 with AMB_FLAG_TILE_ROWS_28).
  * pairs_per_cta: sliding kernel: warp pairs per CTA (1, 2 or 4); tile kernel: groups of 256
- *   threads per CTA (1, 2 or 4).
+ *   threads per CTA (1, 2 or 4; FP32: 4 runs as 2).
  * flags: AMB_FLAG_PERSISTENT (tile kernel): all nsteps of the call in one cooperative launch,
  *   a grid-wide barrier between the steps (for grids too small to fill the GPU, where a launch
  *   per step costs more than the step; ignored while the stream is being captured). The
@@ -92,7 +93,9 @@ typedef struct amb_model
  *   warp pair); pairs_per_cta then counts warps per CTA (1, 2 or 4). Bitwise the same results.
  *   AMB_FLAG_TILE_ROWS_28 (tile kernel): output tiles of 28 rows x 32 columns instead of 32 x 32
  *   (balances small grids over the SMs: 512 x 512 is 304 tiles, two per SM). Bitwise the same
- *   results. */
+ *   results.
+ *   AMB_FLAG_TILE_COLS_64 (FP32 tile kernel): 64 output columns per tile instead of 32. Bitwise the
+ *   same results. */
 typedef struct amb_kernel_config
 {
     int kernel;
@@ -103,6 +106,7 @@ typedef struct amb_kernel_config
 #define AMB_FLAG_PERSISTENT 1
 #define AMB_FLAG_FUSED 2
 #define AMB_FLAG_TILE_ROWS_28 4
+#define AMB_FLAG_TILE_COLS_64 8
 
 /* Number of FP64 planes written by amb_terms_*: mu_p, mu_a, J_p(y,x), J_l(y,x), J_c(y,x), J_r(y,x). */
 #define AMB_NTERMS 10
@@ -199,6 +203,13 @@ int amb_step_f32_ex(const amb_stencil* stencil, const amb_model* model, uint64_t
                     float* field, float* spare, uint16_t* residual, int64_t step0, int nsteps,
                     const float* injected_noise, const amb_kernel_config* config, void* stream,
                     int* result_in_spare);
+/* amb_step_f32_ex with a workspace (amb_step_workspace_bytes(AMB_F32, nrows, ncols) bytes; the rules of
+ * amb_step_f64_ws): the persistent tile kernel's barrier counter lives there instead of being
+ * allocated from the stream's pool in each call. */
+int amb_step_f32_ws(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
+                    float* field, float* spare, uint16_t* residual, int64_t step0, int nsteps,
+                    const float* injected_noise, const amb_kernel_config* config, void* workspace,
+                    size_t workspace_bytes, void* stream, int* result_in_spare);
 
 /* Every term of the reference's forces/currents kernels (src/integrator.cu:46-176) at
  * timestep `step`, as AMB_NTERMS FP64 device planes in `out` (order in AMB_NTERMS).
