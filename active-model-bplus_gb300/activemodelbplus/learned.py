@@ -138,6 +138,20 @@ def conv_wgrad(x, dz, *, cin: int, npad: int, error=None):
     return dw
 
 
+def param_grads(x, dz, *, cin: int, npad: int, cin_used: int, cout: int, scratch: _Scratch, bias: bool = True, error=None):
+    """Gradients of one layer's weights [cout, cin_used, 5, 5] and (``bias``) of its bias [npad], else None
+    (``amb_conv5x5_param_grads``)."""
+    torch = _torch()
+    B, _, H, W, _ = x.shape
+    lib = N.lib()
+    buf = scratch.get(lib.amb_conv5x5_wgrad_scratch_bytes(B, H, W, cin, npad), x.device)
+    gw = torch.empty(cout, cin_used, 5, 5, dtype=torch.float32, device=x.device)
+    gb = torch.empty(npad, dtype=torch.float32, device=x.device) if bias else None
+    _check(lib.amb_conv5x5_param_grads(_ptr(x), _ptr(dz), B, H, W, cin, npad, cin_used, cout, _ptr(gw), _ptr(gb),
+                                       _ptr(buf), buf.numel() * 4, _ptr(error), _stream()))
+    return gw, gb
+
+
 def network_input(phi, params):
     """phi [B, H, W] FP32, params [B, 3] (zeta, lambda, T) -> bf16 chunk planes [B, 2, H, W, 8]."""
     torch = _torch()
@@ -183,6 +197,7 @@ class FluxNet:
         self._images = None
         self._dimages = None
         self._saved = None
+        self._scratch = _Scratch()
 
     # -- parameters
     def parameters(self):
@@ -190,9 +205,25 @@ class FluxNet:
 
     def refresh(self) -> None:
         """Rebuild the bf16 operand images after the FP32 weights changed."""
-        self._images = [weight_image(w, self.cin[l], self.npad[l]) for l, w in enumerate(self.weights)]
-        self._dimages = [None] + [dgrad_image(self.weights[l], self.cin[l], self.npad[l])
-                                  for l in range(1, self.nlayers)]
+        torch = _torch()
+        if not all(w.is_cuda for w in self.weights):
+            self._images = [weight_image(w, self.cin[l], self.npad[l]) for l, w in enumerate(self.weights)]
+            self._dimages = [None] + [dgrad_image(self.weights[l], self.cin[l], self.npad[l])
+                                      for l in range(1, self.nlayers)]
+            return
+        # one kernel per layer builds both images, in a buffer of their own (a captured macro step
+        # keeps reading the images that it was captured with)
+        sizes = [25 * self.cin[l] * self.npad[l] for l in range(self.nlayers)]
+        buf = torch.empty(2 * sum(sizes), dtype=torch.bfloat16, device=self.weights[0].device)
+        self._images, self._dimages, at = [], [], 0
+        for l, (w, n) in enumerate(zip(self.weights, sizes)):
+            img, dimg = buf[at:at + n], buf[at + n:at + 2 * n] if l else None
+            at += 2 * n
+            w = w.detach().to(torch.float32).contiguous()
+            _check(N.lib().amb_conv5x5_images(_ptr(w), self.cout[l], self.cin_used[l], self.cin[l], self.npad[l],
+                                              _ptr(img), _ptr(dimg), _stream()))
+            self._images.append(img)
+            self._dimages.append(dimg)
 
     def state_dict(self) -> dict:
         d = {}
@@ -257,8 +288,8 @@ class FluxNet:
         gw, gb = [None] * self.nlayers, [None] * self.nlayers
         dz = to_chunks(dflux, NOUT_PAD)
         L = self.nlayers - 1
-        gw[L] = wgrad_to_weights(conv_wgrad(inputs[L], dz, cin=self.cin[L], npad=self.npad[L], error=self.error),
-                                 self.cout[L], self.cin_used[L])
+        gw[L], _ = param_grads(inputs[L], dz, cin=self.cin[L], npad=self.npad[L], cin_used=self.cin_used[L],
+                               cout=self.cout[L], scratch=self._scratch, bias=False, error=self.error)
         gb[L] = torch.nn.functional.pad(dflux.sum(dim=(0, 2, 3)), (0, NOUT_PAD - NOUT))
         B, _, H, W, _ = dz.shape
         for l in range(L, 0, -1):
@@ -267,9 +298,8 @@ class FluxNet:
                          epilogue=N.AMB_EPI_GELU_BWD, out=prev, gate=pres[l - 1], error=self.error)
             dz = prev
             k = l - 1
-            gw[k] = wgrad_to_weights(conv_wgrad(inputs[k], dz, cin=self.cin[k], npad=self.npad[k],
-                                                error=self.error), self.cout[k], self.cin_used[k])
-            gb[k] = from_chunks(dz, self.npad[k]).sum(dim=(0, 2, 3))
+            gw[k], gb[k] = param_grads(inputs[k], dz, cin=self.cin[k], npad=self.npad[k], cin_used=self.cin_used[k],
+                                       cout=self.cout[k], scratch=self._scratch, error=self.error)
         self._saved = None
         return gw, gb
 
@@ -769,6 +799,7 @@ class LearnedStepper:
             with torch.cuda.graph(g):  # records only; the state changes at replay
                 self._apply(noisy=noisy)
             self._graph = g
+            self._held = (self.net._images, list(self.net.biases))  # what the captured kernels read
         if self._graph is not None:
             self._graph.replay()
         else:

@@ -28,12 +28,20 @@
 // the channel roles swapped, so the same kernel serves it with the
 // GELU-derivative epilogue.
 //
-// Weight-gradient kernel (conv_wgrad_kernel): dW[tap][ci][co] = sum over sites
-// of X[ci][site + tap] dZ[co][site]. Per MMA: M = 128 rows = (ky block, ci), with
-// 16/(Cin/8) ky values stacked along M (the staged rows sit at a uniform pitch,
-// so (ky, chunk) is one uniform M stride), N = Cout, K = 16 sites; both operands
-// MN-major. Partial sums per CTA go to scratch and a second kernel reduces them
-// in a fixed order (deterministic gradients).
+// Weight-gradient kernel (conv_wgrad_kernel): dW[ky][kx][ci][co] = sum over sites and rows of
+// X[ci][row j + ky - 2][site + kx - 2] dZ[co][row j][site]. A block of 16/(Cin/8) X rows is stacked along
+// M ((row, ci), 128 rows) and all dZ rows within two of them along N ((chunk, row, channel), up to 384), so ONE
+// instruction per x tap and 16 sites accumulates every (X row, dZ row) pair, of which the diagonals
+// ky = X row - dZ row are the taps: the other pairs (3 of 8) are not read. Both operands MN-major. Against
+// five y taps as separate 128 x 32 instructions, whose cost does not fall below that of N = 128, this
+// takes a sixth of the tensor time. A persistent CTA keeps its x taps' accumulators in TMEM over all its
+// row blocks (double-buffered bulk copies), sums the diagonals once at the end and writes one partial;
+// a second kernel reduces the partials in a fixed order (deterministic gradients). The same CTAs sum dZ
+// over the sites while it is staged (bias gradients).
+// Measured for 16 x 128^2 sites, 32 x 32 channels: 25 us and 3.6 us for the reduction (one 128 x 32
+// instruction per tap, 256 partials: 80 and 17 us). 9 us of it are instructions, the rest the copies, which
+// the copy engine takes one by one (dZ rows that follow one another in memory go as one), and the
+// epilogue.
 #include "amb_gb300.h"
 #include "amb_kernels.h"
 #include "amb_tc.cuh"
@@ -83,8 +91,10 @@ namespace
     {
         const uint16_t* x;   // [batch][cin/8][nrows][ncols][8]
         const uint16_t* dz;  // [batch][npad/8][nrows][ncols][8]
-        float* partial;      // [grid][25][cin][npad]
-        int batch, nrows, ncols, cin_chunks, npad, rows_per_cta;
+        float* partial;      // [CTA][x tap of the CTA][5 ky][cin][npad]
+        float* bias;         // [CTA of group 0][npad], or null
+        int batch, nrows, ncols;
+        int first[6];        // first CTA of each x-tap group
         int* error;
     };
 
@@ -109,23 +119,25 @@ namespace
         return c;
     }
 
-    // wgrad: ky blocks per MMA along M, staged X rows per output-row range
-    __host__ __device__ inline int wg_kb(int cc) { return 16 / cc; }
-    __host__ __device__ inline int wg_nstarts(int cc) { return wg_kb(cc) >= 5 ? 1 : 2; }
-    __host__ __device__ inline int wg_start(int cc, int si) { return si == 0 ? 0 : 5 - wg_kb(cc); }
-    __host__ __device__ inline int wg_extra_rows(int cc) { return wg_kb(cc) - 1 > 4 ? wg_kb(cc) - 1 : 4; }
-    __host__ __device__ inline uint32_t wg_x_bytes(int cc, int rows) { return uint32_t(rows + wg_extra_rows(cc)) * cc * kRowPlane; }
-    __host__ __device__ inline uint32_t wg_dz_bytes(int npad, int rows) { return uint32_t(rows) * (npad / 8) * kTile * 16u; }
-    __host__ __device__ inline uint32_t wg_bar_offset(int cc, int npad, int rows)
+    // wgrad geometry for Cin = 8 CC and NPAD gradient channels
+    template <int CC, int NPAD>
+    struct Wg
     {
-        return align128(wg_x_bytes(cc, rows)) + align128(wg_dz_bytes(npad, rows));
-    }
-    constexpr uint32_t kWgradMinSmem = 120u * 1024u;  // keeps one wgrad CTA per SM (it owns all of TMEM)
-    __host__ __device__ inline uint32_t wg_smem_bytes(int cc, int npad, int rows)
-    {
-        uint32_t need = wg_bar_offset(cc, npad, rows) + 256u;
-        return need > kWgradMinSmem ? need : kWgradMinSmem;
-    }
+        static constexpr int CIN = 8 * CC, NQ = NPAD / 8;
+        static constexpr int XR = 16 / CC;           // X rows of a block: M = 128 = (row, ci)
+        static constexpr int ZR = XR + 4;            // dZ rows of a block: N = (row, co)
+        static constexpr int COLS = ZR * NPAD;       // TMEM columns of one x tap
+        static constexpr int KPC = 512 / COLS;       // x taps per CTA
+        static constexpr int GROUPS = (5 + KPC - 1) / KPC;
+        static constexpr uint32_t XB = (uint32_t(XR) * CC * kRowPlane + 127u) & ~127u;
+        static constexpr uint32_t STAGE = XB + uint32_t(ZR) * NQ * kTile * 16u;
+        static constexpr int NST = 2 * STAGE + 1024u <= kSmemLimit ? 2 : 1;
+        static constexpr uint32_t BARS = NST * STAGE;
+        static constexpr uint32_t SMEM = BARS + 128u + 4u * 32u * 4u;
+        static constexpr int ROW = NPAD + 4;         // floats of an accumulator row in shared memory
+        static constexpr int PART = KPC * 5 * CIN * NPAD;  // floats of one CTA's partial
+        static_assert(KPC * 5 * CIN * ROW * 4 <= int(NST * STAGE), "accumulators fit where the stages were");
+    };
 
     __device__ __forceinline__ void give_up(int* error, volatile int* abort, int code)
     {
@@ -530,41 +542,51 @@ namespace
     }
 
     // =========================================================== weight grad
-    __global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(const WgradArgs a)
+    template <int CC, int NPAD>
+    __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const WgradArgs a)
     {
+        using G = Wg<CC, NPAD>;
         extern __shared__ __align__(1024) uint8_t smem[];
-        const int cc = a.cin_chunks, npad = a.npad, nq = npad / 8;
-        const int R = a.rows_per_cta;
-        const uint32_t xrow = uint32_t(cc) * kRowPlane;    // bytes per staged X row
-        const uint32_t dzrow = uint32_t(nq) * kTile * 16;  // bytes per staged dZ row
-        uint8_t* xs = smem;
-        uint8_t* dzs = smem + align128(wg_x_bytes(cc, R));
-        uint64_t* bars = reinterpret_cast<uint64_t*>(smem + wg_bar_offset(cc, npad, R));
-        uint64_t* ld = bars;
-        uint64_t* done = bars + 1;
-        uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
+        uint64_t* full = reinterpret_cast<uint64_t*>(smem + G::BARS);
+        uint64_t* empty = full + 2;
+        uint64_t* done = empty + 2;
+        uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
         volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
+        float* bsum = reinterpret_cast<float*>(smem + G::BARS + 128);
 
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int nwin = a.ncols / kTile;
-        const int ngroups = (a.nrows + R - 1) / R;
-        int t = blockIdx.x;
-        const int cw = t % nwin;
-        t /= nwin;
-        const int rg = t % ngroups;
-        const int b = t / ngroups;
-        const int c0 = cw * kTile;
-        const int r0 = rg * R;
-        const int nout = min(R, a.nrows - r0);
-        const int nx_rows = nout + wg_extra_rows(cc);
-        const int kb = wg_kb(cc), nst = wg_nstarts(cc);
+        int group = 0;
+        while (int(blockIdx.x) >= a.first[group + 1]) ++group;
+        const int kx0 = group * G::KPC, nkx = min(G::KPC, 5 - kx0);
+        const int cta = blockIdx.x - a.first[group], nctas = a.first[group + 1] - a.first[group];
+        const int nwin = a.ncols / kTile, nblk = (a.nrows + G::XR - 1) / G::XR;
+        const int total = a.batch * nwin * nblk;
+        const int mine = cta < total ? (total - cta + nctas - 1) / nctas : 0;  // row blocks of this CTA
 
-        // the X windows' wrapped sites (first and last windows) are copied by the epilogue
-        // warps, one arrival on `ld` each (see the forward kernel)
-        const int wleft = c0 == 0 ? 2 : 0, wright = c0 + kTile == a.ncols ? 2 : 0;
+        struct Block
+        {
+            int b, c0, r0, rows, left, right;  // image, first column, first X row, X rows, wrapped sites
+        };
+        const auto block = [&](int i) {
+            int t = cta + i * nctas;
+            Block k;
+            k.r0 = t % nblk * G::XR;
+            t /= nblk;
+            k.c0 = t % nwin * kTile;
+            k.b = t / nwin;
+            k.rows = min(G::XR, a.nrows - k.r0);
+            k.left = k.c0 == 0 ? 2 : 0;
+            k.right = k.c0 + kTile == a.ncols ? 2 : 0;
+            return k;
+        };
+
         if (threadIdx.x == 0)
         {
-            mbar_init(ld, 1 + nx_rows * cc * (wleft + wright));
+            for (int i = 0; i < G::NST; ++i)
+            {
+                mbar_init(&full[i], 1 + 4);   // the loader and the four helper warps
+                mbar_init(&empty[i], 1 + 4);  // the MMAs' completion and the helper warps
+            }
             mbar_init(done, 1);
             *abort = 0;
             fence_mbar_init();
@@ -581,112 +603,231 @@ namespace
 
         if (warp == 0)
         {
-            if (lane == 0)
             {
-                const int lo = c0 - 2 + wleft, run = kSites - wleft - wright;  // in-range run of a window
-                const uint32_t bytes = uint32_t(nx_rows * cc * run) * 16u + uint32_t(nout) * dzrow;
-                mbar_expect_tx(ld, bytes);
-                for (int i = 0; i < nx_rows; ++i)
+                // the copies of a block spread over the warp's lanes: one thread takes about 120 cycles to issue
+                // each, the copy engine 75 per 2 KB and 148 per 8 KB
+                int issued = 0;
+                bool ok = true;
+                for (int i = 0; i < mine; ++i)
                 {
-                    const int row = wrap_row(r0 - 2 + i, a.nrows);
-                    for (int q = 0; q < cc; ++q)
+                    const int st = i % G::NST;
+                    if (i >= G::NST)
+                        ok = __all_sync(0xffffffffu, mbar_wait(&empty[st], (i / G::NST - 1) & 1, abort));
+                    if (!ok) break;
+                    const Block k = block(i);
+                    const int lo = k.c0 - 2 + k.left, run = kSites - k.left - k.right;
+                    uint8_t* xs = smem + st * G::STAGE;
+                    uint8_t* zs = xs + G::XB;
+                    if (lane == 0)
+                        mbar_expect_tx(&full[st], uint32_t(k.rows * CC * run) * 16u + uint32_t(G::ZR * G::NQ) * kTile * 16u);
+                    __syncwarp();
+                    const int nxc = k.rows * CC;
+                    for (int c = lane; c < nxc; c += 32)
+                        bulk_g2s(xs + c * kRowPlane + k.left * 16,
+                                 a.x + ((size_t(k.b * CC + c % CC) * a.nrows + k.r0 + c / CC) * size_t(a.ncols) + lo) * 8,
+                                 uint32_t(run) * 16u, &full[st]);
+                    // dZ rows r0 - 2 .. r0 + XR + 1, a chunk's rows one after the other: one copy per row, or, where
+                    // the window is the whole row, one per run of rows up to the image's end
+                    const bool runs = a.ncols == kTile && a.nrows >= G::ZR;
+                    const int z0 = wrap_row(k.r0 - 2, a.nrows), n0 = runs ? min(G::ZR, a.nrows - z0) : 1;
+                    const int per = runs ? (n0 < G::ZR ? 2 : 1) : G::ZR;
+                    for (int c = lane; c < G::NQ * per; c += 32)
                     {
-                        const uint16_t* src = a.x + (size_t(b * cc + q) * a.nrows + row) * size_t(a.ncols) * 8;
-                        bulk_g2s(xs + i * xrow + q * kRowPlane + wleft * 16, src + size_t(lo) * 8,
-                                 uint32_t(run) * 16u, ld);
+                        const int q = c / per, e = c - q * per;
+                        const int r = runs ? e * n0 : e, n = runs ? (e ? G::ZR - n0 : n0) : 1;
+                        bulk_g2s(zs + (q * G::ZR + r) * (kTile * 16),
+                                 a.dz + ((size_t(k.b * G::NQ + q) * a.nrows + wrap_row(k.r0 - 2 + r, a.nrows))
+                                             * size_t(a.ncols) + k.c0) * 8,
+                                 uint32_t(n) * kTile * 16u, &full[st]);
                     }
+                    __syncwarp();
+                    ++issued;
                 }
-                for (int j = 0; j < nout; ++j)
-                    for (int q = 0; q < nq; ++q)
-                    {
-                        const uint16_t* src =
-                            a.dz + ((size_t(b * nq + q) * a.nrows + (r0 + j)) * size_t(a.ncols) + c0) * 8;
-                        bulk_g2s(dzs + j * dzrow + q * (kTile * 16), src, kTile * 16, ld);
-                    }
-                if (!mbar_wait(ld, 0, nullptr)) give_up(a.error, abort, 4);
+                if (!ok && lane == 0) give_up(a.error, abort, 4);
+                // no copy may still be in flight when the CTA exits (the last of each stage completes last)
+                for (int i = max(0, issued - G::NST); i < issued; ++i)
+                    mbar_wait(&full[i % G::NST], (i / G::NST) & 1, nullptr);
             }
         }
         else if (warp == 1)
         {
             if (lane == 0)
             {
-                const uint32_t idesc = idesc_bf16(128, npad, true, true);
-                const uint32_t xa = smem_u32(xs), za = smem_u32(dzs);
-                bool ok = mbar_wait(ld, 0, abort);
-                if (ok)
+                constexpr int N0 = G::COLS < 256 ? G::COLS : 256, N1 = G::COLS - N0;
+                const uint32_t id0 = idesc_bf16(128, N0, true, true), id1 = idesc_bf16(128, N1 > 0 ? N1 : 16, true, true);
+                const uint32_t sa = smem_u32(smem);
+                bool ok = true, issued = false;
+                for (int i = 0; ok && i < mine; ++i)
                 {
-                    for (int j = 0; j < nout; ++j)
+                    const int st = i % G::NST;
+                    if (!mbar_wait(&full[st], (i / G::NST) & 1, abort))
+                    {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t xa = sa + st * G::STAGE, za = xa + G::XB;
+                    for (int kxi = 0; kxi < nkx; ++kxi)
                         for (int ks = 0; ks < kTile / 16; ++ks)
-                            for (int kx = 0; kx < 5; ++kx)
-                                for (int si = 0; si < nst; ++si)
-                                {
-                                    const uint32_t astart =
-                                        xa + (j + wg_start(cc, si)) * xrow + (ks * 16 + kx) * 16;
-                                    const uint64_t ad = smem_desc(astart, 128, kRowPlane);
-                                    const uint64_t bd = smem_desc(za + j * dzrow + ks * 256, 128, kTile * 16);
-                                    const uint32_t d = tbase + uint32_t((kx * nst + si) * npad);
-                                    mma_bf16(d, ad, bd, idesc, (j | ks) ? 1u : 0u);
-                                }
-                    mma_commit(done);
-                    if (!mbar_wait(done, 0, nullptr)) give_up(a.error, abort, 5);
+                        {
+                            const uint64_t ad = smem_desc(xa + uint32_t(ks * 16 + kx0 + kxi) * 16u, 128, kRowPlane);
+                            const uint32_t d = tbase + uint32_t(kxi * G::COLS), acc = (i | ks) ? 1u : 0u;
+                            mma_bf16(d, ad, smem_desc(za + ks * 256, 128, kTile * 16), id0, acc);
+                            if constexpr (N1 > 0)
+                                mma_bf16(d + N0, ad, smem_desc(za + (N0 / 8) * (kTile * 16) + ks * 256, 128, kTile * 16),
+                                         id1, acc);
+                        }
+                    mma_commit(&empty[st]);
+                    issued = true;
                 }
-                else
-                    give_up(a.error, abort, 6);
+                if (!ok) give_up(a.error, abort, 5);
+                if (issued || ok)
+                {
+                    mma_commit(done);
+                    if (!mbar_wait(done, 0, nullptr)) give_up(a.error, abort, 6);
+                }
             }
         }
         else
         {
-            const int q4 = warp & 3;
-            const int m = q4 * 32 + lane;  // accumulator row = (ky block, channel chunk, channel)
-            const int g = m >> 3, e = m & 7;
-            const int kyb = g / cc, ci = (g % cc) * 8 + e;
-            const int cin = cc * 8;
-            {
-                const int per_chunk = wleft + wright, per_row = cc * per_chunk;
-                for (int it = int(threadIdx.x) - 64; it < nx_rows * per_row; it += kThreads - 64)
+            const int t = int(threadIdx.x) - 64;
+            const bool bias = a.bias != nullptr && group == 0;
+            float bs[G::NQ][8];
+#pragma unroll
+            for (int q = 0; q < G::NQ; ++q)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) bs[q][e] = 0.f;
+            bool ok = true;
+            // ahead of the MMAs: the wrapped sites of a stage's X rows, zeros in the rows past the image
+            const auto prepare = [&](int i) {
+                const int st = i % G::NST;
+                if (i >= G::NST) ok = __all_sync(0xffffffffu, ok && mbar_wait(&empty[st], (i / G::NST - 1) & 1, abort));
+                if (!ok) return;
+                const Block k = block(i);
+                uint8_t* xs = smem + st * G::STAGE;
+                const int per_chunk = k.left + k.right, per_row = CC * per_chunk;
+                for (int it = t; it < k.rows * per_row; it += 128)
                 {
-                    const int i = it / per_row, rem = it - i * per_row;
+                    const int r = it / per_row, rem = it - r * per_row;
                     const int q = rem / per_chunk, s = rem - q * per_chunk;
-                    const bool at_left = s < wleft;
-                    const int wsite = at_left ? s : kSites - wright + (s - wleft);
-                    const int gcol = at_left ? a.ncols - 2 + s : s - wleft;
-                    const int row = wrap_row(r0 - 2 + i, a.nrows);
-                    const uint4 v = *reinterpret_cast<const uint4*>(
-                        a.x + ((size_t(b * cc + q) * a.nrows + row) * size_t(a.ncols) + gcol) * 8);
-                    *reinterpret_cast<uint4*>(xs + i * xrow + q * kRowPlane + wsite * 16) = v;
-                    fence_proxy_async();
-                    mbar_arrive(ld);
+                    const bool at_left = s < k.left;
+                    const int wsite = at_left ? s : kSites - k.right + (s - k.left);
+                    const int gcol = at_left ? a.ncols - 2 + s : s - k.left;
+                    *reinterpret_cast<uint4*>(xs + (r * CC + q) * kRowPlane + wsite * 16) = *reinterpret_cast<const uint4*>(
+                        a.x + ((size_t(k.b * CC + q) * a.nrows + k.r0 + r) * size_t(a.ncols) + gcol) * 8);
                 }
-            }
-            bool ok = mbar_wait(done, 0, abort);
-            ok = __all_sync(0xffffffffu, ok);
-            if (ok)
+                for (int it = t; it < (G::XR - k.rows) * CC * kSites; it += 128)
+                    *reinterpret_cast<uint4*>(xs + k.rows * CC * kRowPlane + it * 16) = make_uint4(0, 0, 0, 0);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[st]);
+            };
+            const auto finish = [&](int i) {
+                const int st = i % G::NST;
+                if (bias)
+                {
+                    ok = __all_sync(0xffffffffu, ok && mbar_wait(&full[st], (i / G::NST) & 1, abort));
+                    if (!ok) return;
+                    const Block k = block(i);
+                    const uint8_t* zs = smem + st * G::STAGE + G::XB;
+                    for (int r = 2; r < 2 + k.rows; ++r)  // the dZ rows with the block's X rows' numbers
+#pragma unroll
+                        for (int q = 0; q < G::NQ; ++q)
+                        {
+                            float v[8];
+                            unpack_bf16x8(*reinterpret_cast<const uint4*>(zs + (q * G::ZR + r) * (kTile * 16) + t * 16), v);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) bs[q][e] += v[e];
+                        }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[st]);
+            };
+            for (int i = 0; ok && i < mine + G::NST - 1; ++i)
             {
-                tc_fence_after();
-                for (int kx = 0; kx < 5; ++kx)
-                    for (int si = 0; si < nst; ++si)
+                if (i < mine) prepare(i);
+                if (ok && i >= G::NST - 1) finish(i - (G::NST - 1));
+            }
+            if (!ok && lane == 0) give_up(a.error, abort, 7);
+            ok = __all_sync(0xffffffffu, mbar_wait(done, 0, abort) && ok);
+            if (!ok && lane == 0) give_up(a.error, abort, 8);
+            tc_fence_after();
+
+            // The diagonals, summed over the X rows of the block in shared memory (where the stages were).
+            // The lane's accumulator row is X row xr, channel ci; tap ky is dZ row xr - ky + 4 of the block.
+            float* acc = reinterpret_cast<float*>(smem);
+            const auto sync4 = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+            sync4();
+            for (int e = t; e < G::KPC * 5 * G::CIN * G::ROW; e += 128) acc[e] = 0.f;
+            sync4();
+            const int q4 = warp & 3;
+            const uint32_t lanes = uint32_t(q4 * 32) << 16;
+            const auto load = [&](int kxi, int zr, float (&v)[32]) {  // the NPAD channels of dZ row zr
+#pragma unroll
+                for (int q = 0; q < G::NQ; ++q)
+                    tmem_ld8(tbase + lanes + uint32_t(kxi * G::COLS + (q * G::ZR + zr) * 8), v + 8 * q);
+                tmem_wait_ld();
+            };
+            const auto add = [&](int kxi, int ky, int ci, const float (&v)[32]) {
+                float* row = acc + ((kxi * 5 + ky) * G::CIN + ci) * G::ROW;
+#pragma unroll
+                for (int n = 0; n < NPAD; n += 4)
+                {
+                    float4 w = *reinterpret_cast<float4*>(row + n);
+                    w.x += v[n]; w.y += v[n + 1]; w.z += v[n + 2]; w.w += v[n + 3];
+                    *reinterpret_cast<float4*>(row + n) = w;
+                }
+            };
+            if constexpr (CC == 4)  // one X row per warp: in each turn every warp adds to a tap of its own
+                for (int turn = 0; turn < 5; ++turn)
+                {
+                    const int ky = (q4 + turn) % 5;
+                    for (int kxi = 0; ok && mine > 0 && kxi < nkx; ++kxi)
                     {
                         float v[32];
-                        const uint32_t taddr = tbase + (uint32_t(q4 * 32) << 16) + uint32_t((kx * nst + si) * npad);
-                        if (npad == 32) tmem_ld32(taddr, v);
-                        else tmem_ld16(taddr, v);
-                        tmem_wait_ld();
-                        const int ky = wg_start(cc, si) + kyb;
-                        // keep each ky once: start 0 covers [0, kb), the second start only ky >= kb
-                        const bool keep = ky < 5 && (si == 0 || ky >= kb);
-                        if (keep)
-                        {
-                            float* dst = a.partial + ((size_t(blockIdx.x) * kTaps + ky * 5 + kx) * cin + ci) * npad;
-#pragma unroll
-                            for (int n = 0; n < 32; n += 4)
-                                if (n < npad)
-                                    *reinterpret_cast<float4*>(dst + n) =
-                                        make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
-                        }
+                        load(kxi, q4 - ky + 4, v);
+                        add(kxi, ky, lane, v);
                     }
+                    sync4();
+                }
+            else  // two X rows per warp, the warps one after the other
+                for (int turn = 0; turn < 4; ++turn)
+                {
+                    for (int kxi = 0; ok && mine > 0 && turn == q4 && kxi < nkx; ++kxi)
+                        for (int ky = 0; ky < 5; ++ky)
+                        {
+                            float v0[32], v1[32];
+                            load(kxi, 2 * q4 - ky + 4, v0);
+                            load(kxi, 2 * q4 - ky + 5, v1);
+                            if (lane < 16) add(kxi, ky, lane, v0);
+                            __syncwarp();
+                            if (lane >= 16) add(kxi, ky, lane - 16, v1);
+                            __syncwarp();
+                        }
+                    sync4();
+                }
+            float* part = a.partial + size_t(blockIdx.x) * G::PART;
+            for (int e = t; e < nkx * 5 * G::CIN * (NPAD / 4); e += 128)
+            {
+                const int row = e / (NPAD / 4), n = (e - row * (NPAD / 4)) * 4;
+                *reinterpret_cast<float4*>(part + size_t(row) * NPAD + n) =
+                    *reinterpret_cast<const float4*>(acc + row * G::ROW + n);
             }
-            else if (lane == 0)
-                give_up(a.error, abort, 7);
+            if (bias)
+            {
+#pragma unroll
+                for (int q = 0; q < G::NQ; ++q)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                    {
+                        float v = bs[q][e];
+#pragma unroll
+                        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                        if (lane == 0) bsum[(warp - 2) * 32 + q * 8 + e] = v;
+                    }
+                sync4();
+                if (t < NPAD) a.bias[size_t(cta) * NPAD + t] = ((bsum[t] + bsum[32 + t]) + bsum[64 + t]) + bsum[96 + t];
+            }
         }
 
         tc_fence_before();
@@ -698,13 +839,95 @@ namespace
         }
     }
 
-    __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int nparts, int total, float* __restrict__ dw)
+    struct WgradReduceArgs
     {
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+        const float* partial;
+        const float* bias_partial;
+        int first[6];          // CTAs of each x-tap group
+        int kpc, cin, npad;
+        float* dw;             // [25][cin][npad], or null
+        float* gw;             // [cout][cin_used][5][5], or null
+        float* gb;             // [npad], or null
+        int cout, cin_used;
+    };
+
+    // Sum of the CTAs' partials, four channels per thread, eight slices of the CTAs per element added in a
+    // fixed order; the last block sums the bias partials.
+    __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const WgradReduceArgs a)
+    {
+        __shared__ float4 sums[8][32];
+        const int el = threadIdx.x & 31, slice = threadIdx.x >> 5;
+        const int n4 = a.npad / 4, total = 25 * a.cin * n4;
+        const int e = blockIdx.x * 32 + el;
+        if (blockIdx.x * 32 >= total)  // the bias block
         {
             float s = 0.f;
-            for (int p = 0; p < nparts; ++p) s += partial[size_t(p) * total + i];
-            dw[i] = s;
+            if (el < a.npad)
+                for (int c = slice; c < a.first[1]; c += 8) s += a.bias_partial[size_t(c) * a.npad + el];
+            sums[slice][el].x = s;
+            __syncthreads();
+            if (slice == 0 && el < a.npad)
+            {
+                float v = sums[0][el].x;
+                for (int i = 1; i < 8; ++i) v += sums[i][el].x;
+                a.gb[el] = v;
+            }
+            return;
+        }
+        const int tap = e / (a.cin * n4), ci = e / n4 - tap * a.cin, n = e % n4;
+        const int ky = tap / 5, kx = tap - ky * 5, g = kx / a.kpc;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < total)
+        {
+            const size_t part = size_t(a.kpc) * 5 * a.cin * a.npad;
+            const float* p = a.partial + ((size_t(kx - g * a.kpc) * 5 + ky) * a.cin + ci) * a.npad + n * 4;
+            for (int c = a.first[g] + slice; c < a.first[g + 1]; c += 8)
+            {
+                const float4 v = *reinterpret_cast<const float4*>(p + size_t(c) * part);
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+        }
+        sums[slice][el] = s;
+        __syncthreads();
+        if (slice != 0 || e >= total) return;
+        for (int i = 1; i < 8; ++i)
+        {
+            const float4 v = sums[i][el];
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        if (a.dw) *reinterpret_cast<float4*>(a.dw + (size_t(tap) * a.cin + ci) * a.npad + n * 4) = s;
+        if (a.gw && ci < a.cin_used)
+        {
+            const float v[4] = {s.x, s.y, s.z, s.w};
+            for (int q = 0; q < 4; ++q)
+                if (n * 4 + q < a.cout) a.gw[(size_t(n * 4 + q) * a.cin_used + ci) * 25 + tap] = v[q];
+        }
+    }
+
+    // Operand images of one layer's weights w [cout][cin][5][5]: the forward convolution's
+    // [5 kx][cin_pad/8][5 (4 - ky)][npad][8] and, with the kernel flipped and the channel roles swapped, the data
+    // gradient's [5 kx][npad/8][5 (4 - ky)][cin_pad][8], zero in the padding.
+    __global__ void weight_images_kernel(const float* __restrict__ w, int cout, int cin, int cin_pad, int npad,
+                                         __nv_bfloat16* __restrict__ img, __nv_bfloat16* __restrict__ dimg)
+    {
+        const int n = 25 * cin_pad * npad;
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * n; t += gridDim.x * blockDim.x)
+        {
+            const bool fwd = t < n;
+            if (!(fwd ? img : dimg)) continue;
+            const int k = fwd ? cin_pad : npad, m = fwd ? npad : cin_pad;  // channels along K, along N
+            int e = fwd ? t : t - n;
+            const int e0 = e % 8;
+            e /= 8;
+            const int row = e % m;
+            e /= m;
+            const int s = e % 5;
+            e /= 5;
+            const int kc = (e % (k / 8)) * 8 + e0, kx = e / (k / 8);
+            const int co = fwd ? row : kc, ci = fwd ? kc : row;
+            float v = 0.f;
+            if (co < cout && ci < cin) v = w[((size_t(co) * cin + ci) * 5 + (fwd ? 4 - s : s)) * 5 + (fwd ? kx : 4 - kx)];
+            (fwd ? img : dimg)[fwd ? t : t - n] = __float2bfloat16_rn(v);
         }
     }
 
@@ -1012,12 +1235,10 @@ namespace
         return best;
     }
 
-    constexpr int kWgradRows = 8;
-
     // Raises a kernel's dynamic shared-memory limit once per device (so that later
     // launches, e.g. inside a stream capture, make no attribute calls).
     std::mutex g_attr_mutex;
-    int g_attr_selftest[64], g_attr_fwd[64], g_attr_fwd2[64], g_attr_wgrad[64];
+    int g_attr_selftest[64], g_attr_fwd[64], g_attr_fwd2[64], g_attr_wgrad[4][64];
 
     cudaError_t set_smem_attr(const void* fn, uint32_t bytes, int (&done)[64])
     {
@@ -1114,54 +1335,134 @@ extern "C" int amb_conv5x5_forward(const void* in, int batch, int nrows, int nco
     return e == cudaSuccess ? AMB_OK : fail_cuda("amb_conv5x5_forward", e);
 }
 
-static long long wgrad_grid(int batch, int nrows, int ncols)
+namespace
 {
-    return (long long)batch * (ncols / kTile) * ((nrows + kWgradRows - 1) / kWgradRows);
+    struct WgradPlan
+    {
+        int first[6] = {};
+        int groups = 0, kpc = 0, part = 0;
+        size_t bytes(int npad) const { return (size_t(first[groups]) * part + size_t(first[1]) * npad) * sizeof(float); }
+    };
+
+    // CTAs per x-tap group in proportion to its taps, one CTA per SM, no more than there are row blocks.
+    template <int CC, int NPAD>
+    WgradPlan wgrad_plan_of(int batch, int nrows, int ncols)
+    {
+        using G = Wg<CC, NPAD>;
+        WgradPlan p;
+        p.groups = G::GROUPS;
+        p.kpc = G::KPC;
+        p.part = G::PART;
+        const long long blocks = (long long)batch * (ncols / kTile) * ((nrows + G::XR - 1) / G::XR);
+        for (int g = 0; g < G::GROUPS; ++g)
+        {
+            const int taps = std::min(G::KPC, 5 - g * G::KPC);
+            p.first[g + 1] = p.first[g] + int(std::min<long long>(blocks, std::max(1, sm_count() * taps / 5)));
+        }
+        for (int g = G::GROUPS; g < 5; ++g) p.first[g + 1] = p.first[g];
+        return p;
+    }
+
+    WgradPlan wgrad_plan(int batch, int nrows, int ncols, int cin, int npad)
+    {
+        if (cin == 32) return npad == 32 ? wgrad_plan_of<4, 32>(batch, nrows, ncols) : wgrad_plan_of<4, 16>(batch, nrows, ncols);
+        return npad == 32 ? wgrad_plan_of<2, 32>(batch, nrows, ncols) : wgrad_plan_of<2, 16>(batch, nrows, ncols);
+    }
+
+    template <int CC, int NPAD>
+    cudaError_t launch_wgrad(const WgradArgs& a, int grid, int (&attr)[64], cudaStream_t s)
+    {
+        auto kern = conv_wgrad_kernel<CC, NPAD>;
+        cudaError_t e = set_smem_attr(reinterpret_cast<const void*>(kern), Wg<CC, NPAD>::SMEM, attr);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, kThreads, Wg<CC, NPAD>::SMEM, s>>>(a);
+        return cudaGetLastError();
+    }
+
+    int param_grads(const char* name, const void* x, const void* dz, int batch, int nrows, int ncols, int cin, int npad,
+                    int cin_used, int cout, float* dw, float* gw, float* gb, float* scratch, size_t scratch_bytes,
+                    int* error, void* stream)
+    {
+        if (!x || !dz || !scratch || !valid_geometry(batch, nrows, ncols) || (cin != 16 && cin != 32) ||
+            (npad != 16 && npad != 32) || cin_used < 1 || cin_used > cin || cout < 1 || cout > npad)
+            return fail_invalid("weight gradient: need ncols % 128 == 0, nrows >= 3, cin and npad in {16, 32}");
+        const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+        if (!al16(x) || !al16(dz) || !al16(scratch) || (dw && !al16(dw)))
+            return fail_invalid("weight gradient: buffers must be 16-byte aligned");
+        const WgradPlan plan = wgrad_plan(batch, nrows, ncols, cin, npad);
+        if (scratch_bytes < plan.bytes(npad))
+            return fail_invalid("weight gradient: scratch too small (see amb_conv5x5_wgrad_scratch_bytes)");
+        WgradArgs a{};
+        a.x = static_cast<const uint16_t*>(x);
+        a.dz = static_cast<const uint16_t*>(dz);
+        a.partial = scratch;
+        a.bias = gb ? scratch + size_t(plan.first[plan.groups]) * plan.part : nullptr;
+        a.batch = batch;
+        a.nrows = nrows;
+        a.ncols = ncols;
+        std::copy(plan.first, plan.first + 6, a.first);
+        a.error = error;
+        auto s = static_cast<cudaStream_t>(stream);
+        const int grid = plan.first[plan.groups];
+        cudaError_t e = cin == 32 ? (npad == 32 ? launch_wgrad<4, 32>(a, grid, g_attr_wgrad[0], s)
+                                                : launch_wgrad<4, 16>(a, grid, g_attr_wgrad[1], s))
+                                  : (npad == 32 ? launch_wgrad<2, 32>(a, grid, g_attr_wgrad[2], s)
+                                                : launch_wgrad<2, 16>(a, grid, g_attr_wgrad[3], s));
+        if (e == cudaSuccess)
+        {
+            WgradReduceArgs r{};
+            r.partial = a.partial;
+            r.bias_partial = a.bias;
+            std::copy(plan.first, plan.first + 6, r.first);
+            r.kpc = plan.kpc;
+            r.cin = cin;
+            r.npad = npad;
+            r.dw = dw;
+            r.gw = gw;
+            r.gb = gb;
+            r.cout = cout;
+            r.cin_used = cin_used;
+            const int total = 25 * cin * npad / 4;
+            wgrad_reduce_kernel<<<(total + 31) / 32 + (gb ? 1 : 0), 256, 0, s>>>(r);
+            e = cudaGetLastError();
+        }
+        return e == cudaSuccess ? AMB_OK : fail_cuda(name, e);
+    }
 }
 
 extern "C" size_t amb_conv5x5_wgrad_scratch_bytes(int batch, int nrows, int ncols, int cin, int npad)
 {
     if (!valid_geometry(batch, nrows, ncols)) return 0;
-    return size_t(wgrad_grid(batch, nrows, ncols)) * kTaps * cin * npad * sizeof(float);
+    return wgrad_plan(batch, nrows, ncols, cin, npad).bytes(npad);
 }
 
 extern "C" int amb_conv5x5_wgrad(const void* x, const void* dz, int batch, int nrows, int ncols, int cin, int npad,
                                  float* dw, float* scratch, size_t scratch_bytes, int* error, void* stream)
 {
-    if (!x || !dz || !dw || !scratch || !valid_geometry(batch, nrows, ncols) || (cin != 16 && cin != 32) ||
-        (npad != 16 && npad != 32))
-        return fail_invalid("amb_conv5x5_wgrad: need ncols % 128 == 0, nrows >= 3, cin and npad in {16, 32}");
-    if (scratch_bytes < amb_conv5x5_wgrad_scratch_bytes(batch, nrows, ncols, cin, npad))
-        return fail_invalid("amb_conv5x5_wgrad: scratch too small (see amb_conv5x5_wgrad_scratch_bytes)");
-    WgradArgs a{};
-    a.x = static_cast<const uint16_t*>(x);
-    a.dz = static_cast<const uint16_t*>(dz);
-    a.partial = scratch;
-    a.batch = batch;
-    a.nrows = nrows;
-    a.ncols = ncols;
-    a.cin_chunks = cin / 8;
-    a.npad = npad;
-    a.rows_per_cta = kWgradRows;
-    a.error = error;
-    const uint32_t smem = wg_smem_bytes(a.cin_chunks, npad, kWgradRows);
-    cudaError_t e = set_smem_attr(reinterpret_cast<const void*>(conv_wgrad_kernel),
-                                  std::max(wg_smem_bytes(4, 32, kWgradRows), wg_smem_bytes(2, 32, kWgradRows)),
-                                  g_attr_wgrad);
-    auto s = static_cast<cudaStream_t>(stream);
-    const long long grid = wgrad_grid(batch, nrows, ncols);
-    if (e == cudaSuccess)
-    {
-        conv_wgrad_kernel<<<unsigned(grid), kThreads, smem, s>>>(a);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess)
-    {
-        const int total = kTaps * cin * npad;
-        wgrad_reduce_kernel<<<(total + 255) / 256, 256, 0, s>>>(scratch, int(grid), total, dw);
-        e = cudaGetLastError();
-    }
-    return e == cudaSuccess ? AMB_OK : fail_cuda("amb_conv5x5_wgrad", e);
+    if (!dw) return fail_invalid("amb_conv5x5_wgrad: dw must not be NULL");
+    return param_grads("amb_conv5x5_wgrad", x, dz, batch, nrows, ncols, cin, npad, cin, npad, dw, nullptr, nullptr,
+                       scratch, scratch_bytes, error, stream);
+}
+
+extern "C" int amb_conv5x5_param_grads(const void* x, const void* dz, int batch, int nrows, int ncols, int cin, int npad,
+                                       int cin_used, int cout, float* gw, float* gb, float* scratch, size_t scratch_bytes,
+                                       int* error, void* stream)
+{
+    if (!gw) return fail_invalid("amb_conv5x5_param_grads: gw must not be NULL");
+    return param_grads("amb_conv5x5_param_grads", x, dz, batch, nrows, ncols, cin, npad, cin_used, cout, nullptr, gw, gb,
+                       scratch, scratch_bytes, error, stream);
+}
+
+extern "C" int amb_conv5x5_images(const float* w, int cout, int cin, int cin_pad, int npad, void* img, void* dimg,
+                                  void* stream)
+{
+    if (!w || (!img && !dimg) || cin < 1 || cout < 1 || cin > cin_pad || cout > npad || cin_pad % 8 || npad % 8)
+        return fail_invalid("amb_conv5x5_images: bad arguments");
+    const int n = 2 * 25 * cin_pad * npad;
+    weight_images_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        w, cout, cin, cin_pad, npad, static_cast<__nv_bfloat16*>(img), static_cast<__nv_bfloat16*>(dimg));
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? AMB_OK : fail_cuda("amb_conv5x5_images", e);
 }
 
 extern "C" int amb_learned_input(const float* phi, const float* params, int batch, int nrows, int ncols, void* x,

@@ -167,6 +167,17 @@ namespace tc
         for (int i = 16; i < 32; ++i) v[i] = 0.f;
     }
 
+    __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v)
+    {
+        uint32_t r[8];
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr)
+                     : "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+    }
+
     // Each thread of the warp writes zeros to 16 consecutive columns of its own TMEM lane.
     __device__ __forceinline__ void tmem_st16_zero(uint32_t taddr)
     {

@@ -333,6 +333,16 @@ size_t amb_conv5x5_wgrad_scratch_bytes(int batch, int nrows, int ncols, int cin,
 int amb_conv5x5_wgrad(const void* x, const void* dz, int batch, int nrows, int ncols, int cin, int npad, float* dw,
                       float* scratch, size_t scratch_bytes, int* error, void* stream);
 
+/* The parameter gradients of one layer in its weights' own layout: gw[cout][cin_used][5][5] as
+ * amb_conv5x5_wgrad sums it, and gb[npad] = sum over batch and sites of dz (NULL: not formed). Scratch
+ * as amb_conv5x5_wgrad. */
+int amb_conv5x5_param_grads(const void* x, const void* dz, int batch, int nrows, int ncols, int cin, int npad,
+                            int cin_used, int cout, float* gw, float* gb, float* scratch, size_t scratch_bytes,
+                            int* error, void* stream);
+/* bf16 operand images of weights w[cout][cin][5][5] (FP32): img for amb_conv5x5_forward with cin_pad input
+ * and npad output channels, dimg for its data gradient (npad input, cin_pad output); either may be NULL. */
+int amb_conv5x5_images(const float* w, int cout, int cin, int cin_pad, int npad, void* img, void* dimg, void* stream);
+
 /* Network input planes (16 channels, 2 chunks): bf16(phi), 256*(phi - bf16(phi)), zeta/4,
  * lambda, 10*T, zeros. phi: [batch][nrows][ncols] FP32; params: [batch][3] = (zeta, lambda, T). */
 int amb_learned_input(const float* phi, const float* params, int batch, int nrows, int ncols, void* x, void* stream);
