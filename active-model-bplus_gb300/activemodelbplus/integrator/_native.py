@@ -97,6 +97,8 @@ SIGNATURES = {
     "amb_ensemble_info": (_I, [_VP, ctypes.POINTER(_I64), _IP, _IP]),
     "amb_ensemble_form": (_I, [_VP, _I, _IP]),
     "amb_radial_spectrum": (_I, [_VP, _I, _I, ctypes.c_double, ctypes.c_double, _VP, _I, _VP, _VP, _VP]),
+    "amb_radial_rfft": (_I, [_VP, _I, _I, _I64, _I64, _I, ctypes.c_double, ctypes.c_double, ctypes.c_double, _VP, _I, _VP,
+                             _VP, _VP]),
     "amb_label_components_f64": (_I, [_VP, _I, _I, ctypes.c_double, _VP, _VP, _VP]),
     "amb_label_components_f32": (_I, [_VP, _I, _I, ctypes.c_double, _VP, _VP, _VP]),
     "amb_check_finite_f64": (_I, [_VP, _I64, _VP, _VP]),

@@ -281,6 +281,13 @@ int amb_ensemble_scatter(amb_ensemble* h, const float* src);
  * (nedges each) are zeroed first. */
 int amb_radial_spectrum(const double* power, int nrows, int ncols, double dx, double dy, const double* edges,
                         int nedges, double* sum, unsigned long long* count, void* stream);
+/* The same for a real field's transform (complex128, element strides row_stride and col_stride, 16-byte
+ * aligned): its rfft2 spectrum [nrows][ncols/2 + 1], or (packed, nrows even) the transform
+ * [nrows/2][ncols] of even rows + i odd rows. Bins |scale z|^2 over all nrows * ncols modes of the field,
+ * half of them through their symmetry. */
+int amb_radial_rfft(const void* spectrum, int nrows, int ncols, int64_t row_stride, int64_t col_stride, int packed,
+                    double scale, double dx, double dy, const double* edges, int nedges, double* sum,
+                    unsigned long long* count, void* stream);
 
 /* 4-connected components of {field > threshold} on the periodic grid (no reference
  * counterpart; the droplet count of the analysis). labels: nrows*ncols ints, set to the
