@@ -230,7 +230,6 @@ class Integrator:
         self._timestep = 0
         self._terms_step = None
         self._terms_dev = None
-        self._terms_host = None
         self._events = None  # optional (start, end) CUDA events recorded around the step launches
         self._s = N.stencil_struct(self._stencil)
         self._m = N.model_struct(self._model)
@@ -377,8 +376,8 @@ class Integrator:
         self._raise_if_flagged()
 
     # ------------------------------------------------------------- getters
-    def _terms(self) -> np.ndarray:
-        """The ten FP64 term planes at the current timestep, cached per timestep
+    def _terms(self):
+        """The ten FP64 term planes at the current timestep (device tensor), cached per timestep
         like the reference's lazy current recompute (src/integrator.cu:477-495)."""
         if self._terms_step != self._timestep:
             torch = _torch()
@@ -390,33 +389,17 @@ class Integrator:
             _check(fn(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
                       self._buf[self._cur].data_ptr(), self._timestep, None, self._terms_dev.data_ptr(),
                       self._stream()))
-            self._terms_host = self._terms_dev.cpu().numpy()
             self._terms_step = self._timestep
-        return self._terms_host
+        return self._terms_dev
 
     def _current(self, which: str):
-        t = self._terms()
-        out = []
-        for c in range(2):
-            jp, jl, jc, jr = t[2 + c], t[4 + c], t[6 + c], t[8 + c]
-            # sums in the reference's order (src/integrator.cu:406-465)
-            if which == "passive":
-                v = jp.copy()
-            elif which == "lambda":
-                v = jl.copy()
-            elif which == "circulating":
-                v = jc.copy()
-            elif which == "random":
-                v = jr.copy()
-            else:
-                active = jc + jl
-                if which == "active":
-                    v = active
-                else:
-                    det = active + jp
-                    v = det if which == "deterministic" else det + jr
-            out.append(v)
-        return out
+        """Fresh host copies of both components, summed on the device in the reference's order
+        (src/integrator.cu:406-465)."""
+        terms = self._terms()
+        out = _torch().empty((2, self._ny, self._nx), dtype=terms.dtype, device=terms.device)
+        _check(N.lib().amb_current_from_terms(terms.data_ptr(), self._ny, self._nx, N.CURRENTS[which], out.data_ptr(),
+                                              self._stream()))
+        return [v.cpu().numpy() for v in out]
 
     @property
     def current(self):
@@ -451,15 +434,15 @@ class Integrator:
     def chemical_potential(self) -> np.ndarray:
         """mu_p + mu_a (src/integrator.cu:385-388; not bound in the reference's module)."""
         t = self._terms()
-        return t[0] + t[1]
+        return (t[0] + t[1]).cpu().numpy()
 
     @property
     def passive_chemical_potential(self) -> np.ndarray:
-        return self._terms()[0].copy()
+        return self._terms()[0].cpu().numpy()
 
     @property
     def active_chemical_potential(self) -> np.ndarray:
-        return self._terms()[1].copy()
+        return self._terms()[1].cpu().numpy()
 
     # ---------------------------------------------------------- additions
     @property

@@ -85,6 +85,7 @@ SIGNATURES = {
                               ctypes.POINTER(ctypes.c_double)]),
     "amb_terms_f64": (_I, [_SP, _MP, _U64, _I, _I, _VP, _I64, _VP, _VP, _VP]),
     "amb_terms_f32": (_I, [_SP, _MP, _U64, _I, _I, _VP, _I64, _VP, _VP, _VP]),
+    "amb_current_from_terms": (_I, [_VP, _I, _I, _I, _VP, _VP]),
     "amb_mass_scratch_bytes": (ctypes.c_size_t, [_I64]),
     "amb_mass_f64": (_I, [_VP, _I64, _VP, _VP, ctypes.c_size_t, _VP]),
     "amb_mass_f32": (_I, [_VP, _I64, _VP, _VP, ctypes.c_size_t, _VP]),

@@ -335,6 +335,15 @@ extern "C" int amb_terms_f32(const amb_stencil* stencil, const amb_model* model,
     return e == cudaSuccess ? AMB_OK : cuda_fail(e, "amb_terms_f32");
 }
 
+extern "C" int amb_current_from_terms(const double* terms, int nrows, int ncols, int which, double* out, void* stream)
+{
+    if (int rc = check_shape(nrows, ncols)) return rc;
+    if (!terms || !out) return fail(AMB_ERR_INVALID, "terms and out must not be NULL");
+    if (which < AMB_CURRENT_TOTAL || which > AMB_CURRENT_RANDOM) return fail(AMB_ERR_INVALID, "unknown current");
+    cudaError_t e = amb::launch_current(terms, size_t(nrows) * ncols, which, out, as_stream(stream));
+    return e == cudaSuccess ? AMB_OK : cuda_fail(e, "amb_current_from_terms");
+}
+
 // ------------------------------------------------------------- reductions
 
 extern "C" size_t amb_mass_scratch_bytes(int64_t n)
@@ -406,9 +415,8 @@ struct amb_integrator
     void* workspace = nullptr;  // step workspace, allocated at the first run if there is room
     bool workspace_tried = false;
     double* stage = nullptr;  // float64 staging plane for FP32 fields, allocated on first transfer
-    double* terms = nullptr;  // AMB_NTERMS planes, allocated on first getter call
+    double* terms = nullptr;  // AMB_NTERMS planes and two of a current, allocated on first getter call
     int* flag = nullptr;
-    std::vector<double> host_terms;
 
     size_t n() const { return size_t(nrows) * ncols; }
     size_t elem() const { return precision == AMB_F64 ? sizeof(double) : sizeof(float); }
@@ -462,7 +470,7 @@ namespace
         if (h->terms_timestep == h->timestep) return AMB_OK;
         if (!h->terms)
         {
-            cudaError_t e = cudaMalloc(&h->terms, h->n() * AMB_NTERMS * sizeof(double));
+            cudaError_t e = cudaMalloc(&h->terms, h->n() * (AMB_NTERMS + 2) * sizeof(double));
             if (e != cudaSuccess) return fail(AMB_ERR_NOMEM, "terms buffer: " + std::string(cudaGetErrorString(e)));
         }
         int rc = h->precision == AMB_F64
@@ -471,16 +479,21 @@ namespace
                      : amb_terms_f32(&h->stencil, &h->model, h->seed, h->nrows, h->ncols,
                                      static_cast<const float*>(h->buf[h->cur]), h->timestep, nullptr, h->terms, h->stream);
         if (rc) return rc;
-        h->host_terms.resize(h->n() * AMB_NTERMS);
-        cudaError_t e = cudaMemcpyAsync(h->host_terms.data(), h->terms, h->n() * AMB_NTERMS * sizeof(double),
-                                        cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess) return cuda_fail(e, "terms readback");
         h->terms_timestep = h->timestep;
         return AMB_OK;
     }
 
-    const double* plane(const amb_integrator* h, int k) { return h->host_terms.data() + size_t(k) * h->n(); }
+    int read_plane(amb_integrator* h, const double* dev, double* host)
+    {
+        cudaError_t e = cudaMemcpyAsync(host, dev, h->n() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        return e == cudaSuccess ? AMB_OK : cuda_fail(e, "terms readback");
+    }
+
+    int wait_read(amb_integrator* h)
+    {
+        cudaError_t e = cudaStreamSynchronize(h->stream);
+        return e == cudaSuccess ? AMB_OK : cuda_fail(e, "terms readback");
+    }
 }
 
 extern "C" int amb_integrator_create(const double* host_field, int nrows, int ncols, const amb_stencil* stencil,
@@ -608,10 +621,17 @@ extern "C" int amb_integrator_get_chemical_potential(amb_integrator* h, int whic
     if (which < AMB_MU_TOTAL || which > AMB_MU_ACTIVE) return fail(AMB_ERR_INVALID, "unknown chemical potential");
     if (int rc = compute_terms(h)) return rc;
     const size_t n = h->n();
-    const double *mp = plane(h, 0), *ma = plane(h, 1);
-    for (size_t i = 0; i < n; ++i)
-        host_out[i] = which == AMB_MU_PASSIVE ? mp[i] : which == AMB_MU_ACTIVE ? ma[i] : mp[i] + ma[i];
-    return AMB_OK;
+    int rc = read_plane(h, h->terms + (which == AMB_MU_ACTIVE ? n : 0), host_out);
+    std::vector<double> active;
+    if (!rc && which == AMB_MU_TOTAL)
+    {
+        active.resize(n);
+        rc = read_plane(h, h->terms + n, active.data());
+    }
+    if (!rc) rc = wait_read(h);
+    if (!rc)
+        for (size_t i = 0; i < active.size(); ++i) host_out[i] += active[i];
+    return rc;
 }
 
 extern "C" int amb_integrator_get_current(amb_integrator* h, int which, double* host_y, double* host_x)
@@ -620,30 +640,11 @@ extern "C" int amb_integrator_get_current(amb_integrator* h, int which, double* 
     if (which < AMB_CURRENT_TOTAL || which > AMB_CURRENT_RANDOM) return fail(AMB_ERR_INVALID, "unknown current");
     if (int rc = compute_terms(h)) return rc;
     const size_t n = h->n();
-    double* out[2] = {host_y, host_x};
-    for (int c = 0; c < 2; ++c)
-    {
-        const double *jp = plane(h, 2 + c), *jl = plane(h, 4 + c), *jc = plane(h, 6 + c), *jr = plane(h, 8 + c);
-        for (size_t i = 0; i < n; ++i)
-        {
-            // Sums in the reference's order (src/integrator.cu:406-465).
-            double active = jc[i] + jl[i];
-            double det = active + jp[i];
-            double v = 0;
-            switch (which)
-            {
-            case AMB_CURRENT_TOTAL: v = det + jr[i]; break;
-            case AMB_CURRENT_DETERMINISTIC: v = det; break;
-            case AMB_CURRENT_PASSIVE: v = jp[i]; break;
-            case AMB_CURRENT_ACTIVE: v = active; break;
-            case AMB_CURRENT_LAMBDA: v = jl[i]; break;
-            case AMB_CURRENT_CIRCULATING: v = jc[i]; break;
-            default: v = jr[i]; break;
-            }
-            out[c][i] = v;
-        }
-    }
-    return AMB_OK;
+    double* planes = h->terms + AMB_NTERMS * n;
+    int rc = amb_current_from_terms(h->terms, h->nrows, h->ncols, which, planes, h->stream);
+    if (!rc) rc = read_plane(h, planes, host_y);
+    if (!rc) rc = read_plane(h, planes + n, host_x);
+    return rc ? rc : wait_read(h);
 }
 
 extern "C" int amb_integrator_get_timestep(const amb_integrator* h, int64_t* out)

@@ -73,6 +73,8 @@ namespace amb
     cudaError_t launch_terms(const Real* phi, double* out, const StepParams& p, int noise_mode, const Real* injected,
                              cudaStream_t stream);
 
+    cudaError_t launch_current(const double* terms, size_t n, int which, double* out, cudaStream_t stream);
+
     int mass_partials(size_t n);
     template <typename Real>
     cudaError_t launch_mass(const Real* f, size_t n, double* out, double* scratch, int nparts, cudaStream_t stream);

@@ -94,6 +94,30 @@ namespace amb
         }
     }
 
+    // One current from the term planes, summed in the reference's order (src/integrator.cu:406-465).
+    __device__ __forceinline__ double current_of(int which, double jp, double jl, double jc, double jr)
+    {
+        const double active = __dadd_rn(jc, jl);
+        const double det = __dadd_rn(active, jp);
+        switch (which)
+        {
+        case AMB_CURRENT_TOTAL: return __dadd_rn(det, jr);
+        case AMB_CURRENT_DETERMINISTIC: return det;
+        case AMB_CURRENT_PASSIVE: return jp;
+        case AMB_CURRENT_ACTIVE: return active;
+        case AMB_CURRENT_LAMBDA: return jl;
+        case AMB_CURRENT_CIRCULATING: return jc;
+        default: return jr;
+        }
+    }
+
+    // Both components of a current from the ten planes: the host reads two planes instead of ten.
+    __global__ void current_kernel(const double* __restrict__ terms, size_t n, int which, double* __restrict__ out)
+    {
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < 2 * n; i += (size_t)gridDim.x * blockDim.x)
+            out[i] = current_of(which, terms[2 * n + i], terms[4 * n + i], terms[6 * n + i], terms[8 * n + i]);
+    }
+
     static int grid_for(size_t n, int block)
     {
         size_t g = (n + block - 1) / block;
@@ -108,6 +132,12 @@ namespace amb
         int g = grid_for(n, 256);
         terms_local_kernel<Real><<<g, 256, 0, stream>>>(phi, out, p, noise_mode, injected);
         terms_currents_kernel<<<g, 256, 0, stream>>>(out, p);
+        return cudaGetLastError();
+    }
+
+    cudaError_t launch_current(const double* terms, size_t n, int which, double* out, cudaStream_t stream)
+    {
+        current_kernel<<<grid_for(2 * n, 256), 256, 0, stream>>>(terms, n, which, out);
         return cudaGetLastError();
     }
 

@@ -218,6 +218,9 @@ int amb_terms_f64(const amb_stencil* stencil, const amb_model* model, uint64_t s
                   const double* field, int64_t step, const double* injected_noise, double* out, void* stream);
 int amb_terms_f32(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
                   const float* field, int64_t step, const float* injected_noise, double* out, void* stream);
+/* A current (AMB_CURRENT_*) from the planes amb_terms_* wrote: out gets nrows*ncols values of its y
+ * component, then of its x component, summed in the reference's order (src/integrator.cu:406-465). */
+int amb_current_from_terms(const double* terms, int nrows, int ncols, int which, double* out, void* stream);
 
 /* FP64 compensated sum of a device field into out_sum (one double, device memory).
  * scratch: device memory of at least amb_mass_scratch_bytes(n) bytes. */
