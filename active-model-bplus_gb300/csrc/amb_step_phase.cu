@@ -1,5 +1,7 @@
-// Launcher of the three-phase step kernel (amb_step_phase.cuh).
+// Launcher of the FP64 step kernels: one tile per SM for small grids (amb_step_dtile.cuh), three
+// grid-wide phases for the others (amb_step_phase.cuh).
 #include "amb_kernels.h"
+#include "amb_step_dtile.cuh"
 #include "amb_step_phase.cuh"
 
 #include <algorithm>
@@ -15,6 +17,7 @@ namespace amb
         // Sites x steps of one launch, about half a second of FP64 work, so that a long run stays a
         // queue of launches.
         constexpr double kLaunchWork = 4e9;
+        constexpr size_t kTileSmem = size_t(200) << 10;
 
         template <typename Real>
         size_t workspace_bytes(int ny, int nx, int* band)
@@ -36,6 +39,46 @@ namespace amb
             const int nb = int((size_t(ny) + rows - 2 * phase::kBandHalo - 1) / (rows - 2 * phase::kBandHalo));
             *band = (ny + nb - 1) / nb;  // even bands
             return phase::kHeader + row * (*band + 2 * phase::kBandHalo);
+        }
+    }
+
+    namespace
+    {
+        // FP64 warp instructions of one step of a tile, as its lists are packed (runs of about one item per
+        // thread), plus what the barriers and the halo load cost beside them.
+        double tile_cost(int ty, int tx)
+        {
+            const auto list = [](int w, int h, double per_site, double per_run) {
+                const int l = std::max(1, w * h / dtile::kThreads), items = w * ((h + l - 1) / l);
+                return double((items + 31) / 32) * (l * per_site + per_run);
+            };
+            return list(tx + 4, ty + 4, 25, 4) + list(2 * tx, 6, 11, 2) + list(12, ty, 11, 2) + list(tx + 2, ty + 2, 9, 8)
+                   + list(tx, ty + 8, 9, 0) + list(tx + 8, ty, 9, 0) + list(tx, ty, 9, 8) + 2 * list(tx, ty, 8, 0)
+                   + list(tx, ty, 3, 0);
+        }
+
+        // The tile shape that spreads a grid over the SMs, one tile each, at the least cost (64^2: 4 x 8, 6.4 us;
+        // 1 x 64 12.3). False above 400 sites per SM, where the halo costs more than two grid barriers (us per
+        // step, tiles and phases: 128^2 9.3 and 13.2, 200 x 300 18.8 and 20.1, 256^2 19.9 and 20.0, 350^2 35.8
+        // and 29.5).
+        bool tile_shape(int ny, int nx, int sms, dtile::Shape* best)
+        {
+            double least = 1e300;
+            if (double(ny) * nx > 400.0 * sms) return false;
+            for (int tx : {8, 12, 16, 24, 32, 48})
+            {
+                const int across = (nx + tx - 1) / tx, down = sms / across;
+                if (down < 1) continue;
+                const dtile::Shape t{std::max(1, (ny + down - 1) / down), tx};
+                if (t.doubles() * sizeof(double) > kTileSmem) continue;
+                const double cost = tile_cost(t.ty, t.tx);
+                if (cost < least)
+                {
+                    least = cost;
+                    *best = t;
+                }
+            }
+            return least < 1e300;
         }
     }
 
@@ -65,6 +108,20 @@ namespace amb
                 if (dev < 64) sms_of[dev] = sms;
             }
         }
+        dtile::Shape tile{};
+        const bool small = tile_shape(p.ny, p.nx, sms, &tile);
+        if (small)
+        {
+            static std::mutex attr_mutex;
+            static bool configured[64];
+            std::lock_guard<std::mutex> lock(attr_mutex);
+            if (dev >= 64 || !configured[dev])
+            {
+                e = cudaFuncSetAttribute(dtile::step_dtile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileSmem));
+                if (e != cudaSuccess) return e;
+                if (dev < 64) configured[dev] = true;
+            }
+        }
         int band = 0;
         workspace_bytes<double>(p.ny, p.nx, &band);
         const phase::Coef k(p);
@@ -79,6 +136,17 @@ namespace amb
             double* in = (done & 1) ? b : a;
             double* out = (done & 1) ? a : b;
             int m = n;
+            if (small)
+            {
+                const int tiles = ((p.ny + tile.ty - 1) / tile.ty) * ((p.nx + tile.tx - 1) / tile.tx);
+                unsigned* count = static_cast<unsigned*>(workspace);
+                void* args[] = {&in, &out, &count, &pp, const_cast<phase::Coef*>(&k), &tile, &noise_mode, &inj, &m};
+                e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(dtile::step_dtile_kernel), dim3(tiles),
+                                                dim3(dtile::kThreads), args, tile.doubles() * sizeof(double), stream);
+                if (e != cudaSuccess) return e;
+                done += n;
+                continue;
+            }
             void* args[] = {&in, &out, &workspace, &pp, const_cast<phase::Coef*>(&k), &noise_mode, &inj, &m, &band};
             e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(phase::step_phase_kernel<double>), dim3(sms),
                                             dim3(phase::kThreads), args, 0, stream);

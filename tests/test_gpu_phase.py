@@ -1,4 +1,5 @@
-"""The three-phase FP64 step kernel (amb_step_f64_ws) against the oracle and the tile kernel."""
+"""The FP64 step kernels behind amb_step_f64_ws (one tile per SM on small grids, three grid-wide phases
+on the others) against the oracle and the tile kernel."""
 import ctypes
 
 import numpy as np
@@ -8,9 +9,10 @@ import oracle
 from activemodelbplus.integrator import Integrator, Model, Stencil
 from activemodelbplus.integrator import _native as N
 
-# one site, grids narrower than the stencils, blocks of 32 columns with and without remainder, more
-# rows than warps and fewer
-SHAPES = [(1, 1), (2, 7), (9, 31), (33, 64), (65, 33), (20, 257), (300, 40)]
+# tiles: one site, grids narrower than the stencils and than a tile, partial tiles, tall and wide grids;
+# phases: blocks of 32 columns with and without remainder, more rows than warps and fewer
+SHAPES = [(1, 1), (2, 7), (9, 31), (33, 64), (65, 33), (20, 257), (300, 40), (6000, 9), (3, 15000),
+          (250, 260), (11, 7001), (20000, 7)]
 
 
 def _params(T):
