@@ -129,11 +129,12 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
     {
         // Segment heights that put m tasks on each SM: a task costs its rows plus about eight rows of
         // pipeline fill, so the best height is one whose task count just fills the SMs, with as many
-        // resident tasks as pay for their fill (1536^2: 24 rows, 30.8 us; 16 and 32 rows 37).
+        // resident tasks as pay for their fill (1536^2: 24 rows, 30.8 us; 16 and 32 rows 37). Heights are even:
+        // a warp pair takes two rows per round.
         const int strips = (ncols + 111) / 112;
         const auto rows_for = [&](int m) {
             const int segs = std::max(1, std::min(nrows, sms * m / strips));
-            return (nrows + segs - 1) / segs;
+            return ((nrows + segs - 1) / segs + 1) & ~1;
         };
         const auto add = [&](std::initializer_list<int> ms, int pairs, int flags) {
             std::vector<int> rows{0};

@@ -45,7 +45,6 @@ namespace amb
                                         const StepParams& p, int noise_mode, const float* injected, int variant,
                                         cudaStream_t stream);
     bool step_f32_sliding_supported(int ny, int nx, int variant);
-    int sliding_default_seg_h(int ny, int nx);
 
     // ------------------------------------------------------------- ensemble
     // One replica of a batched ensemble (device array of these, filled by the host).
@@ -62,7 +61,6 @@ namespace amb
     };
     size_t sliding_coef_bytes();
     void sliding_make_coef(const StepParams& p, void* out);  // host: per-replica coefficient block
-    int sliding_default_seg_h_for(int ny, int nx, int resident_pairs);
     // fused: one warp per task running every stage (otherwise a producer/consumer warp pair).
     cudaError_t launch_sliding_ensemble(const EnsembleReplica* reps, const void* coefs, const EnsembleTask* tasks,
                                         int ntasks, int parity, const int64_t* step_counter, int step_offset,

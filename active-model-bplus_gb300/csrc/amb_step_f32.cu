@@ -1,13 +1,13 @@
 // Register-sliding FP32 step kernel: the FP32 performance path.
 //
 // Work decomposition: a strip of 128 computed columns (4 per lane) whose middle 112 are its
-// output slides down a segment of rows, one row per round. A producer and a consumer warp share
-// the round's work and meet at one named barrier (or, in the fused form, one warp does it all);
+// output slides down a segment of rows, two rows per round (one in the fused form). A producer and a consumer warp
+// share the round and meet at one named barrier (or, in the fused form, one warp does it all);
 // x-neighbours come from warp shuffles (radius 1) or a shared-memory row (radius 4), and the
 // y-direction order-8 stencils (D8_y o D8_y of the passive current, radius 8) read shared-memory
 // rings of the rows held per lane.
 //
-// Round k:
+// For row k:
 //   stage A (row k)     lap, grad phi, mu_p, mu_a, zeta*lap*grad phi from phi rows k-1..k+1   (producer)
 //   J1_y   (row k-4)    -D8_y mu_p + mag xi_y                      mu_p ring, rows k-8..k     (producer)
 //   DY8    (row k-8)    D8_y J1_y                                  J1_y ring                  (producer)
@@ -16,17 +16,17 @@
 //   output (row k-8)    J1_x = -D8_x mu_p + mag xi_x, DX8 = D8_x J1_x (row exchange),
 //                       div J = DX8 + DY8 + divTj (delayed 6 rows), compensated update.       (consumer)
 //
-// Bound by instruction issue and the shared-memory pipe: 195 issue slots per output site and 159
-// wavefronts per round (80 % of the pipe's peak at T = 0). All arithmetic runs on packed pairs of
-// columns, with the constants read as pairs from the constant bank; odd x offsets of D8, whose
-// pairs are not aligned, are differenced as scalars. The phi rows are plain 16-byte loads, one row
-// ahead, with an L2 prefetch: staging them in shared memory by bulk copies cost the issue slots
-// of the copies, mbarrier waits and row reads, and 9 KB per pair. us per step at 4096^2,
-// f32c: 137.7 at T = 0.05 and 108.8 at T = 0 (bulk copies, scalar x stencils and per-row ring selects
-// before: 182.9 and 144.4, 260 slots per site). Other splits measured at 4096^2, T = 0.05: rings as register windows
-// 164 (spills at 16 warps per SM), the Tjhung chain moved to the producer 148, three warps per strip 174,
-// producer and consumer two rounds apart on split barriers 133 (but 119 at T = 0, and half the CTAs fit
-// in the one-pair form), main loops unrolled by 2 or 3 136-142 and 109-122 at T = 0.
+// Bound by the FP32 and integer pipes and what latency 16 warps leave uncovered: 186 issue slots per output
+// site, 62 % of the issue slots and 54 % of the shared-memory pipe in use. All arithmetic runs on packed
+// pairs of columns, with the constants read as pairs from the constant bank; odd x offsets of D8, whose
+// pairs are not aligned, are differenced as scalars. Two rows per round share each D8_y window: 8 row
+// reads per ring for two rows instead of 15, no mirrored ring rows, half the barriers. The phi rows are
+// plain 16-byte loads, one row ahead, with an L2 prefetch. us per step at 4096^2, f32c, T = 0.05 and T = 0,
+// 4 pairs per CTA: 132 and 98 (one row per round, mirrored rings: 138 and 109; bulk copies, scalar x
+// stencils and per-row ring selects: 183 and 144). Other splits measured there at T = 0.05 against 138: rings
+// as register windows 164 (spills at 16 warps per SM), the Tjhung chain moved to the producer 148, three
+// warps per strip 174, producer and consumer two rounds apart on split barriers 133 (119 at T = 0, and half
+// the CTAs fit in the one-pair form).
 //
 // Requirements (checked by step_f32_sliding_supported): ncols % 4 == 0 and
 // ncols >= 112 (one strip's output width); any nrows >= 1.
@@ -51,21 +51,26 @@ namespace amb
         constexpr int kHalo = 8;                // mu_p halo on each side
         constexpr int kOut = kCols - 2 * kHalo; // 112 output columns per warp
         constexpr int kDelay = 6;               // rounds from divTj of a row to its output
-        constexpr int kMupRing = 10;            // mu_p rows k-9..k: 9 in use + 1 the producer fills while the consumer reads
-        constexpr int kJ1Ring = 9;              // J1_y rows k-12..k-4: the 9 rows of one D8_y
+        constexpr int kMupRing = 10;            // fused form: mu_p rows k-9..k (mirrored)
+        constexpr int kJ1Ring = 9;              // fused form: J1_y rows k-12..k-4, the 9 rows of one D8_y (mirrored)
 
-        // The y rings are written in two places, N rows apart, so that a window of rows is contiguous
-        // wherever it starts: its rows are constant offsets from one base.
+        constexpr int kPairMup = 16;  // mu_p rows k-8..k+1 in use and the two the producer fills meanwhile
+        constexpr int kPairJ1 = 8;    // J1_y rows k-12..k-5 (rows k-4, k-3 replace the oldest two once they are read)
+
+        // What a warp pair shares. A round takes two rows, so the rings advance by two rows and a window is
+        // four row pairs, each contiguous.
         struct __align__(16) PairSmem
         {
-            float mup[2 * kMupRing][kCols];  // producer writes row k, D8_y reads k-8..k-1, consumer reads k-8
-            float j1y[2 * kJ1Ring][kCols];   // producer only
-            float hand[2][4][kCols];         // producer -> consumer rows: mu_a(k), J_c,y(k), J_c,x(k), DY8(k-8)
-            float dtj[kDelay][kCols];        // divTj rows k-8..k-3 (consumer only)
-            float xch[2][kCols];             // J1_x row exchange of the consumer's lanes
+            float mup[kPairMup][kCols];   // row r at (r - 1) mod 16
+            float j1y[kPairJ1][kCols];    // row r at (r - 1) mod 8 (producer only)
+            float hand[2][2][4][kCols];   // producer -> consumer, by round and row: mu_a(k), J_c,y(k), J_c,x(k), DY8(k-8)
+            float dtj[kDelay][kCols];     // divTj rows k-8..k-3 (consumer only)
+            float xch[2][2][kCols];       // J1_x row exchange of the consumer's lanes
         };
 
-        // Shared memory of one warp that runs every stage of its strip (the fused form).
+        // Shared memory of one warp that runs every stage of its strip (the fused form). The y rings are
+        // written in two places, N rows apart, so that a window of rows is contiguous wherever it starts:
+        // its rows are constant offsets from one base.
         struct __align__(16) WarpSmem
         {
             float mup[2 * kMupRing][kCols];
@@ -75,7 +80,7 @@ namespace amb
         };
 
         // Rows are read one round ahead of use, which covers the L2's latency; the DRAM's is covered by a
-        // prefetch into the L2 some rows earlier (4096^2: 136.6 us with it, 146.1 without).
+        // prefetch into the L2 some rows earlier (4096^2, one row per round: 136.6 us with it, 146.1 without).
         constexpr int kPrefetch = 4;
         __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -256,176 +261,231 @@ namespace amb
             }
         };
 
-        // J1_x, DX8, the update and the stores of the output rows.
-        template <int COMP, int NOISE>
+        // J1_x, DX8, the update and the stores of the output rows, R rows at a time.
+        template <int COMP, int NOISE, int R>
         struct Output
         {
             const float* phi_in;
             float* phi_out;
             __nv_bfloat16* residual;
             const float* injected;
-            float* xch;      // this warp's two exchange rows
-            int ny, nx, gcol, grow, lane, flip = 0;
+            float* xch;       // this lane's columns of the warp's exchange rows, two sets of R
+            int ny, nx, gcol, grow, last, flip = 0;
             int left, right;  // offsets of the neighbouring quads in a shared row (within it at its ends)
             bool store;
-            Quad xi;         // noise of the next output row, drawn one round ahead
-            float4 fnext;    // phi and residual of the next output row
-            uint2 rnext;
+            float4 fnext[R];  // phi and residual of the next output rows
+            uint2 rnext[R];
 
-            __device__ __forceinline__ void ahead(const StepParams& p, const Coef& k)
+            // Output rows don't wrap; a row past the segment's last is computed from rows in range and not stored.
+            __device__ __forceinline__ int at(int j) const { return R == 1 ? min(grow, ny - 1) : min(grow + j, ny - 1); }
+            __device__ __forceinline__ void ahead()
             {
-                xi = normals<NOISE>(p, k, injected, grow, gcol, 1);
-                const size_t i = (size_t)grow * nx + gcol;
-                fnext = *reinterpret_cast<const float4*>(phi_in + i);
-                if constexpr (COMP == COMP_BF16)
+#pragma unroll
+                for (int j = 0; j < R; ++j)
                 {
-                    rnext = *reinterpret_cast<const uint2*>(residual + i);
-                    prefetch_l2(residual + (grow + kPrefetch < ny ? i + (size_t)kPrefetch * nx : i));
+                    const int r = at(j);
+                    const size_t i = (size_t)r * nx + gcol;
+                    fnext[j] = *reinterpret_cast<const float4*>(phi_in + i);
+                    if constexpr (COMP == COMP_BF16)
+                    {
+                        rnext[j] = *reinterpret_cast<const uint2*>(residual + i);
+                        prefetch_l2(residual + (r + kPrefetch < ny ? i + (size_t)kPrefetch * nx : i));
+                    }
                 }
             }
             __device__ __forceinline__ Output(const float* in, float* out, __nv_bfloat16* res, const float* inj, float* x,
-                                              int ny_, int nx_, const Task& t, int lane_)
-                : phi_in(in), phi_out(out), residual(res), injected(inj), xch(x), ny(ny_), nx(nx_), grow(t.r0), lane(lane_)
+                                              int ny_, int nx_, const Task& t, int lane)
+                : phi_in(in), phi_out(out), residual(res), injected(inj), xch(x + 4 * lane), ny(ny_), nx(nx_), grow(t.r0),
+                  last(t.r1)
             {
                 const int scol = t.c0 - 8 + 4 * lane;
                 gcol = wrap_index(scol, nx);
                 store = lane >= 2 && lane < 30 && scol >= t.store_lo && scol < nx;
                 left = lane == 0 ? 0 : -4;
                 right = lane == 31 ? 0 : 4;
-                rnext = make_uint2(0u, 0u);
             }
-            // row grow, given its mu_p row (this lane's columns of a shared row), divTj and DY8
-            __device__ __forceinline__ void row(const StepParams& p, const Coef& k, const float* mup, Quad dtj, Quad dy8)
+            // rows grow .. grow + R - 1, given their consecutive mu_p rows (this lane's columns of shared rows),
+            // divTj and DY8
+            __device__ __forceinline__ void rows(const StepParams& p, const Coef& k, const float* mup, const Quad (&dtj)[R],
+                                                 const Quad (&dy8)[R])
             {
-                const Quad x = xi, f = quad(fnext);
-                const uint2 rv = rnext;
-                const size_t gi = (size_t)grow * nx + gcol;
-                grow = grow + 1 == ny ? 0 : grow + 1;
-                ahead(p, k);
-                const Quad j1x = fma4(k.mag, x, d8x(k.nx8, load_quad(mup + left), load_quad(mup), load_quad(mup + right)));
-                float* e = xch + flip * kCols + 4 * lane;
+                float* e = xch + flip * R * kCols;
                 flip ^= 1;
-                store_quad(e, j1x);
-                __syncwarp();  // the other row is rewritten only after the next round's
-                const Quad div = d8x(k.px8, load_quad(e + left), j1x, load_quad(e + right)) + (dtj + dy8);
-                if constexpr (COMP == COMP_BF16)
+                Quad j1x[R], f[R];
+                uint2 rv[R];
+#pragma unroll
+                for (int j = 0; j < R; ++j)
                 {
-                    const Quad rr{make_float2(__uint_as_float(rv.x << 16), __uint_as_float(rv.x & 0xffff0000u)),
-                                  make_float2(__uint_as_float(rv.y << 16), __uint_as_float(rv.y & 0xffff0000u))};
-                    const Quad F = fma4(k.dt, div, rr);
-                    const Quad nf = f - F;
-                    const Quad nr = (nf - f) + F;
-                    if (store)
-                    {
-                        store_quad(phi_out + gi, nf);
-                        __nv_bfloat162 lo = __floats2bfloat162_rn(nr.a.x, nr.a.y), hi = __floats2bfloat162_rn(nr.b.x, nr.b.y);
-                        uint2 w;
-                        w.x = *reinterpret_cast<uint32_t*>(&lo);
-                        w.y = *reinterpret_cast<uint32_t*>(&hi);
-                        *reinterpret_cast<uint2*>(residual + gi) = w;
-                    }
+                    const float* m = mup + j * kCols;
+                    const Quad xi = normals<NOISE>(p, k, injected, at(j), gcol, 1);
+                    j1x[j] = fma4(k.mag, xi, d8x(k.nx8, load_quad(m + left), load_quad(m), load_quad(m + right)));
+                    store_quad(e + j * kCols, j1x[j]);
+                    f[j] = quad(fnext[j]);
+                    if constexpr (COMP == COMP_BF16) rv[j] = rnext[j];
                 }
-                else if (store)
-                    store_quad(phi_out + gi, fma4(k.ndt, div, f));
+                const int row = grow;
+                grow += R;
+                ahead();
+                __syncwarp();  // the other set is rewritten only after the next round's
+#pragma unroll
+                for (int j = 0; j < R; ++j)
+                {
+                    const Quad div = d8x(k.px8, load_quad(e + j * kCols + left), j1x[j], load_quad(e + j * kCols + right))
+                                   + (dtj[j] + dy8[j]);
+                    const size_t gi = (size_t)(row + j) * nx + gcol;
+                    const bool st = store && (j == 0 || row + j < last);
+                    if constexpr (COMP == COMP_BF16)
+                    {
+                        const Quad rr{make_float2(__uint_as_float(rv[j].x << 16), __uint_as_float(rv[j].x & 0xffff0000u)),
+                                      make_float2(__uint_as_float(rv[j].y << 16), __uint_as_float(rv[j].y & 0xffff0000u))};
+                        const Quad F = fma4(k.dt, div, rr);
+                        const Quad nf = f[j] - F;
+                        const Quad nr = (nf - f[j]) + F;
+                        if (st)
+                        {
+                            store_quad(phi_out + gi, nf);
+                            __nv_bfloat162 lo = __floats2bfloat162_rn(nr.a.x, nr.a.y),
+                                           hi = __floats2bfloat162_rn(nr.b.x, nr.b.y);
+                            uint2 w;
+                            w.x = *reinterpret_cast<uint32_t*>(&lo);
+                            w.y = *reinterpret_cast<uint32_t*>(&hi);
+                            *reinterpret_cast<uint2*>(residual + gi) = w;
+                        }
+                    }
+                    else if (st)
+                        store_quad(phi_out + gi, fma4(k.ndt, div, f[j]));
+                }
             }
         };
 
-        // Producer warp: stage A, the mu_p ring, J1_y with its noise, and DY8. Rounds 1..6 feed no divTj row
-        // that an output reads, rounds 1..8 no J1_y row and rounds 1..16 no DY8 row: they run the body
-        // without those parts (the first six without a hand-off).
+        // The windows of a round that takes rows k and k+1: rows w[0..7] = r-8..r-1 of a ring before its rows r = n0
+        // and r+1 = n1; D8 along y centred on rows r-4 and r-3.
+        template <int N>
+        __device__ __forceinline__ void d8y_two(const float2 (&c)[4], const float* ring, int row, Quad n0, Quad n1, Quad& d0,
+                                                Quad& d1)
+        {
+            Quad w[8];
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+            {
+                const float* q = ring + ((row + 2 * p) & (N - 1)) * kCols;
+                w[2 * p] = load_quad(q);
+                w[2 * p + 1] = load_quad(q + kCols);
+            }
+            d0 = c[0] * (w[5] - w[3]);
+            d0 = fma4(c[1], w[6] - w[2], d0);
+            d0 = fma4(c[2], w[7] - w[1], d0);
+            d0 = fma4(c[3], n0 - w[0], d0);
+            d1 = c[0] * (w[6] - w[4]);
+            d1 = fma4(c[1], w[7] - w[3], d1);
+            d1 = fma4(c[2], n0 - w[2], d1);
+            d1 = fma4(c[3], n1 - w[1], d1);
+        }
+
+        // Producer warp: stage A, the mu_p ring, J1_y with its noise, and DY8, two rows per round: round q takes
+        // rows k = 2q + 1 and k + 1. Rows 1..6 feed no divTj row that an output reads, rows 1..8 no J1_y row and
+        // rows 1..16 no DY8 row: their rounds run the body without those parts (the first three without a hand-off).
         template <int NOISE>
         __device__ __forceinline__ void producer(PairSmem& sm, const float* __restrict__ phi_in, const StepParams& p,
                                                  const Coef& k, const float* __restrict__ injected, const Task& t,
                                                  int lane, int bar_id)
         {
-            const int total = t.r1 - t.r0 + 16;   // rounds kl = 1 .. H + 16
+            const int rounds = (t.r1 - t.r0 + 17) / 2;
             Local loc(phi_in, p.ny, p.nx, t, lane);
-            Passive pas{&sm.mup[0][4 * lane], &sm.j1y[0][4 * lane]};
-            float* hand = &sm.hand[1][0][4 * lane];
-            Quad xi = zero_quad();  // xi_y of this round's J1_y row, formed one round ahead
-            int nrow = 0;           // global row of the next round's
+            float *mup = &sm.mup[0][4 * lane], *j1y = &sm.j1y[0][4 * lane], *hands = &sm.hand[0][0][0][4 * lane];
+            int nrow = wrap_index(t.r0 - 4, p.ny);  // global row of the next J1_y row
             const auto draw = [&]() {
-                xi = normals<NOISE>(p, k, injected, nrow, loc.gcol, 0);
+                const Quad z = normals<NOISE>(p, k, injected, nrow, loc.gcol, 0);
                 nrow = nrow + 1 == p.ny ? 0 : nrow + 1;
+                return z;
             };
-            const auto round = [&](auto hand_tag, auto j1_tag, auto dy_tag) {
+            const auto round = [&](int q, auto hand_tag, auto j1_tag, auto dy_tag) {
                 constexpr bool HAND = decltype(hand_tag)::value, J1 = decltype(j1_tag)::value, DY = decltype(dy_tag)::value;
-                Quad mup, mua, jcy, jcx;
-                loc.step(k, mup, mua, jcy, jcx);
-                const float* w = pas.put_mup(mup);
-                if constexpr (HAND)
+                float* hand = hands + (q & 1) * 8 * kCols;
+                Quad m[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
                 {
-                    store_quad(hand, mua);
-                    store_quad(hand + kCols, jcy);
-                    store_quad(hand + 2 * kCols, jcx);
+                    Quad mua, jcy, jcx;
+                    loc.step(k, m[i], mua, jcy, jcx);
+                    store_quad(mup + ((2 * q + i) & (kPairMup - 1)) * kCols, m[i]);
+                    if constexpr (HAND)
+                    {
+                        store_quad(hand + 4 * i * kCols, mua);
+                        store_quad(hand + (4 * i + 1) * kCols, jcy);
+                        store_quad(hand + (4 * i + 2) * kCols, jcx);
+                    }
                 }
                 if constexpr (J1)
                 {
-                    const Quad x = xi;
-                    draw();  // now, so that its Philox chain overlaps this round
-                    const Quad j1y = fma4(k.mag, x, Passive::d8y(k.ny8, w, mup));
-                    const float* v = pas.put_j1y(j1y);
-                    if constexpr (DY) store_quad(hand + 3 * kCols, Passive::d8y(k.py8, v, j1y));
+                    const Quad x0 = draw(), x1 = draw();
+                    Quad s0, s1;
+                    d8y_two<kPairMup>(k.ny8, mup, 2 * q - 8, m[0], m[1], s0, s1);
+                    const Quad j0 = fma4(k.mag, x0, s0), j1 = fma4(k.mag, x1, s1);
+                    if constexpr (DY)
+                    {
+                        Quad d0, d1;
+                        d8y_two<kPairJ1>(k.py8, j1y, 2 * q + 4, j0, j1, d0, d1);
+                        store_quad(hand + 3 * kCols, d0);
+                        store_quad(hand + 7 * kCols, d1);
+                    }
+                    float* o = j1y + ((2 * q + 4) & (kPairJ1 - 1)) * kCols;  // where rows k-12, k-11 were
+                    store_quad(o, j0);
+                    store_quad(o + kCols, j1);
                 }
-                if constexpr (HAND)
-                {
-                    hand = hand == &sm.hand[1][0][4 * lane] ? &sm.hand[0][0][4 * lane] : &sm.hand[1][0][4 * lane];
-                    pair_sync(bar_id);
-                }
+                if constexpr (HAND) pair_sync(bar_id);
             };
             using F = std::false_type;
             using T = std::true_type;
+            int q = 0;
 #pragma unroll 1
-            for (int kl = 1; kl <= 6; ++kl) round(F{}, F{}, F{});
-            round(T{}, F{}, F{});
-            round(T{}, F{}, F{});
-            nrow = wrap_index(t.r0 - 4, p.ny);  // J1_y rows from local row 5 (round 9) on
-            draw();
+            for (; q < 3; ++q) round(q, F{}, F{}, F{});
+            round(q++, T{}, F{}, F{});
 #pragma unroll 1
-            for (int kl = 9; kl <= 16; ++kl) round(T{}, T{}, F{});
+            for (; q < 8; ++q) round(q, T{}, T{}, F{});
 #pragma unroll 1
-            for (int kl = 17; kl <= total; ++kl) round(T{}, T{}, T{});
+            for (; q < rounds; ++q) round(q, T{}, T{}, T{});
         }
 
-        // Consumer warp: the Tjhung chain from round 7 on (divTj of the first output row takes mu_a from row 7), the output rows from round 17 on.
+        // Consumer warp: the Tjhung chain from row 7 on (divTj of the first output row takes mu_a from row 7), the
+        // output rows k-8 and k-7 from round 8 on. A segment of an odd height computes one row more than it stores.
         template <int COMP, int NOISE>
         __device__ __forceinline__ void consumer(PairSmem& sm, const float* __restrict__ phi_in,
                                                  float* __restrict__ phi_out, __nv_bfloat16* residual, const StepParams& p,
                                                  const Coef& k, const float* __restrict__ injected, const Task& t, int lane,
                                                  int bar_id)
         {
-            const int total = t.r1 - t.r0 + 16;
+            const int rounds = (t.r1 - t.r0 + 17) / 2;
             Active act;
-            Output<COMP, NOISE> out(phi_in, phi_out, residual, injected, &sm.xch[0][0], p.ny, p.nx, t, lane);
-            const float* hand = &sm.hand[1][0][4 * lane];
+            Output<COMP, NOISE, 2> out(phi_in, phi_out, residual, injected, &sm.xch[0][0][0], p.ny, p.nx, t, lane);
+            const float* hands = &sm.hand[0][0][0][4 * lane];
             float* delay = &sm.dtj[0][4 * lane];
-            const auto tjhung = [&]() -> Quad {  // stores divTj(k-2), returns divTj(k-8)
-                const Quad v = act.step(k, load_quad(hand), load_quad(hand + kCols), load_quad(hand + 2 * kCols));
-                const Quad old = load_quad(delay);
-                store_quad(delay, v);
-                delay = delay == &sm.dtj[kDelay - 1][4 * lane] ? &sm.dtj[0][4 * lane] : delay + kCols;
-                return old;
+            const auto tjhung = [&](const float* hand, Quad (&old)[2]) {  // divTj into the ring, six rows older ones out
+#pragma unroll
+                for (int i = 0; i < 2; ++i, hand += 4 * kCols)
+                {
+                    const Quad v = act.step(k, load_quad(hand), load_quad(hand + kCols), load_quad(hand + 2 * kCols));
+                    old[i] = load_quad(delay + i * kCols);
+                    store_quad(delay + i * kCols, v);
+                }
+                delay = delay == &sm.dtj[kDelay - 2][4 * lane] ? &sm.dtj[0][4 * lane] : delay + 2 * kCols;
             };
-            const auto flip = [&]() {
-                hand = hand == &sm.hand[1][0][4 * lane] ? &sm.hand[0][0][4 * lane] : &sm.hand[1][0][4 * lane];
-            };
+            Quad dtj[2];
 #pragma unroll 1
-            for (int kl = 7; kl <= 16; ++kl)
+            for (int q = 3; q < 8; ++q)
             {
                 pair_sync(bar_id);
-                tjhung();
-                flip();
+                tjhung(hands + (q & 1) * 8 * kCols, dtj);
             }
-            out.ahead(p, k);
-            int mo = 16 % kMupRing;  // position of mu_p row k-8: (k - 1) mod 10
+            out.ahead();
 #pragma unroll 1
-            for (int kl = 17; kl <= total; ++kl)
+            for (int q = 8; q < rounds; ++q)
             {
+                const float* hand = hands + (q & 1) * 8 * kCols;
                 pair_sync(bar_id);
-                const Quad dtj = tjhung();
-                out.row(p, k, &sm.mup[mo][4 * lane], dtj, load_quad(hand + 3 * kCols));
-                mo = mo + 1 == kMupRing ? 0 : mo + 1;
-                flip();
+                tjhung(hand, dtj);
+                const Quad dy8[2] = {load_quad(hand + 3 * kCols), load_quad(hand + 7 * kCols)};
+                out.rows(p, k, &sm.mup[(2 * q - 8) & (kPairMup - 1)][4 * lane], dtj, dy8);
             }
         }
 
@@ -442,7 +502,7 @@ namespace amb
             Local loc(phi_in, p.ny, p.nx, t, lane);
             Passive pas{&sm.mup[0][4 * lane], &sm.j1y[0][4 * lane]};
             Active act;
-            Output<COMP, NOISE> out(phi_in, phi_out, residual, injected, &sm.xch[0][0], p.ny, p.nx, t, lane);
+            Output<COMP, NOISE, 1> out(phi_in, phi_out, residual, injected, &sm.xch[0][0], p.ny, p.nx, t, lane);
             float* delay = &sm.dtj[0][4 * lane];
             Quad xi = zero_quad();
             int nrow = 0;
@@ -452,7 +512,7 @@ namespace amb
             };
             const auto round = [&](auto j1_tag, auto out_tag) {
                 constexpr bool J1 = decltype(j1_tag)::value, OUT = decltype(out_tag)::value;
-                Quad mup, mua, jcy, jcx, dy8;
+                Quad mup, mua, jcy, jcx, dy8[1];
                 loc.step(k, mup, mua, jcy, jcx);
                 const float* w = pas.put_mup(mup);
                 if constexpr (J1)
@@ -461,14 +521,14 @@ namespace amb
                     draw();
                     const Quad j1y = fma4(k.mag, x, Passive::d8y(k.ny8, w, mup));
                     const float* v = pas.put_j1y(j1y);
-                    if constexpr (OUT) dy8 = Passive::d8y(k.py8, v, j1y);
+                    if constexpr (OUT) dy8[0] = Passive::d8y(k.py8, v, j1y);
                 }
                 const Quad v = act.step(k, mua, jcy, jcx);
-                const Quad dtj = load_quad(delay);
+                const Quad dtj[1] = {load_quad(delay)};
                 store_quad(delay, v);
                 delay = delay == &sm.dtj[kDelay - 1][4 * lane] ? &sm.dtj[0][4 * lane] : delay + kCols;
-                // row k-8's neighbour columns: other lanes wrote them rounds ago (out.row synchronises each round)
-                if constexpr (OUT) out.row(p, k, w, dtj, dy8);
+                // row k-8's neighbour columns: other lanes wrote them rounds ago (out.rows synchronises each round)
+                if constexpr (OUT) out.rows(p, k, w, dtj, dy8);
                 else __syncwarp();
             };
             using F = std::false_type;
@@ -479,7 +539,7 @@ namespace amb
             draw();
 #pragma unroll 1
             for (int kl = 9; kl <= 16; ++kl) round(T{}, F{});
-            out.ahead(p, k);
+            out.ahead();
 #pragma unroll 1
             for (int kl = 17; kl <= total; ++kl) round(T{}, T{});
         }
@@ -708,11 +768,6 @@ namespace amb
         }
     }
 
-    int sliding_default_seg_h(int ny, int nx)
-    {
-        return choose_seg_h(ny, nx, 152 * 8);
-    }
-
     // variant: 0 = defaults; otherwise (seg_h << 4) | fused (8) | code, code 1 -> 1, 2 -> 2, 3 -> 4 warp
     // pairs (fused: warps) per CTA.
     cudaError_t launch_step_f32_sliding(const float* phi_in, float* phi_out, __nv_bfloat16* comp, int comp_mode,
@@ -734,7 +789,7 @@ namespace amb
             if (wpb == 2) return by_noise_fused<COMP_NONE, 2>(phi_in, phi_out, comp, p, noise_mode, injected, seg_h, stream);
             return by_noise_fused<COMP_NONE, 4>(phi_in, phi_out, comp, p, noise_mode, injected, seg_h, stream);
         }
-        if (wpb == 0) wpb = 1;
+        if (wpb == 0) wpb = 2;  // faster than 1 from 1000 x 1700 to 4096^2, by 3 to 12 %
         if (comp_mode == COMP_BF16)
         {
             if (wpb == 1) return by_noise<COMP_BF16, 1>(phi_in, phi_out, comp, p, noise_mode, injected, seg_h, stream);
@@ -762,11 +817,6 @@ namespace amb
     {
         sliding::Coef k(p);
         std::memcpy(out, &k, sizeof(k));
-    }
-
-    int sliding_default_seg_h_for(int ny, int nx, int resident_pairs)
-    {
-        return choose_seg_h(ny, nx, resident_pairs);
     }
 
     namespace
