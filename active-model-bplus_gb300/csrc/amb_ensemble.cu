@@ -28,6 +28,7 @@ struct amb_ensemble
     std::vector<void*> allocations;
     amb::EnsembleReplica* d_reps = nullptr;
     void* d_coefs = nullptr;
+    std::vector<unsigned char> shared_coef;  // a coefficient block whose stencil part is every replica's, or empty
     amb::EnsembleTask* d_tasks = nullptr;
     int ntasks = 0, seg_h = 0;
     bool fused = false;  // one warp per task (fused form) instead of a warp pair; chosen by measurement
@@ -86,7 +87,7 @@ namespace
     // One step for all replicas: launch with the current parity and step offset.
     cudaError_t launch_step(amb_ensemble* h, int parity, int offset)
     {
-        return amb::launch_sliding_ensemble(h->d_reps, h->d_coefs, h->d_tasks, h->ntasks, parity, h->d_step, offset,
+        return amb::launch_sliding_ensemble(h->d_reps, h->d_coefs, h->shared_coef.empty() ? nullptr : h->shared_coef.data(), h->d_tasks, h->ntasks, parity, h->d_step, offset,
                                             h->precision == AMB_F32C ? amb::COMP_BF16 : amb::COMP_NONE,
                                             h->noise ? amb::NOISE_PHILOX : amb::NOISE_OFF, h->fused, h->stream);
     }
@@ -281,6 +282,9 @@ extern "C" int amb_ensemble_create(int nreplicas, const int* nrows, const int* n
         amb::sliding_make_coef(p, coefs.data() + amb::sliding_coef_bytes() * r);
         h->host_reps.push_back(rep);
     }
+
+    if (amb::sliding_same_stencil(coefs.data(), int(h->host_reps.size())) && !h->host_reps.empty())
+        h->shared_coef.assign(coefs.begin(), coefs.begin() + amb::sliding_coef_bytes());
 
     // task table: a start from the occupancy model, then segment heights per size class chosen by
     // measurement (below, once the replicas are on the device)

@@ -61,10 +61,12 @@ namespace amb
     };
     size_t sliding_coef_bytes();
     void sliding_make_coef(const StepParams& p, void* out);  // host: per-replica coefficient block
+    bool sliding_same_stencil(const void* coefs, int n);     // host: n blocks agree in their stencil parts
+    // shared_coef (host): a coefficient block whose stencil part is every replica's, or null.
     // fused: one warp per task running every stage (otherwise a producer/consumer warp pair).
-    cudaError_t launch_sliding_ensemble(const EnsembleReplica* reps, const void* coefs, const EnsembleTask* tasks,
-                                        int ntasks, int parity, const int64_t* step_counter, int step_offset,
-                                        int comp_mode, int noise_mode, bool fused, cudaStream_t stream);
+    cudaError_t launch_sliding_ensemble(const EnsembleReplica* reps, const void* coefs, const void* shared_coef,
+                                        const EnsembleTask* tasks, int ntasks, int parity, const int64_t* step_counter,
+                                        int step_offset, int comp_mode, int noise_mode, bool fused, cudaStream_t stream);
     cudaError_t ensemble_resident_pairs(int* out, bool fused);
 
     template <typename Real>

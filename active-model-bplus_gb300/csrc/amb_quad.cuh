@@ -9,35 +9,49 @@ namespace amb
 {
     // Canon's constants as duplicated pairs, which packed operations read from the constant bank,
     // and the Philox round keys of the seed.
-    struct QuadCoef
+    struct QuadStencil
     {
         float2 lA, lB, lC, lD, gxa, gxb, gya, gyb;
         float2 ny8[4], nx8[4], py8[4], px8[4];
-        float2 a, b, c, nkappa, lambda, zeta, mag;
         float2 ndy, jx1, jx3, dyInv, tx1, tx3, dt, ndt, p1, p3;
+    };
+    struct QuadModel
+    {
+        float2 a, b, c, nkappa, lambda, zeta, mag;
         uint32_t rk0[10], rk1[10];
+    };
+    struct QuadCoef
+    {
+        QuadStencil s;
+        QuadModel m;
         __host__ explicit QuadCoef(const StepParams& p)
         {
             const Canon<float> k(p);
             const auto d = [](float v) { return make_float2(v, v); };
-            lA = d(k.lA); lB = d(k.lB); lC = d(k.lC); lD = d(k.lD);
-            gxa = d(k.gxa); gxb = d(k.gxb); gya = d(k.gya); gyb = d(k.gyb);
+            s.lA = d(k.lA); s.lB = d(k.lB); s.lC = d(k.lC); s.lD = d(k.lD);
+            s.gxa = d(k.gxa); s.gxb = d(k.gxb); s.gya = d(k.gya); s.gyb = d(k.gyb);
             for (int j = 0; j < 4; ++j)
             {
-                ny8[j] = d(k.ny8[j]); nx8[j] = d(k.nx8[j]);
-                py8[j] = d(k.py8[j]); px8[j] = d(k.px8[j]);
+                s.ny8[j] = d(k.ny8[j]); s.nx8[j] = d(k.nx8[j]);
+                s.py8[j] = d(k.py8[j]); s.px8[j] = d(k.px8[j]);
             }
-            a = d(k.a); b = d(k.b); c = d(k.c);
-            nkappa = d(k.nkappa); lambda = d(k.lambda); zeta = d(k.zeta); mag = d(k.mag);
-            ndy = d(k.ndy); jx1 = d(k.jx1); jx3 = d(k.jx3);
-            dyInv = d(k.dyInv); tx1 = d(k.tx1); tx3 = d(k.tx3);
-            dt = d(k.dt); ndt = d(k.ndt); p1 = d(k.p1); p3 = d(k.p3);
+            s.ndy = d(k.ndy); s.jx1 = d(k.jx1); s.jx3 = d(k.jx3);
+            s.dyInv = d(k.dyInv); s.tx1 = d(k.tx1); s.tx3 = d(k.tx3);
+            s.dt = d(k.dt); s.ndt = d(k.ndt); s.p1 = d(k.p1); s.p3 = d(k.p3);
+            m.a = d(k.a); m.b = d(k.b); m.c = d(k.c);
+            m.nkappa = d(k.nkappa); m.lambda = d(k.lambda); m.zeta = d(k.zeta); m.mag = d(k.mag);
             for (int r = 0; r < 10; ++r)
             {
-                rk0[r] = uint32_t(p.seed) + uint32_t(r) * 0x9E3779B9u;
-                rk1[r] = uint32_t(p.seed >> 32) + uint32_t(r) * 0xBB67AE85u;
+                m.rk0[r] = uint32_t(p.seed) + uint32_t(r) * 0x9E3779B9u;
+                m.rk1[r] = uint32_t(p.seed >> 32) + uint32_t(r) * 0xBB67AE85u;
             }
         }
+    };
+    // The two parts from different places (one stencil for many models).
+    struct QuadCoefParts
+    {
+        const QuadStencil& s;
+        const QuadModel& m;
     };
 
     struct Quad

@@ -94,15 +94,15 @@ namespace amb
         using Coef = QuadCoef;
 
         // Four normals of this lane's quad (global quad at column gcol) for one row and component.
-        template <int NOISE>
-        __device__ __forceinline__ Quad normals(const StepParams& p, const Coef& k, const float* __restrict__ injected,
+        template <int NOISE, class K>
+        __device__ __forceinline__ Quad normals(const StepParams& p, const K& k, const float* __restrict__ injected,
                                                 int grow, int gcol, int comp)
         {
             if constexpr (NOISE == NOISE_PHILOX)
             {
                 U4 ctr{uint32_t(gcol) >> 2, uint32_t(grow), uint32_t(uint64_t(p.step)),
                        (uint32_t(uint64_t(p.step) >> 32) << 1) | uint32_t(comp)};
-                U4 q = philox4x32_10_rk(ctr, k.rk0, k.rk1);
+                U4 q = philox4x32_10_rk(ctr, k.m.rk0, k.m.rk1);
                 float2 zc, zs;  // (r cos, r sin) of the draws (x, y) and (z, w)
                 box_muller_f32x2(make_uint2(q.x, q.z), make_uint2(q.y, q.w), zc, zs);
                 return {make_float2(zc.x, zs.x), make_float2(zc.y, zs.y)};
@@ -177,20 +177,21 @@ namespace amb
                 fetch();
             }
             // mu_p, mu_a and J_c of the next row
-            __device__ __forceinline__ void step(const Coef& k, Quad& mup, Quad& mua, Quad& jcy, Quad& jcx)
+            template <class K>
+            __device__ __forceinline__ void step(const K& k, Quad& mup, Quad& mua, Quad& jcy, Quad& jcx)
             {
                 Quad Ap, Dp;
                 const Quad dn = take(Ap, Dp);
                 fetch();
-                Quad l = k.lA * (Am + Ap);
-                l = fma4(k.lB, um + dn, l);
-                l = fma4(k.lC, A0, l);
-                const Quad lap = fma4(k.lD, f, l);
-                const Quad gx = fma4(k.gxb, D0, k.gxa * (Dm + Dp));
-                const Quad gy = fma4(k.gyb, dn - um, k.gya * (Ap - Am));
-                mup = fma4(k.nkappa, lap, fma4(fma4(k.c, f, k.b), f, k.a) * f);
-                mua = k.lambda * fma4(gy, gy, gx * gx);
-                const Quad zl = k.zeta * lap;
+                Quad l = k.s.lA * (Am + Ap);
+                l = fma4(k.s.lB, um + dn, l);
+                l = fma4(k.s.lC, A0, l);
+                const Quad lap = fma4(k.s.lD, f, l);
+                const Quad gx = fma4(k.s.gxb, D0, k.s.gxa * (Dm + Dp));
+                const Quad gy = fma4(k.s.gyb, dn - um, k.s.gya * (Ap - Am));
+                mup = fma4(k.m.nkappa, lap, fma4(fma4(k.m.c, f, k.m.b), f, k.m.a) * f);
+                mua = k.m.lambda * fma4(gy, gy, gx * gx);
+                const Quad zl = k.m.zeta * lap;
                 jcy = zl * gy;
                 jcx = zl * gx;
                 um = f; f = dn;
@@ -240,21 +241,22 @@ namespace amb
             {
                 sxm0 = sxm1 = dxm0 = dxm1 = sxj0 = sxj1 = dxj0 = dxj1 = jcy = jcx = zero_quad();
             }
-            __device__ __forceinline__ Quad step(const Coef& k, Quad mua, Quad ncy, Quad ncx)
+            template <class K>
+            __device__ __forceinline__ Quad step(const K& k, Quad mua, Quad ncy, Quad ncx)
             {
                 const float ml = __shfl_up_sync(0xffffffffu, mua.b.y, 1), mr = __shfl_down_sync(0xffffffffu, mua.a.x, 1);
-                const Quad sx = fma4(k.p1, nsum(ml, mua, mr), k.p3 * mua), dx = ndiff(ml, mua, mr);
-                const Quad j2y = fma4(k.ndy, sx - sxm0, jcy);
-                const Quad j2x = fma4(k.jx3, dxm1, fma4(k.jx1, dx + dxm0, jcx));
+                const Quad sx = fma4(k.s.p1, nsum(ml, mua, mr), k.s.p3 * mua), dx = ndiff(ml, mua, mr);
+                const Quad j2y = fma4(k.s.ndy, sx - sxm0, jcy);
+                const Quad j2x = fma4(k.s.jx3, dxm1, fma4(k.s.jx1, dx + dxm0, jcx));
                 sxm0 = sxm1; sxm1 = sx;
                 dxm0 = dxm1; dxm1 = dx;
                 jcy = ncy; jcx = ncx;
                 const float yl = __shfl_up_sync(0xffffffffu, j2y.b.y, 1), yr = __shfl_down_sync(0xffffffffu, j2y.a.x, 1);
                 const float xl = __shfl_up_sync(0xffffffffu, j2x.b.y, 1), xr = __shfl_down_sync(0xffffffffu, j2x.a.x, 1);
-                const Quad sj = fma4(k.p1, nsum(yl, j2y, yr), k.p3 * j2y), dj = ndiff(xl, j2x, xr);
-                Quad v = k.tx1 * (dxj0 + dj);
-                v = fma4(k.tx3, dxj1, v);
-                v = fma4(k.dyInv, sj - sxj0, v);
+                const Quad sj = fma4(k.s.p1, nsum(yl, j2y, yr), k.s.p3 * j2y), dj = ndiff(xl, j2x, xr);
+                Quad v = k.s.tx1 * (dxj0 + dj);
+                v = fma4(k.s.tx3, dxj1, v);
+                v = fma4(k.s.dyInv, sj - sxj0, v);
                 sxj0 = sxj1; sxj1 = sj;
                 dxj0 = dxj1; dxj1 = dj;
                 return v;
@@ -306,7 +308,8 @@ namespace amb
             }
             // rows grow .. grow + R - 1, given their consecutive mu_p rows (this lane's columns of shared rows),
             // divTj and DY8
-            __device__ __forceinline__ void rows(const StepParams& p, const Coef& k, const float* mup, const Quad (&dtj)[R],
+            template <class K>
+            __device__ __forceinline__ void rows(const StepParams& p, const K& k, const float* mup, const Quad (&dtj)[R],
                                                  const Quad (&dy8)[R])
             {
                 float* e = xch + flip * R * kCols;
@@ -318,7 +321,7 @@ namespace amb
                 {
                     const float* m = mup + j * kCols;
                     const Quad xi = normals<NOISE>(p, k, injected, at(j), gcol, 1);
-                    j1x[j] = fma4(k.mag, xi, d8x(k.nx8, load_quad(m + left), load_quad(m), load_quad(m + right)));
+                    j1x[j] = fma4(k.m.mag, xi, d8x(k.s.nx8, load_quad(m + left), load_quad(m), load_quad(m + right)));
                     store_quad(e + j * kCols, j1x[j]);
                     f[j] = quad(fnext[j]);
                     if constexpr (COMP == COMP_BF16) rv[j] = rnext[j];
@@ -330,7 +333,7 @@ namespace amb
 #pragma unroll
                 for (int j = 0; j < R; ++j)
                 {
-                    const Quad div = d8x(k.px8, load_quad(e + j * kCols + left), j1x[j], load_quad(e + j * kCols + right))
+                    const Quad div = d8x(k.s.px8, load_quad(e + j * kCols + left), j1x[j], load_quad(e + j * kCols + right))
                                    + (dtj[j] + dy8[j]);
                     const size_t gi = (size_t)(row + j) * nx + gcol;
                     const bool st = store && (j == 0 || row + j < last);
@@ -338,7 +341,7 @@ namespace amb
                     {
                         const Quad rr{make_float2(__uint_as_float(rv[j].x << 16), __uint_as_float(rv[j].x & 0xffff0000u)),
                                       make_float2(__uint_as_float(rv[j].y << 16), __uint_as_float(rv[j].y & 0xffff0000u))};
-                        const Quad F = fma4(k.dt, div, rr);
+                        const Quad F = fma4(k.s.dt, div, rr);
                         const Quad nf = f[j] - F;
                         const Quad nr = (nf - f[j]) + F;
                         if (st)
@@ -353,7 +356,7 @@ namespace amb
                         }
                     }
                     else if (st)
-                        store_quad(phi_out + gi, fma4(k.ndt, div, f[j]));
+                        store_quad(phi_out + gi, fma4(k.s.ndt, div, f[j]));
                 }
             }
         };
@@ -385,9 +388,9 @@ namespace amb
         // Producer warp: stage A, the mu_p ring, J1_y with its noise, and DY8, two rows per round: round q takes
         // rows k = 2q + 1 and k + 1. Rows 1..6 feed no divTj row that an output reads, rows 1..8 no J1_y row and
         // rows 1..16 no DY8 row: their rounds run the body without those parts (the first three without a hand-off).
-        template <int NOISE>
+        template <int NOISE, class K>
         __device__ __forceinline__ void producer(PairSmem& sm, const float* __restrict__ phi_in, const StepParams& p,
-                                                 const Coef& k, const float* __restrict__ injected, const Task& t,
+                                                 const K& k, const float* __restrict__ injected, const Task& t,
                                                  int lane, int bar_id)
         {
             const int rounds = (t.r1 - t.r0 + 17) / 2;
@@ -420,12 +423,12 @@ namespace amb
                 {
                     const Quad x0 = draw(), x1 = draw();
                     Quad s0, s1;
-                    d8y_two<kPairMup>(k.ny8, mup, 2 * q - 8, m[0], m[1], s0, s1);
-                    const Quad j0 = fma4(k.mag, x0, s0), j1 = fma4(k.mag, x1, s1);
+                    d8y_two<kPairMup>(k.s.ny8, mup, 2 * q - 8, m[0], m[1], s0, s1);
+                    const Quad j0 = fma4(k.m.mag, x0, s0), j1 = fma4(k.m.mag, x1, s1);
                     if constexpr (DY)
                     {
                         Quad d0, d1;
-                        d8y_two<kPairJ1>(k.py8, j1y, 2 * q + 4, j0, j1, d0, d1);
+                        d8y_two<kPairJ1>(k.s.py8, j1y, 2 * q + 4, j0, j1, d0, d1);
                         store_quad(hand + 3 * kCols, d0);
                         store_quad(hand + 7 * kCols, d1);
                     }
@@ -449,10 +452,10 @@ namespace amb
 
         // Consumer warp: the Tjhung chain from row 7 on (divTj of the first output row takes mu_a from row 7), the
         // output rows k-8 and k-7 from round 8 on. A segment of an odd height computes one row more than it stores.
-        template <int COMP, int NOISE>
+        template <int COMP, int NOISE, class K>
         __device__ __forceinline__ void consumer(PairSmem& sm, const float* __restrict__ phi_in,
                                                  float* __restrict__ phi_out, __nv_bfloat16* residual, const StepParams& p,
-                                                 const Coef& k, const float* __restrict__ injected, const Task& t, int lane,
+                                                 const K& k, const float* __restrict__ injected, const Task& t, int lane,
                                                  int bar_id)
         {
             const int rounds = (t.r1 - t.r0 + 17) / 2;
@@ -492,10 +495,10 @@ namespace amb
         // One warp runs every stage of its strip: the producer's and the consumer's work of each round in
         // one instruction stream, with no hand-off buffers and no barrier between warps. The same
         // operations in the same order as the warp pair, so the same bits.
-        template <int COMP, int NOISE>
+        template <int COMP, int NOISE, class K>
         __device__ __forceinline__ void fused_strip(WarpSmem& sm, const float* __restrict__ phi_in,
                                                     float* __restrict__ phi_out, __nv_bfloat16* residual,
-                                                    const StepParams& p, const Coef& k,
+                                                    const StepParams& p, const K& k,
                                                     const float* __restrict__ injected, const Task& t, int lane)
         {
             const int total = t.r1 - t.r0 + 16;
@@ -519,9 +522,9 @@ namespace amb
                 {
                     const Quad x = xi;
                     draw();
-                    const Quad j1y = fma4(k.mag, x, Passive::d8y(k.ny8, w, mup));
+                    const Quad j1y = fma4(k.m.mag, x, Passive::d8y(k.s.ny8, w, mup));
                     const float* v = pas.put_j1y(j1y);
-                    if constexpr (OUT) dy8[0] = Passive::d8y(k.py8, v, j1y);
+                    if constexpr (OUT) dy8[0] = Passive::d8y(k.s.py8, v, j1y);
                 }
                 const Quad v = act.step(k, mua, jcy, jcx);
                 const Quad dtj[1] = {load_quad(delay)};
@@ -580,69 +583,38 @@ namespace amb
 
     namespace sliding
     {
-        // Batched form: one warp pair per task of a task table that spans many replicas of
-        // different sizes and parameters; the step index comes from device memory so that
-        // a captured CUDA graph of several steps can be replayed.
-        // The per-replica coefficients are copied from their table into the pair's shared memory
-        // at the start of the task and read from there (8 one-pair CTAs per SM, as the
-        // single-field kernel: at most 128 registers).
-        template <int COMP, int NOISE>
-        __global__ void __launch_bounds__(64, 8)
+        // Batched form: one warp pair (FUSED: one warp) per task of a task table that spans many replicas of
+        // different sizes and parameters; the step index comes from device memory so that a captured CUDA
+        // graph of several steps can be replayed. The replica's coefficients are copied from their table into
+        // shared memory at the start of the task and read from there, where each read costs an instruction and
+        // a wavefront; with one stencil for all replicas (SAME) only the model's are, and the stencil's, most
+        // of the reads, come from the constant bank as in the single-field kernel (32 replicas of 128 to 1024
+        // rows and columns, 6.5 M sites: 76.9 us per step, 85.2 with all coefficients in shared memory).
+        // 8 one-pair CTAs per SM: at most 128 registers.
+        template <int COMP, int NOISE, bool FUSED, bool SAME>
+        __global__ void __launch_bounds__(FUSED ? 32 : 64, FUSED ? 9 : 8)
         sliding_ensemble_kernel(const EnsembleReplica* __restrict__ reps, const Coef* __restrict__ coefs,
-                                const EnsembleTask* __restrict__ tasks, int parity,
+                                const QuadStencil stencil, const EnsembleTask* __restrict__ tasks, int parity,
                                 const int64_t* __restrict__ step_counter, int step_offset)
         {
             extern __shared__ __align__(16) unsigned char smem_raw[];
-            const int role = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
-            PairSmem& sm = *reinterpret_cast<PairSmem*>(smem_raw);
-            const EnsembleTask bt = tasks[blockIdx.x];
-            const EnsembleReplica& rd = reps[bt.replica];
-            StepParams p = rd.p;
-            p.step = *step_counter + step_offset;
-            Coef* kc = reinterpret_cast<Coef*>(smem_raw + sizeof(PairSmem));
-            {
-                const uint32_t* src = reinterpret_cast<const uint32_t*>(coefs + bt.replica);
-                uint32_t* dst = reinterpret_cast<uint32_t*>(kc);
-                for (int i = threadIdx.x; i < int(sizeof(Coef) / 4); i += 64) dst[i] = src[i];
-            }
-            __syncthreads();
-            const Coef& k = *kc;
-            Task t;
-            int c0 = bt.strip * kOut;
-            t.store_lo = c0;
-            if (c0 + kOut > p.nx) c0 = p.nx - kOut;
-            t.c0 = c0;
-            t.r0 = bt.r0;
-            t.r1 = bt.r1;
-            if (role == 0)
-                producer<NOISE>(sm, rd.phi[parity], p, k, nullptr, t, lane, 1);
-            else
-                consumer<COMP, NOISE>(sm, rd.phi[parity], rd.phi[parity ^ 1], rd.residual, p, k, nullptr, t, lane, 1);
-        }
-
-        // The batched form with one warp per task running every stage (the fused form), its
-        // replica's coefficient block in shared memory beside the warp's rings.
-        template <int COMP, int NOISE>
-        __global__ void __launch_bounds__(32)
-        sliding_ensemble_fused_kernel(const EnsembleReplica* __restrict__ reps, const Coef* __restrict__ coefs,
-                                      const EnsembleTask* __restrict__ tasks, int parity,
-                                      const int64_t* __restrict__ step_counter, int step_offset)
-        {
-            extern __shared__ __align__(16) unsigned char smem_raw[];
+            using Smem = typename std::conditional<FUSED, WarpSmem, PairSmem>::type;
+            constexpr int NT = FUSED ? 32 : 64;
             const int lane = threadIdx.x & 31;
-            WarpSmem& sm = *reinterpret_cast<WarpSmem*>(smem_raw);
+            Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
             const EnsembleTask bt = tasks[blockIdx.x];
             const EnsembleReplica& rd = reps[bt.replica];
             StepParams p = rd.p;
             p.step = *step_counter + step_offset;
-            Coef* kc = reinterpret_cast<Coef*>(smem_raw + sizeof(WarpSmem));
+            Coef* kc = reinterpret_cast<Coef*>(smem_raw + sizeof(Smem));
             {
+                constexpr int skip = SAME ? int(sizeof(QuadStencil) / 4) : 0;
                 const uint32_t* src = reinterpret_cast<const uint32_t*>(coefs + bt.replica);
                 uint32_t* dst = reinterpret_cast<uint32_t*>(kc);
-                for (int i = lane; i < int(sizeof(Coef) / 4); i += 32) dst[i] = src[i];
+                for (int i = skip + threadIdx.x; i < int(sizeof(Coef) / 4); i += NT) dst[i] = src[i];
             }
-            __syncwarp();
-            const Coef& k = *kc;
+            if constexpr (FUSED) __syncwarp();
+            else __syncthreads();
             Task t;
             int c0 = bt.strip * kOut;
             t.store_lo = c0;
@@ -650,7 +622,12 @@ namespace amb
             t.c0 = c0;
             t.r0 = bt.r0;
             t.r1 = bt.r1;
-            fused_strip<COMP, NOISE>(sm, rd.phi[parity], rd.phi[parity ^ 1], rd.residual, p, k, nullptr, t, lane);
+            const QuadCoefParts k{SAME ? stencil : kc->s, kc->m};
+            const float* in = rd.phi[parity];
+            float* out = rd.phi[parity ^ 1];
+            if constexpr (FUSED) fused_strip<COMP, NOISE>(sm, in, out, rd.residual, p, k, nullptr, t, lane);
+            else if (threadIdx.x < 32) producer<NOISE>(sm, in, p, k, nullptr, t, lane, 1);
+            else consumer<COMP, NOISE>(sm, in, out, rd.residual, p, k, nullptr, t, lane, 1);
         }
     }
 
@@ -809,8 +786,44 @@ namespace amb
     namespace
     {
         // A pair's (or, fused, a warp's) shared memory plus its replica's coefficient block.
-        constexpr size_t ensemble_smem_bytes() { return sizeof(sliding::PairSmem) + sizeof(sliding::Coef); }
-        constexpr size_t ensemble_fused_smem_bytes() { return sizeof(sliding::WarpSmem) + sizeof(sliding::Coef); }
+        template <bool FUSED>
+        constexpr size_t ensemble_smem_bytes()
+        {
+            return (FUSED ? sizeof(sliding::WarpSmem) : sizeof(sliding::PairSmem)) + sizeof(sliding::Coef);
+        }
+
+        template <int COMP, int NOISE, bool FUSED, bool SAME>
+        cudaError_t ensemble_launch(const EnsembleReplica* reps, const sliding::Coef* coefs, const QuadStencil& stencil,
+                                    const EnsembleTask* tasks, int ntasks, int parity, const int64_t* step_counter,
+                                    int step_offset, cudaStream_t stream)
+        {
+            auto kern = sliding::sliding_ensemble_kernel<COMP, NOISE, FUSED, SAME>;
+            constexpr size_t smem = ensemble_smem_bytes<FUSED>();
+            static bool configured = false;
+            if (!configured)
+            {
+                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+                if (e != cudaSuccess) return e;
+                configured = true;
+            }
+            kern<<<ntasks, FUSED ? 32 : 64, smem, stream>>>(reps, coefs, stencil, tasks, parity, step_counter, step_offset);
+            return cudaGetLastError();
+        }
+
+        template <bool FUSED>
+        cudaError_t ensemble_resident(int* out)
+        {
+            auto kern = sliding::sliding_ensemble_kernel<COMP_BF16, NOISE_PHILOX, FUSED, true>;
+            constexpr size_t smem = ensemble_smem_bytes<FUSED>();
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+            int dev = 0, sms = 0, blocks = 0;
+            if (e == cudaSuccess) e = cudaGetDevice(&dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e == cudaSuccess)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, FUSED ? 32 : 64, smem);
+            if (e == cudaSuccess) *out = blocks * sms > 0 ? blocks * sms : 1;
+            return e;
+        }
     }
 
     void sliding_make_coef(const StepParams& p, void* out)
@@ -819,69 +832,42 @@ namespace amb
         std::memcpy(out, &k, sizeof(k));
     }
 
-    namespace
+    bool sliding_same_stencil(const void* coefs, int n)
     {
-        template <int COMP, int NOISE, bool FUSED>
-        cudaError_t launch_ensemble_variant(const EnsembleReplica* reps, const void* coefs, const EnsembleTask* tasks,
-                                            int ntasks, int parity, const int64_t* step_counter, int step_offset,
-                                            cudaStream_t stream)
-        {
-            using namespace sliding;
-            auto kern = FUSED ? sliding_ensemble_fused_kernel<COMP, NOISE> : sliding_ensemble_kernel<COMP, NOISE>;
-            const size_t smem = FUSED ? ensemble_fused_smem_bytes() : ensemble_smem_bytes();
-            static bool configured = false;
-            if (!configured)
-            {
-                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-                if (e != cudaSuccess) return e;
-                configured = true;
-            }
-            kern<<<ntasks, FUSED ? 32 : 64, smem, stream>>>(reps, static_cast<const Coef*>(coefs), tasks, parity,
-                                                           step_counter, step_offset);
-            return cudaGetLastError();
-        }
-
-        template <bool FUSED>
-        cudaError_t launch_ensemble_form(const EnsembleReplica* reps, const void* coefs, const EnsembleTask* tasks,
-                                         int ntasks, int parity, const int64_t* step_counter, int step_offset,
-                                         int comp_mode, bool noise, cudaStream_t stream)
-        {
-            if (comp_mode == COMP_BF16)
-                return noise ? launch_ensemble_variant<COMP_BF16, NOISE_PHILOX, FUSED>(reps, coefs, tasks, ntasks, parity,
-                                                                                       step_counter, step_offset, stream)
-                             : launch_ensemble_variant<COMP_BF16, NOISE_OFF, FUSED>(reps, coefs, tasks, ntasks, parity,
-                                                                                    step_counter, step_offset, stream);
-            return noise ? launch_ensemble_variant<COMP_NONE, NOISE_PHILOX, FUSED>(reps, coefs, tasks, ntasks, parity,
-                                                                                   step_counter, step_offset, stream)
-                         : launch_ensemble_variant<COMP_NONE, NOISE_OFF, FUSED>(reps, coefs, tasks, ntasks, parity,
-                                                                                step_counter, step_offset, stream);
-        }
+        const auto* k = static_cast<const sliding::Coef*>(coefs);
+        for (int r = 1; r < n; ++r)
+            if (std::memcmp(&k[r].s, &k[0].s, sizeof(QuadStencil)) != 0) return false;
+        return true;
     }
 
     cudaError_t ensemble_resident_pairs(int* out, bool fused)
     {
-        using namespace sliding;
-        const void* kern = fused ? reinterpret_cast<const void*>(sliding_ensemble_fused_kernel<COMP_BF16, NOISE_PHILOX>)
-                                 : reinterpret_cast<const void*>(sliding_ensemble_kernel<COMP_BF16, NOISE_PHILOX>);
-        const size_t smem = fused ? ensemble_fused_smem_bytes() : ensemble_smem_bytes();
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        int dev = 0, sms = 0, blocks = 0;
-        if (e == cudaSuccess) e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, fused ? 32 : 64, smem);
-        if (e == cudaSuccess) *out = blocks * sms > 0 ? blocks * sms : 1;
-        return e;
+        return fused ? ensemble_resident<true>(out) : ensemble_resident<false>(out);
     }
 
-    cudaError_t launch_sliding_ensemble(const EnsembleReplica* reps, const void* coefs, const EnsembleTask* tasks,
-                                        int ntasks, int parity, const int64_t* step_counter, int step_offset,
-                                        int comp_mode, int noise_mode, bool fused, cudaStream_t stream)
+    cudaError_t launch_sliding_ensemble(const EnsembleReplica* reps, const void* coefs, const void* shared_coef,
+                                        const EnsembleTask* tasks, int ntasks, int parity, const int64_t* step_counter,
+                                        int step_offset, int comp_mode, int noise_mode, bool fused, cudaStream_t stream)
     {
         if (ntasks <= 0) return cudaSuccess;
+        const auto* table = static_cast<const sliding::Coef*>(coefs);
+        QuadStencil st{};
+        if (shared_coef) st = static_cast<const sliding::Coef*>(shared_coef)->s;
+        const auto go = [&](auto comp, auto noise) {
+            constexpr int C = decltype(comp)::value, N = decltype(noise)::value;
+            const auto run = [&](auto f, auto s) {
+                return ensemble_launch<C, N, decltype(f)::value, decltype(s)::value>(reps, table, st, tasks, ntasks, parity,
+                                                                                     step_counter, step_offset, stream);
+            };
+            if (fused) return shared_coef ? run(std::true_type{}, std::true_type{}) : run(std::true_type{}, std::false_type{});
+            return shared_coef ? run(std::false_type{}, std::true_type{}) : run(std::false_type{}, std::false_type{});
+        };
+        using Bf16 = std::integral_constant<int, COMP_BF16>;
+        using None = std::integral_constant<int, COMP_NONE>;
+        using Philox = std::integral_constant<int, NOISE_PHILOX>;
+        using Off = std::integral_constant<int, NOISE_OFF>;
         const bool noise = noise_mode == NOISE_PHILOX;
-        return fused ? launch_ensemble_form<true>(reps, coefs, tasks, ntasks, parity, step_counter, step_offset,
-                                                  comp_mode, noise, stream)
-                     : launch_ensemble_form<false>(reps, coefs, tasks, ntasks, parity, step_counter, step_offset,
-                                                   comp_mode, noise, stream);
+        if (comp_mode == COMP_BF16) return noise ? go(Bf16{}, Philox{}) : go(Bf16{}, Off{});
+        return noise ? go(None{}, Philox{}) : go(None{}, Off{});
     }
 }

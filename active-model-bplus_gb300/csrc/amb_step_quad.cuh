@@ -91,7 +91,7 @@ namespace amb
                 const auto quad_at = [&](int col) {  // the normals of the noise quad that holds column col
                     const U4 ctr{uint32_t(col) >> 2, uint32_t(row), uint32_t(uint64_t(step)),
                                  (uint32_t(uint64_t(step) >> 32) << 1) | uint32_t(comp)};
-                    const U4 q = philox4x32_10_rk(ctr, p.k.rk0, p.k.rk1);
+                    const U4 q = philox4x32_10_rk(ctr, p.k.m.rk0, p.k.m.rk1);
                     float2 zc, zs;
                     box_muller_f32x2(make_uint2(q.x, q.z), make_uint2(q.y, q.w), zc, zs);
                     return make_float4(zc.x, zs.x, zc.y, zs.y);
@@ -192,19 +192,19 @@ namespace amb
                         s += G::PW;
                         const Quad dn = load_quad(s);
                         const Quad Ap = nsum(s[-1], dn, s[4]), Dp = ndiff(s[-1], dn, s[4]);
-                        Quad l = k.lA * (Am + Ap);
-                        l = fma4(k.lB, um + dn, l);
-                        l = fma4(k.lC, A0, l);
-                        const Quad lap = fma4(k.lD, f, l);
-                        store_quad(m, fma4(k.nkappa, lap, fma4(fma4(k.c, f, k.b), f, k.a) * f));
+                        Quad l = k.s.lA * (Am + Ap);
+                        l = fma4(k.s.lB, um + dn, l);
+                        l = fma4(k.s.lC, A0, l);
+                        const Quad lap = fma4(k.s.lD, f, l);
+                        store_quad(m, fma4(k.m.nkappa, lap, fma4(fma4(k.m.c, f, k.m.b), f, k.m.a) * f));
                         if (near && i >= -2 && i < ty + 2)
                         {
-                            const Quad gx = fma4(k.gxb, D0, k.gxa * (Dm + Dp));
-                            const Quad gy = fma4(k.gyb, dn - um, k.gya * (Ap - Am));
-                            store_quad(a.mua + e, k.lambda * fma4(gy, gy, gx * gx));
+                            const Quad gx = fma4(k.s.gxb, D0, k.s.gxa * (Dm + Dp));
+                            const Quad gy = fma4(k.s.gyb, dn - um, k.s.gya * (Ap - Am));
+                            store_quad(a.mua + e, k.m.lambda * fma4(gy, gy, gx * gx));
                             if (i >= -1 && i < ty + 1)
                             {
-                                const Quad zl = k.zeta * lap;
+                                const Quad zl = k.m.zeta * lap;
                                 store_quad(a.j2y + e - G::AW, zl * gy);
                                 store_quad(a.j2x + e - G::AW, zl * gx);
                             }
@@ -231,20 +231,20 @@ namespace amb
                         const int i = t / QY, j = t - i * QY;  // row i - 4
                         const float* c = a.mup + (i + 4) * G::MW + 4 * j + G::M0;
                         constexpr int L = G::MW;
-                        Quad s = k.ny8[0] * (load_quad(c + L) - load_quad(c - L));
-                        s = fma4(k.ny8[1], load_quad(c + 2 * L) - load_quad(c - 2 * L), s);
-                        s = fma4(k.ny8[2], load_quad(c + 3 * L) - load_quad(c - 3 * L), s);
-                        s = fma4(k.ny8[3], load_quad(c + 4 * L) - load_quad(c - 4 * L), s);
+                        Quad s = k.s.ny8[0] * (load_quad(c + L) - load_quad(c - L));
+                        s = fma4(k.s.ny8[1], load_quad(c + 2 * L) - load_quad(c - 2 * L), s);
+                        s = fma4(k.s.ny8[2], load_quad(c + 3 * L) - load_quad(c - 3 * L), s);
+                        s = fma4(k.s.ny8[3], load_quad(c + 4 * L) - load_quad(c - 4 * L), s);
                         float* e = a.j1y + i * TX + 4 * j;
-                        store_quad(e, fma4(k.mag, noisy ? load_quad(e) : zero_quad(), s));
+                        store_quad(e, fma4(k.m.mag, noisy ? load_quad(e) : zero_quad(), s));
                     }
                     else if (t < n2)
                     {
                         const int i = (t - n1) / QX, j = t - n1 - i * QX;
                         const float* c = a.mup + (i + 8) * G::MW + 4 * j - G::A0 + G::M0;
-                        const Quad s = d8x(k.nx8, load_quad(c - 4), load_quad(c), load_quad(c + 4));
+                        const Quad s = d8x(k.s.nx8, load_quad(c - 4), load_quad(c), load_quad(c + 4));
                         float* e = a.j1x + i * G::AW + 4 * j;
-                        store_quad(e, fma4(k.mag, noisy ? load_quad(e) : zero_quad(), s));
+                        store_quad(e, fma4(k.m.mag, noisy ? load_quad(e) : zero_quad(), s));
                     }
                     else
                     {
@@ -254,12 +254,12 @@ namespace amb
                         const float* u = a.mua + i * G::AW + 4 * j;
                         const float *m = u + G::AW, *d = m + G::AW;
                         const Quad uq = load_quad(u), mq = load_quad(m), dq = load_quad(d);
-                        const Quad su = fma4(k.p1, nsum(u[l], uq, u[r]), k.p3 * uq);
-                        const Quad sd = fma4(k.p1, nsum(d[l], dq, d[r]), k.p3 * dq);
+                        const Quad su = fma4(k.s.p1, nsum(u[l], uq, u[r]), k.s.p3 * uq);
+                        const Quad sd = fma4(k.s.p1, nsum(d[l], dq, d[r]), k.s.p3 * dq);
                         const Quad du = ndiff(u[l], uq, u[r]), dm = ndiff(m[l], mq, m[r]), dd = ndiff(d[l], dq, d[r]);
                         const int e = i * G::AW + 4 * j;
-                        store_quad(a.j2y + e, fma4(k.ndy, sd - su, load_quad(a.j2y + e)));
-                        store_quad(a.j2x + e, fma4(k.jx3, dm, fma4(k.jx1, dd + du, load_quad(a.j2x + e))));
+                        store_quad(a.j2y + e, fma4(k.s.ndy, sd - su, load_quad(a.j2y + e)));
+                        store_quad(a.j2x + e, fma4(k.s.jx3, dm, fma4(k.s.jx1, dd + du, load_quad(a.j2x + e))));
                     }
                 }
             }
@@ -277,20 +277,20 @@ namespace amb
                 const float* x0 = a.j2x + i * G::AW + 4 * j + G::A0;
                 const float *x1 = x0 + G::AW, *x2 = x1 + G::AW;
                 const Quad yu = load_quad(y0), yd = load_quad(y2);
-                const Quad su = fma4(k.p1, nsum(y0[-1], yu, y0[4]), k.p3 * yu);
-                const Quad sd = fma4(k.p1, nsum(y2[-1], yd, y2[4]), k.p3 * yd);
+                const Quad su = fma4(k.s.p1, nsum(y0[-1], yu, y0[4]), k.s.p3 * yu);
+                const Quad sd = fma4(k.s.p1, nsum(y2[-1], yd, y2[4]), k.s.p3 * yd);
                 const Quad du = ndiff(x0[-1], load_quad(x0), x0[4]), dm = ndiff(x1[-1], load_quad(x1), x1[4]),
                            dd = ndiff(x2[-1], load_quad(x2), x2[4]);
-                Quad tj = k.tx1 * (du + dd);
-                tj = fma4(k.tx3, dm, tj);
-                tj = fma4(k.dyInv, sd - su, tj);
+                Quad tj = k.s.tx1 * (du + dd);
+                tj = fma4(k.s.tx3, dm, tj);
+                tj = fma4(k.s.dyInv, sd - su, tj);
                 const float* cy = a.j1y + (i + 4) * TX + 4 * j;
-                Quad s = k.py8[0] * (load_quad(cy + TX) - load_quad(cy - TX));
-                s = fma4(k.py8[1], load_quad(cy + 2 * TX) - load_quad(cy - 2 * TX), s);
-                s = fma4(k.py8[2], load_quad(cy + 3 * TX) - load_quad(cy - 3 * TX), s);
-                s = fma4(k.py8[3], load_quad(cy + 4 * TX) - load_quad(cy - 4 * TX), s);
+                Quad s = k.s.py8[0] * (load_quad(cy + TX) - load_quad(cy - TX));
+                s = fma4(k.s.py8[1], load_quad(cy + 2 * TX) - load_quad(cy - 2 * TX), s);
+                s = fma4(k.s.py8[2], load_quad(cy + 3 * TX) - load_quad(cy - 3 * TX), s);
+                s = fma4(k.s.py8[3], load_quad(cy + 4 * TX) - load_quad(cy - 4 * TX), s);
                 const float* cx = a.j1x + i * G::AW + 4 * j + G::A0;
-                const Quad div = d8x(k.px8, load_quad(cx - 4), load_quad(cx), load_quad(cx + 4)) + (tj + s);
+                const Quad div = d8x(k.s.px8, load_quad(cx - 4), load_quad(cx), load_quad(cx + 4)) + (tj + s);
                 const Quad f = load_quad(a.phi + (i + 9) * G::PW + 4 * j + G::P0);
                 const size_t gi = size_t(gr) * p.nx + gc;
                 if constexpr (COMP == COMP_BF16)
@@ -309,7 +309,7 @@ namespace amb
                         for (int q = 0; q < 4; ++q) v[q] = gc + q < p.nx ? __bfloat162float(comp[gi + q]) : 0.f;
                         rr = {make_float2(v[0], v[1]), make_float2(v[2], v[3])};
                     }
-                    const Quad F = fma4(k.dt, div, rr);
+                    const Quad F = fma4(k.s.dt, div, rr);
                     const Quad nf = f - F;
                     const Quad nr = (nf - f) + F;
                     if (p.vec)
@@ -336,7 +336,7 @@ namespace amb
                 }
                 else
                 {
-                    const Quad nf = fma4(k.ndt, div, f);
+                    const Quad nf = fma4(k.s.ndt, div, f);
                     if (p.vec) store_quad(out + gi, nf);
                     else
                     {

@@ -3,7 +3,7 @@ window wraps round the row, segments shorter than the pipeline. Bitwise the tile
 import numpy as np
 import pytest
 
-from activemodelbplus.integrator import Integrator, Model, Stencil
+from activemodelbplus.integrator import Ensemble, Integrator, Model, Stencil
 
 pytestmark = pytest.mark.gpu
 
@@ -21,3 +21,21 @@ def test_edges(shape, seg_rows, fused, precision):
     a.run(4)
     b.run(4)
     assert np.array_equal(a.field, b.field)
+
+
+@pytest.mark.parametrize("precision", ["f32", "f32c"])
+@pytest.mark.parametrize("fused", [False, True])
+def test_ensemble_of_one_stencil(fused, precision):
+    """Replicas that share a stencil read it from the launch; odd heights, one strip and several."""
+    rng = np.random.default_rng(6)
+    shapes, st = [(1, 112), (33, 116), (70, 340), (129, 228)], Stencil(dt=1e-3, dx=1.0, dy=1.25)
+    fields = [rng.normal(-0.4, 0.1, s) for s in shapes]
+    models = [Model(a=-0.25, b=0.1 * i, c=0.25, kappa=1 + i, lamb=-1, zeta=-4 + i, T=0.05 * i) for i in range(4)]
+    ens = Ensemble(fields, st, models, precision=precision, seeds=list(range(4)), graph_steps=2)
+    ens.fused = fused
+    ens.run(5)
+    for r in range(4):
+        a = Integrator(fields[r], st, models[r], precision=precision, seed=r, kernel="tile")
+        a.run(5)
+        assert np.array_equal(a.field, ens.field(r)), r
+    ens.close()
