@@ -746,12 +746,31 @@ class LearnedStepper:
 
     def _apply(self, noisy: bool) -> None:
         """Network flux, plus (one spectral pass) the linear part and the filtered noise flux,
-        then the exactly conservative fixed-point update."""
+        then the exactly conservative fixed-point update. In a captured macro step the spectral pass
+        is a branch beside the network's, which leaves room for it (one CTA per SM, and the SMs idle
+        between layers); its buffers are the stepper's own, so nothing is allocated on the branch."""
         torch = _torch()
+        noisy = noisy and self.model.T > 0
+        if torch.cuda.is_current_stream_capturing() and not (noisy and self._g is not None and not self.spectral_noise):
+            here, branch = torch.cuda.current_stream(), torch.cuda.Stream()
+            branch.wait_stream(here)
+            with torch.cuda.stream(branch):
+                xi_direct, mag = self._spectral(noisy)
+            net_flux = self.net.forward(self._x)
+            here.wait_stream(branch)
+        else:
+            net_flux = self.net.forward(self._x)
+            xi_direct, mag = self._spectral(noisy)
+        _check(N.lib().amb_learned_update_input(
+            _ptr(net_flux), _ptr(self._extra), *self.shape, self.dtk, self.stencil.dx, self.stencil.dy,
+            _ptr(xi_direct), mag if xi_direct is not None else 0.0, _ptr(self.phi_q), _ptr(self.phi_f), self.bound,
+            _ptr(self.flag), _ptr(self.step_dev), _ptr(self.params), _ptr(self._x), _stream()))
+
+    def _spectral(self, noisy: bool):
+        """The linear part and the noise of one macro step into ``_extra``; the per-site noise that the
+        update kernel adds itself (or None) and the noise magnitude."""
         lib = N.lib()
         ny, nx = self.shape
-        net_flux = self.net.forward(self._x)
-        noisy = noisy and self.model.T > 0
         mag = math.sqrt(2.0 * self.model.T) * math.sqrt(1.0 / (self.dtk * self.stencil.dx * self.stencil.dy))
         xi_direct = None
         if self._g is None and noisy:
@@ -767,10 +786,7 @@ class LearnedStepper:
             self._linear.extra(self.phi_f, self.xi, mag, self._extra)
         else:
             self._linear.extra(self.phi_f, None, 0.0, self._extra)
-        _check(lib.amb_learned_update_input(_ptr(net_flux), _ptr(self._extra), ny, nx, self.dtk, self.stencil.dx,
-                                            self.stencil.dy, _ptr(xi_direct), mag if xi_direct is not None else 0.0,
-                                            _ptr(self.phi_q), _ptr(self.phi_f), self.bound, _ptr(self.flag),
-                                            _ptr(self.step_dev), _ptr(self.params), _ptr(self._x), _stream()))
+        return xi_direct, mag
 
     def _refresh_input(self) -> None:
         _check(N.lib().amb_learned_input(_ptr(self.phi_f), _ptr(self.params), 1, self.shape[0], self.shape[1],
