@@ -21,9 +21,12 @@
 // sit side by side in TMEM (zeroed first). One 128 x 160 x 16 MMA thus replaces
 // five 128 x 32 x 16 ones and the A tile is read from shared memory once instead
 // of five times. Rows at the edges of the CTA's range issue only the slices of
-// the output rows they own. Warp 0 stages rows, warp 1 issues the MMAs and
-// commits one mbarrier per finished output row, warps 2-9 zero TMEM and then run
-// the epilogue (bias, GELU, its derivative, or FP32 output). The data gradient of
+// the output rows they own. Warp 0 stages rows, as soon as the barriers exist, while warp 1 allocates TMEM
+// and warps 2-9 zero it. One elected thread of warp 1 then issues the MMAs and commits one mbarrier per
+// finished output row, warps 2-9 run the epilogue (bias, GELU, its derivative, or FP32 output).
+// Six layers (5 -> 32 -> ... -> 2) at 512^2: 68 us in a graph; 79 with the MMAs issued under lane == 0 and
+// the rows requested once all warps were ready (128^2: 30.5 and 36.1). All layers in one cooperative
+// launch, with flags between neighbouring tiles, took longer than the launches that it saved. The data gradient of
 // a circular convolution is the forward convolution with the kernel flipped and
 // the channel roles swapped, so the same kernel serves it with the
 // GELU-derivative epilogue.
@@ -287,14 +290,14 @@ namespace
     }
 
     // ============================================================== forward
-    // CC = input channel chunks (2 or 4), a compile-time constant so that the MMA issue loop
-    // unrolls and every descriptor is a base plus a constant.
-    template <int CC>
+    // CC = input channel chunks (2 or 4) and NPAD = output channels, compile-time constants so that the
+    // MMA issue loop unrolls and every descriptor is a base plus a constant.
+    template <int CC, int NPAD>
     __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const FwdArgs a)
     {
         extern __shared__ __align__(1024) uint8_t smem[];
-        constexpr int cc = CC;
-        const int npad = a.npad, R = a.rows_per_cta;
+        constexpr int cc = CC, npad = NPAD;
+        const int R = a.rows_per_cta;
         const uint32_t wbytes = fwd_weight_bytes(cc, npad);
         const uint32_t slot_bytes = uint32_t(cc) * kRowPlane;
         const uint32_t tcols = fwd_tmem_cols(npad, R);
@@ -321,56 +324,60 @@ namespace
         const int nout = min(R, a.nrows - r0);
         const int nin = nout + 4;
 
-        if (threadIdx.x == 0)
-        {
-            // a row completes with its bulk copies and one arrival per wrapped site (below)
-            const int wrapped = (c0 == 0 ? 2 : 0) + (c0 + kTile == a.ncols ? 2 : 0);
-            for (int i = 0; i < R + 4; ++i) mbar_init(&full[i], 1 + cc * wrapped);
-            for (int i = 0; i < R; ++i) mbar_init(&accf[i], 1);
-            mbar_init(zbar, 256);
-            mbar_init(wbar, 1);
-            mbar_init(done, 1);
-            *abort = 0;
-            fence_mbar_init();
-        }
+        const int left = c0 == 0 ? 2 : 0, right = c0 + kTile == a.ncols ? 2 : 0;  // wrapped sites
         if (warp == 0)
         {
-            tmem_alloc(tslot, tcols);
-            tmem_relinquish();
+            // a row completes with its bulk copies and one arrival per wrapped site (below)
+            for (int i = lane; i < R + 4; i += 32) mbar_init(&full[i], 1 + cc * (left + right));
+            if (lane < R) mbar_init(&accf[lane], 1);
+            if (lane == 0)
+            {
+                mbar_init(zbar, 256);
+                mbar_init(wbar, 1);
+                mbar_init(done, 1);
+                *abort = 0;
+            }
+            fence_mbar_init();
+            asm volatile("bar.arrive 1, 320;" ::: "memory");  // the others need the barriers, this warp nothing of theirs
+            // The operand image and every input row of this CTA at once, one mbarrier per row, in the order the MMAs consume them. The window's sites c0-2 .. c0+129 of each
+            // (row, channel chunk): the in-range run by ONE bulk copy here; where the window wraps round the
+            // periodic row (first and last windows, 2 sites each side) the epilogue warps copy the wrapped
+            // 16-byte sites before their first wait (one mbarrier arrival each). The copies of a lane issue one
+            // after another, those of a warp's lanes closer together.
+            const int run = kSites - left - right;
+            if (lane == 0)
+            {
+                mbar_expect_tx(wbar, wbytes);
+                bulk_g2s(wsm, a.wimg, wbytes, wbar);
+            }
+            for (int i = lane; i < nin; i += 32) mbar_expect_tx(&full[i], uint32_t(cc * run) * 16u);
+            __syncwarp();
+            for (int it = lane; it < nin * cc; it += 32)
+            {
+                const int i = it / cc, q = it % cc;
+                const int row = wrap_row(r0 - 2 + i, a.nrows);
+                const uint16_t* src = a.in + (size_t(b * cc + q) * a.nrows + row) * size_t(a.ncols) * 8;
+                bulk_g2s(rows + i * slot_bytes + q * kRowPlane + left * 16, src + size_t(c0 - 2 + left) * 8,
+                         uint32_t(run) * 16u, &full[i]);
+            }
         }
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        const uint32_t tbase = *tslot;
+        else
+        {
+            if (warp == 1)
+            {
+                tmem_alloc(tslot, tcols);
+                tmem_relinquish();
+            }
+            tc_fence_before();
+            asm volatile("bar.sync 1, 320;" ::: "memory");
+            tc_fence_after();
+        }
+        const uint32_t tbase = warp ? *tslot : 0u;
 
         if (warp == 0)
         {
-            // The window's sites c0-2 .. c0+129 of each (row, channel chunk): the in-range run by
-            // ONE bulk copy here; where the window wraps round the periodic row (first and last
-            // windows, 2 sites each side) the epilogue warps copy the wrapped 16-byte sites
-            // before their first wait (one mbarrier arrival each).
-            const int left = c0 == 0 ? 2 : 0;
-            const int right = c0 + kTile == a.ncols ? 2 : 0;
-            const int lo = c0 - 2 + left;          // first in-range column of the window
-            const int run = kSites - left - right; // in-range sites
             if (lane == 0)
             {
-                // every input row of this CTA at once, one mbarrier per row, in the order
-                // the MMAs consume them
-                mbar_expect_tx(wbar, wbytes);
-                bulk_g2s(wsm, a.wimg, wbytes, wbar);
-                for (int i = 0; i < nin; ++i)
-                {
-                    const int row = wrap_row(r0 - 2 + i, a.nrows);
-                    mbar_expect_tx(&full[i], uint32_t(cc * run) * 16u);
-                    uint8_t* dst = rows + i * slot_bytes;
-                    for (int q = 0; q < cc; ++q)
-                    {
-                        const uint16_t* src = a.in + (size_t(b * cc + q) * a.nrows + row) * size_t(a.ncols) * 8;
-                        bulk_g2s(dst + q * kRowPlane + left * 16, src + size_t(lo) * 8, uint32_t(run) * 16u,
-                                 &full[i]);
-                    }
-                }
                 // no copy may still be in flight when the CTA exits
                 mbar_wait(wbar, 0, nullptr);
                 for (int i = 0; i < nin; ++i) mbar_wait(&full[i], 0, nullptr);
@@ -378,10 +385,10 @@ namespace
         }
         else if (warp == 1)
         {
-            if (lane == 0)
+            if (elect_one())
             {
                 const uint32_t wsa = smem_u32(wsm), rsa = smem_u32(rows);
-                const uint32_t kblock = 5u * npad * 16u;  // one (x tap, channel chunk) block of the image
+                constexpr uint32_t kblock = 5u * npad * 16u;  // one (x tap, channel chunk) block of the image
                 bool ok = mbar_wait(wbar, 0, abort) && mbar_wait(zbar, 0, abort);
                 tc_fence_after();
                 bool issued_any = false;
@@ -404,7 +411,7 @@ namespace
                         // address field (addresses stay below 256 KiB, so the 14-bit field never carries)
                         const uint64_t a0 = smem_desc(rsa + i * slot_bytes, kRowPlane, 128);
                         const uint64_t b0 = smem_desc(wsa + uint32_t(s_lo * npad * 16), kblock, 128);
-                        const uint64_t bstep = kblock >> 4;
+                        constexpr uint64_t bstep = kblock >> 4;
 #pragma unroll
                         for (int kx = 0; kx < 5; ++kx)
 #pragma unroll
@@ -450,8 +457,6 @@ namespace
             {
                 // the wrapped sites of the staged rows (see warp 0): 16-byte plain copies, made
                 // visible to the async proxy, one arrival on the row's mbarrier each
-                const int left = c0 == 0 ? 2 : 0;
-                const int right = c0 + kTile == a.ncols ? 2 : 0;
                 const int per_chunk = left + right, per_row = cc * per_chunk;
                 for (int it = int(threadIdx.x) - 64; it < nin * per_row; it += kFwdThreads - 64)
                 {
@@ -534,7 +539,7 @@ namespace
 
         tc_fence_before();
         __syncthreads();
-        if (warp == 0)
+        if (warp == 1)
         {
             tc_fence_after();
             tmem_dealloc(tbase, tcols);
@@ -651,7 +656,7 @@ namespace
         }
         else if (warp == 1)
         {
-            if (lane == 0)
+            if (elect_one())
             {
                 constexpr int N0 = G::COLS < 256 ? G::COLS : 256, N1 = G::COLS - N0;
                 const uint32_t id0 = idesc_bf16(128, N0, true, true), id1 = idesc_bf16(128, N1 > 0 ? N1 : 16, true, true);
@@ -668,6 +673,7 @@ namespace
                     tc_fence_after();
                     const uint32_t xa = sa + st * G::STAGE, za = xa + G::XB;
                     for (int kxi = 0; kxi < nkx; ++kxi)
+#pragma unroll
                         for (int ks = 0; ks < kTile / 16; ++ks)
                         {
                             const uint64_t ad = smem_desc(xa + uint32_t(ks * 16 + kx0 + kxi) * 16u, 128, kRowPlane);
@@ -1238,7 +1244,7 @@ namespace
     // Raises a kernel's dynamic shared-memory limit once per device (so that later
     // launches, e.g. inside a stream capture, make no attribute calls).
     std::mutex g_attr_mutex;
-    int g_attr_selftest[64], g_attr_fwd[64], g_attr_fwd2[64], g_attr_wgrad[4][64];
+    int g_attr_selftest[64], g_attr_fwd[4][64], g_attr_wgrad[4][64];
 
     cudaError_t set_smem_attr(const void* fn, uint32_t bytes, int (&done)[64])
     {
@@ -1323,9 +1329,12 @@ extern "C" int amb_conv5x5_forward(const void* in, int batch, int nrows, int nco
     a.rows_per_cta = choose_fwd_rows(batch, nrows, nwin, a.cin_chunks, npad);
     a.error = error;
     const uint32_t smem = fwd_smem_bytes(a.cin_chunks, npad, a.rows_per_cta);
-    auto kern = a.cin_chunks == 4 ? conv_fwd_kernel<4> : conv_fwd_kernel<2>;
-    cudaError_t e = set_smem_attr(reinterpret_cast<const void*>(kern), kSmemLimit,
-                                  a.cin_chunks == 4 ? g_attr_fwd : g_attr_fwd2);
+    const int which = (a.cin_chunks == 4 ? 0 : 2) + (npad == 32 ? 0 : 1);
+    using Kernel = void (*)(FwdArgs);
+    constexpr Kernel kernels[4] = {conv_fwd_kernel<4, 32>, conv_fwd_kernel<4, 16>, conv_fwd_kernel<2, 32>,
+                                   conv_fwd_kernel<2, 16>};
+    const Kernel kern = kernels[which];
+    cudaError_t e = set_smem_attr(reinterpret_cast<const void*>(kern), kSmemLimit, g_attr_fwd[which]);
     if (e == cudaSuccess)
     {
         const long long grid = (long long)batch * nwin * ((nrows + a.rows_per_cta - 1) / a.rows_per_cta);
