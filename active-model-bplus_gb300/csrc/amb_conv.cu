@@ -24,7 +24,7 @@
 // the output rows they own. Warp 0 stages rows, as soon as the barriers exist, while warp 1 allocates TMEM
 // and warps 2-9 zero it. One elected thread of warp 1 then issues the MMAs and commits one mbarrier per
 // finished output row, warps 2-9 run the epilogue (bias, GELU, its derivative, or FP32 output).
-// Six layers (5 -> 32 -> ... -> 2) at 512^2: 68 us in a graph; 79 with the MMAs issued under lane == 0 and
+// Six layers (5 -> 32 -> ... -> 2) at 512^2: 68 us in a graph (66 with the epilogue below), 79 with the MMAs issued under lane == 0 and
 // the rows requested once all warps were ready (128^2: 30.5 and 36.1). All layers in one cooperative
 // launch, with flags between neighbouring tiles, took longer than the launches that it saved. The data gradient of
 // a circular convolution is the forward convolution with the kernel flipped and
@@ -289,6 +289,76 @@ namespace
         }
     }
 
+    // The epilogue of output rows first, first + 2, .. of one lane quarter: `lanes` is the TMEM address of the
+    // quarter, `site` the lane's site in the tile's first row. A warp reads a whole row's channels at once, so
+    // the waits for the accumulators and for TMEM, which the MMAs keep busy, come once for 32 channels, and two
+    // rows are under way (a half row of 16 channels per warp: 68.3 us per forward at 512^2, 65.6 so). False if
+    // a wait gave up.
+    template <int NPAD, int EPI>
+    __device__ __forceinline__ bool epilogue_rows(const FwdArgs& a, uint64_t* accf, const volatile int* abort, uint32_t lanes,
+                                                  int first, int nout, int b, size_t site)
+    {
+        constexpr int NQ = NPAD / 8;
+        const size_t plane = size_t(a.nrows) * a.ncols;
+        float bias[NPAD];
+#pragma unroll
+        for (int e = 0; e < NPAD; ++e) bias[e] = EPI != EPI_GELU_BWD && a.bias ? a.bias[e] : 0.f;
+        for (int j = first; j < nout; j += 2)
+        {
+            const size_t at = site + size_t(j) * a.ncols;
+            uint4 gate[NQ];
+            if constexpr (EPI == EPI_GELU_BWD)
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                    gate[q] = *reinterpret_cast<const uint4*>(a.gate + ((size_t(b) * NQ + q) * plane + at) * 8);
+            if (!__all_sync(0xffffffffu, mbar_wait(&accf[j], 0, abort))) return false;
+            tc_fence_after();
+            float v[32];
+            if constexpr (NPAD == 32) tmem_ld32(lanes + uint32_t(j * NPAD), v);
+            else tmem_ld16(lanes + uint32_t(j * NPAD), v);
+            tmem_wait_ld();
+            if constexpr (EPI == EPI_F32)
+            {
+#pragma unroll
+                for (int e = 0; e < NPAD; ++e)
+                    if (e < a.cout) a.out_f32[(size_t(b) * a.cout + e) * plane + at] = v[e] + bias[e];
+            }
+            else
+            {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                {
+                    const size_t off = ((size_t(b) * NQ + q) * plane + at) * 8;
+                    float o[8];
+                    if constexpr (EPI == EPI_GELU)
+                    {
+                        float z[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                        {
+                            z[e] = v[8 * q + e] + bias[8 * q + e];
+                            o[e] = gelu_f(z[e]);
+                        }
+                        if (a.pre)
+                            *reinterpret_cast<uint4*>(a.pre + off) =
+                                make_uint4(pack_bf16x2(z[0], z[1]), pack_bf16x2(z[2], z[3]), pack_bf16x2(z[4], z[5]),
+                                           pack_bf16x2(z[6], z[7]));
+                    }
+                    else
+                    {
+                        float g[8];
+                        unpack_bf16x8(gate[q], g);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[e] = v[8 * q + e] * gelu_grad_f(g[e]);
+                    }
+                    *reinterpret_cast<uint4*>(a.out + off) = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]),
+                                                                        pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+                }
+            }
+        }
+        return true;
+    }
+
     // ============================================================== forward
     // CC = input channel chunks (2 or 4) and NPAD = output channels, compile-time constants so that the
     // MMA issue loop unrolls and every descriptor is a base plus a constant.
@@ -432,21 +502,9 @@ namespace
         }
         else
         {
-            // warps 2-9: lane quarter (warp % 4) of the tile, column half (warp - 2) / 4
+            // warps 2-9: lane quarter (warp % 4) of the tile, every other output row from (warp - 2) / 4 on
             const int q4 = warp & 3;  // the TMEM lane quarter this warp may access
             const int half = (warp - 2) >> 2;
-            const int m = q4 * 32 + lane;
-            const int col = c0 + m;
-            const int nq = npad / 8;
-            const bool active = half * 16 < npad;  // npad 16: the second half has no columns
-            const size_t plane = size_t(a.nrows) * a.ncols;
-            float bias[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e)
-            {
-                const int n = half * 16 + e;
-                bias[e] = (a.bias && n < npad) ? a.bias[n] : 0.f;
-            }
             // zero this warp's half of the accumulator columns in its lane quarter
             const uint32_t lanes = uint32_t(q4 * 32) << 16;
             for (uint32_t c = half * (tcols / 2); c < (half + 1) * (tcols / 2); c += 16)
@@ -473,68 +531,11 @@ namespace
                     mbar_arrive(&full[i]);
                 }
             }
-            for (int j = 0; j < nout; ++j)
-            {
-                bool ok = mbar_wait(&accf[j], 0, abort);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok)
-                {
-                    if (lane == 0) give_up(a.error, abort, 3);
-                    break;
-                }
-                tc_fence_after();
-                if (!active) continue;
-                float v[32];
-                tmem_ld16(tbase + lanes + uint32_t(j * npad + half * 16), v);
-                tmem_wait_ld();
-
-                const int row = r0 + j;
-                const size_t site = size_t(row) * a.ncols + col;
-                if (a.epilogue == EPI_F32)
-                {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                    {
-                        const int n = half * 16 + e;
-                        if (n < a.cout) a.out_f32[(size_t(b) * a.cout + n) * plane + site] = v[e] + bias[e];
-                    }
-                }
-                else
-                {
-#pragma unroll
-                    for (int qq = 0; qq < 2; ++qq)
-                    {
-                        const int q = half * 2 + qq;
-                        if (q >= nq) break;
-                        const size_t off = ((size_t(b) * nq + q) * plane + site) * 8;
-                        float o[8];
-                        if (a.epilogue == EPI_GELU)
-                        {
-                            float z[8];
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                            {
-                                z[e] = v[8 * qq + e] + bias[8 * qq + e];
-                                o[e] = gelu_f(z[e]);
-                            }
-                            if (a.pre)
-                                *reinterpret_cast<uint4*>(a.pre + off) =
-                                    make_uint4(pack_bf16x2(z[0], z[1]), pack_bf16x2(z[2], z[3]),
-                                               pack_bf16x2(z[4], z[5]), pack_bf16x2(z[6], z[7]));
-                        }
-                        else
-                        {
-                            float g[8];
-                            unpack_bf16x8(*reinterpret_cast<const uint4*>(a.gate + off), g);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) o[e] = v[8 * qq + e] * gelu_grad_f(g[e]);
-                        }
-                        *reinterpret_cast<uint4*>(a.out + off) =
-                            make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]),
-                                       pack_bf16x2(o[6], o[7]));
-                    }
-                }
-            }
+            const size_t site = size_t(r0) * a.ncols + c0 + q4 * 32 + lane;
+            const bool ok = a.epilogue == EPI_GELU  ? epilogue_rows<NPAD, EPI_GELU>(a, accf, abort, tbase + lanes, half, nout, b, site)
+                            : a.epilogue == EPI_F32 ? epilogue_rows<NPAD, EPI_F32>(a, accf, abort, tbase + lanes, half, nout, b, site)
+                                                    : epilogue_rows<NPAD, EPI_GELU_BWD>(a, accf, abort, tbase + lanes, half, nout, b, site);
+            if (!ok && lane == 0) give_up(a.error, abort, 3);
         }
 
         tc_fence_before();
