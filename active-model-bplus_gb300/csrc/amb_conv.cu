@@ -24,10 +24,11 @@
 // the output rows they own. Warp 0 stages rows, as soon as the barriers exist, while warp 1 allocates TMEM
 // and warps 2-9 zero it. One elected thread of warp 1 then issues the MMAs and commits one mbarrier per
 // finished output row, warps 2-9 run the epilogue (bias, GELU, its derivative, or FP32 output).
-// Six layers (5 -> 32 -> ... -> 2) at 512^2: 68 us in a graph (66 with the epilogue below), 79 with the MMAs issued under lane == 0 and
-// the rows requested once all warps were ready (128^2: 30.5 and 36.1). All layers in one cooperative
-// launch, with flags between neighbouring tiles, took longer than the launches that it saved. The data gradient of
-// a circular convolution is the forward convolution with the kernel flipped and
+// Six layers (5 -> 32 -> ... -> 2) at 512^2: 60 us in a graph, at 128^2 29.4 (79 and 36 with the MMAs issued under
+// lane == 0, the rows requested once all warps were ready and half a row's channels per epilogue warp): 0.42 us
+// of MMAs per staged row, 1.3 us before the first and 0.7 after the last. All
+// layers in one cooperative launch, with flags between neighbouring tiles, took longer than the launches that it
+// saved. The data gradient of a circular convolution is the forward convolution with the kernel flipped and
 // the channel roles swapped, so the same kernel serves it with the
 // GELU-derivative epilogue.
 //
@@ -36,8 +37,8 @@
 // M ((row, ci), 128 rows) and all dZ rows within two of them along N ((chunk, row, channel), up to 384), so ONE
 // instruction per x tap and 16 sites accumulates every (X row, dZ row) pair, of which the diagonals
 // ky = X row - dZ row are the taps: the other pairs (3 of 8) are not read. Both operands MN-major. Against
-// five y taps as separate 128 x 32 instructions, whose cost does not fall below that of N = 128, this
-// takes a sixth of the tensor time. A persistent CTA keeps its x taps' accumulators in TMEM over all its
+// five y taps as separate 128 x 32 instructions, each of which reads the whole A tile (33 of its 41 cycles),
+// this takes a third of the tensor time. A persistent CTA keeps its x taps' accumulators in TMEM over all its
 // row blocks (double-buffered bulk copies), sums the diagonals once at the end and writes one partial;
 // a second kernel reduces the partials in a fixed order (deterministic gradients). The same CTAs sum dZ
 // over the sites while it is staged (bias gradients).
@@ -459,38 +460,38 @@ namespace
             {
                 const uint32_t wsa = smem_u32(wsm), rsa = smem_u32(rows);
                 constexpr uint32_t kblock = 5u * npad * 16u;  // one (x tap, channel chunk) block of the image
-                bool ok = mbar_wait(wbar, 0, abort) && mbar_wait(zbar, 0, abort);
+                bool ok = mbar_wait(wbar, 0, abort) && mbar_wait(zbar, 0, abort) && mbar_wait(&full[0], 0, abort);
                 tc_fence_after();
                 bool issued_any = false;
+                // The tensor core holds few MMAs in its queue, so what the issuing thread does between rows must
+                // be short: rows unrolled by 4, so that descriptors are ready ahead, and the next row's barrier
+                // read while MMAs are queued (512^2, six layers: 65.6 us with neither, 63.1 and 60.0).
+#pragma unroll 4
                 for (int i = 0; ok && i < nin; ++i)
                 {
-                    if (!mbar_wait(&full[i], 0, abort))
-                    {
-                        ok = false;
-                        break;
-                    }
                     // slice s of this row's MMA feeds output row i - 4 + s (y tap 4 - s)
                     const int s_lo = i < 4 ? 4 - i : 0;
                     const int s_hi = nout + 3 - i < 4 ? nout + 3 - i : 4;
-                    if (s_lo <= s_hi)
+                    const uint32_t idesc = idesc_bf16(128, npad * (s_hi - s_lo + 1), false, false);
+                    const uint32_t d = tbase + uint32_t((i - 4 + s_lo) * npad);
+                    // base descriptors of this row; every MMA adds (byte offset >> 4) to the start
+                    // address field (addresses stay below 256 KiB, so the 14-bit field never carries)
+                    const uint64_t a0 = smem_desc(rsa + i * slot_bytes, kRowPlane, 128);
+                    const uint64_t b0 = smem_desc(wsa + uint32_t(s_lo * npad * 16), kblock, 128);
+                    constexpr uint64_t bstep = kblock >> 4;
+                    bool next = true;
+#pragma unroll
+                    for (int kx = 0; kx < 5; ++kx)
                     {
-                        const int n = npad * (s_hi - s_lo + 1);
-                        const uint32_t idesc = idesc_bf16(128, n, false, false);
-                        const uint32_t d = tbase + uint32_t((i - 4 + s_lo) * npad);
-                        // base descriptors of this row; every MMA adds (byte offset >> 4) to the start
-                        // address field (addresses stay below 256 KiB, so the 14-bit field never carries)
-                        const uint64_t a0 = smem_desc(rsa + i * slot_bytes, kRowPlane, 128);
-                        const uint64_t b0 = smem_desc(wsa + uint32_t(s_lo * npad * 16), kblock, 128);
-                        constexpr uint64_t bstep = kblock >> 4;
 #pragma unroll
-                        for (int kx = 0; kx < 5; ++kx)
-#pragma unroll
-                            for (int ks = 0; ks < cc / 2; ++ks)
-                                mma_bf16(d, a0 + uint64_t((2 * ks * kRowPlane + kx * 16) >> 4),
-                                         b0 + uint64_t(kx * cc + 2 * ks) * bstep, idesc, 1u);
-                        issued_any = true;
+                        for (int ks = 0; ks < cc / 2; ++ks)
+                            mma_bf16(d, a0 + uint64_t((2 * ks * kRowPlane + kx * 16) >> 4),
+                                     b0 + uint64_t(kx * cc + 2 * ks) * bstep, idesc, 1u);
+                        if (kx == 2 && i + 1 < nin) next = mbar_try_wait(&full[i + 1], 0);
                     }
+                    issued_any = true;
                     if (i >= 4) mma_commit(&accf[i - 4]);  // output row i - 4 has all five y taps
+                    ok = next || mbar_wait(&full[i + 1], 0, abort);
                 }
                 if (!ok) give_up(a.error, abort, 2);
                 if (issued_any)
