@@ -111,6 +111,10 @@ SIGNATURES = {
     "amb_conv5x5_wgrad_scratch_bytes": (ctypes.c_size_t, [_I, _I, _I, _I, _I]),
     "amb_conv5x5_wgrad": (_I, [_VP, _VP, _I, _I, _I, _I, _I, _VP, _VP, ctypes.c_size_t, _VP, _VP]),
     "amb_conv5x5_param_grads": (_I, [_VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP, _VP, _VP, ctypes.c_size_t, _VP, _VP]),
+    "amb_conv5x5_stack_images": (_I, [_I, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP]),
+    "amb_conv5x5_stack_forward": (_I, [_VP, _I, _I, _I, _I, _VP, _VP, _I, _VP, _VP, _VP, _VP, _VP, _VP, _VP]),
+    "amb_conv5x5_stack_backward": (_I, [_VP, _I, _I, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP,
+                                        ctypes.c_size_t, _VP, _VP]),
     "amb_conv5x5_images": (_I, [_VP, _I, _I, _I, _I, _VP, _VP, _VP]),
     "amb_learned_input": (_I, [_VP, _VP, _I, _I, _I, _VP, _VP]),
     "amb_learned_spectral_combine": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, ctypes.c_double, _I64, _VP, _VP, _VP]),

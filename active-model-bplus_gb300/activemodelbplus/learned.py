@@ -55,6 +55,15 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
+def _ptrs(tensors):
+    """Host array of the tensors' device pointers."""
+    return (ctypes.c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
+
+
+def _ints(values):
+    return (ctypes.c_int * len(values))(*values)
+
+
 # ------------------------------------------------------------------ layouts
 
 def to_chunks(x, cpad: int):
@@ -211,19 +220,19 @@ class FluxNet:
             self._dimages = [None] + [dgrad_image(self.weights[l], self.cin[l], self.npad[l])
                                       for l in range(1, self.nlayers)]
             return
-        # one kernel per layer builds both images, in a buffer of their own (a captured macro step
-        # keeps reading the images that it was captured with)
-        sizes = [25 * self.cin[l] * self.npad[l] for l in range(self.nlayers)]
+        # one kernel builds all images, in a buffer of their own (a captured macro step keeps reading the
+        # images that it was captured with)
+        L = self.nlayers
+        sizes = [25 * self.cin[l] * self.npad[l] for l in range(L)]
         buf = torch.empty(2 * sum(sizes), dtype=torch.bfloat16, device=self.weights[0].device)
         self._images, self._dimages, at = [], [], 0
-        for l, (w, n) in enumerate(zip(self.weights, sizes)):
-            img, dimg = buf[at:at + n], buf[at + n:at + 2 * n] if l else None
+        for l, n in enumerate(sizes):
+            self._images.append(buf[at:at + n])
+            self._dimages.append(buf[at + n:at + 2 * n] if l else None)
             at += 2 * n
-            w = w.detach().to(torch.float32).contiguous()
-            _check(N.lib().amb_conv5x5_images(_ptr(w), self.cout[l], self.cin_used[l], self.cin[l], self.npad[l],
-                                              _ptr(img), _ptr(dimg), _stream()))
-            self._images.append(img)
-            self._dimages.append(dimg)
+        ws = [w.detach().to(torch.float32).contiguous() for w in self.weights]
+        _check(N.lib().amb_conv5x5_stack_images(L, _ptrs(ws), _ints(self.cout), _ints(self.cin_used), _ints(self.cin),
+                                                _ints(self.npad), _ptrs(self._images), _ptrs(self._dimages), _stream()))
 
     def state_dict(self) -> dict:
         d = {}
@@ -259,24 +268,21 @@ class FluxNet:
         torch = _torch()
         if self._images is None:
             self.refresh()
-        B, _, H, W, _ = x.shape
-        a = x
-        inputs, pres = [], []
-        for l in range(self.nlayers - 1):
-            out = torch.empty(B, self.npad[l] // 8, H, W, 8, dtype=torch.bfloat16, device=x.device)
-            pre = torch.empty_like(out) if train else None
-            conv_forward(a, self._images[l], self.biases[l], cin=self.cin[l], npad=self.npad[l],
-                         epilogue=N.AMB_EPI_GELU, out=out, pre=pre, error=self.error)
-            if train:
-                inputs.append(a)
-                pres.append(pre)
-            a = out
+        B, q, H, W, e = x.shape
+        if q * 8 != self.cin[0] or e != 8:
+            raise ValueError("input is not in chunk-plane layout with cin channels")
+        L = self.nlayers
+        # the hidden activations of a training pass and their pre-activations, or two that take turns
+        acts = torch.empty(2 * (L - 1) if train else min(2, L - 1), B, HIDDEN // 8, H, W, 8, dtype=torch.bfloat16,
+                           device=x.device)
+        outs = [acts[l if train else l % 2] for l in range(L - 1)]
+        pres = [acts[L - 1 + l] if train else None for l in range(L - 1)]
         flux = torch.empty(B, NOUT, H, W, dtype=torch.float32, device=x.device)
-        conv_forward(a, self._images[-1], self.biases[-1], cin=self.cin[-1], npad=self.npad[-1], cout=NOUT,
-                     epilogue=N.AMB_EPI_F32, out_f32=flux, error=self.error)
+        _check(N.lib().amb_conv5x5_stack_forward(
+            _ptr(x), B, H, W, L, _ints(self.cin), _ints(self.npad), NOUT, _ptrs(self._images), _ptrs(self.biases),
+            _ptrs(outs + [None]), _ptrs(pres + [None]), _ptr(flux), _ptr(self.error), _stream()))
         if train:
-            inputs.append(a)
-            self._saved = (inputs, pres)
+            self._saved = ([x] + outs, pres)
         return flux
 
     def backward(self, dflux):
@@ -285,21 +291,22 @@ class FluxNet:
         if self._saved is None:
             raise RuntimeError("backward() needs a preceding forward(train=True)")
         inputs, pres = self._saved
-        gw, gb = [None] * self.nlayers, [None] * self.nlayers
-        dz = to_chunks(dflux, NOUT_PAD)
-        L = self.nlayers - 1
-        gw[L], _ = param_grads(inputs[L], dz, cin=self.cin[L], npad=self.npad[L], cin_used=self.cin_used[L],
-                               cout=self.cout[L], scratch=self._scratch, bias=False, error=self.error)
-        gb[L] = torch.nn.functional.pad(dflux.sum(dim=(0, 2, 3)), (0, NOUT_PAD - NOUT))
-        B, _, H, W, _ = dz.shape
-        for l in range(L, 0, -1):
-            prev = torch.empty(B, self.cin[l] // 8, H, W, 8, dtype=torch.bfloat16, device=dz.device)
-            conv_forward(dz, self._dimages[l], None, cin=self.npad[l], npad=self.cin[l],
-                         epilogue=N.AMB_EPI_GELU_BWD, out=prev, gate=pres[l - 1], error=self.error)
-            dz = prev
-            k = l - 1
-            gw[k], gb[k] = param_grads(inputs[k], dz, cin=self.cin[k], npad=self.npad[k], cin_used=self.cin_used[k],
-                                       cout=self.cout[k], scratch=self._scratch, error=self.error)
+        lib, L = N.lib(), self.nlayers
+        B, _, H, W, _ = inputs[0].shape
+        if tuple(dflux.shape) != (B, NOUT, H, W):
+            raise ValueError(f"dflux has shape {tuple(dflux.shape)}, the flux {(B, NOUT, H, W)}")
+        dev, f32 = dflux.device, torch.float32
+        d = dflux.to(f32).contiguous()
+        gw = [torch.empty(self.cout[l], self.cin_used[l], 5, 5, dtype=f32, device=dev) for l in range(L)]
+        gb = [torch.empty(self.npad[l], dtype=f32, device=dev) for l in range(L - 1)]
+        gb.append(torch.nn.functional.pad(dflux.sum(dim=(0, 2, 3)), (0, NOUT_PAD - NOUT)))
+        dz = torch.empty(2, B, HIDDEN // 8, H, W, 8, dtype=torch.bfloat16, device=dev)
+        shapes = {(self.cin[l], self.npad[l]) for l in range(L)}
+        scratch = self._scratch.get(max(lib.amb_conv5x5_wgrad_scratch_bytes(B, H, W, c, n) for c, n in shapes), dev)
+        _check(lib.amb_conv5x5_stack_backward(
+            _ptr(d), B, H, W, L, _ints(self.cin), _ints(self.cin_used), _ints(self.npad), _ints(self.cout), _ptrs(inputs),
+            _ptrs(pres + [None]), _ptrs(self._dimages), _ptr(dz[0]), _ptr(dz[1]), _ptrs(gw), _ptrs(gb[:-1] + [None]),
+            _ptr(scratch), scratch.numel() * 4, _ptr(self.error), _stream()))
         self._saved = None
         return gw, gb
 

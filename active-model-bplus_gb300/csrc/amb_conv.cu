@@ -912,18 +912,29 @@ namespace
         }
     }
 
-    // Operand images of one layer's weights w [cout][cin][5][5]: the forward convolution's
-    // [5 kx][cin_pad/8][5 (4 - ky)][npad][8] and, with the kernel flipped and the channel roles swapped, the data
-    // gradient's [5 kx][npad/8][5 (4 - ky)][cin_pad][8], zero in the padding.
-    __global__ void weight_images_kernel(const float* __restrict__ w, int cout, int cin, int cin_pad, int npad,
-                                         __nv_bfloat16* __restrict__ img, __nv_bfloat16* __restrict__ dimg)
+    // Operand images of the layers' weights w [cout][cin][5][5], one layer per blockIdx.y: the forward
+    // convolution's [5 kx][cin_pad/8][5 (4 - ky)][npad][8] and, with the kernel flipped and the channel roles
+    // swapped, the data gradient's [5 kx][npad/8][5 (4 - ky)][cin_pad][8], zero in the padding.
+    constexpr int kImageLayers = 8;
+    struct ImageArgs
     {
-        const int n = 25 * cin_pad * npad;
+        struct Layer
+        {
+            const float* w;
+            __nv_bfloat16 *img, *dimg;
+            int cout, cin, cin_pad, npad;
+        } layer[kImageLayers];
+    };
+
+    __global__ void weight_images_kernel(const __grid_constant__ ImageArgs args)
+    {
+        const ImageArgs::Layer& a = args.layer[blockIdx.y];
+        const int n = 25 * a.cin_pad * a.npad;
         for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * n; t += gridDim.x * blockDim.x)
         {
             const bool fwd = t < n;
-            if (!(fwd ? img : dimg)) continue;
-            const int k = fwd ? cin_pad : npad, m = fwd ? npad : cin_pad;  // channels along K, along N
+            if (!(fwd ? a.img : a.dimg)) continue;
+            const int k = fwd ? a.cin_pad : a.npad, m = fwd ? a.npad : a.cin_pad;  // channels along K, along N
             int e = fwd ? t : t - n;
             const int e0 = e % 8;
             e /= 8;
@@ -934,8 +945,25 @@ namespace
             const int kc = (e % (k / 8)) * 8 + e0, kx = e / (k / 8);
             const int co = fwd ? row : kc, ci = fwd ? kc : row;
             float v = 0.f;
-            if (co < cout && ci < cin) v = w[((size_t(co) * cin + ci) * 5 + (fwd ? 4 - s : s)) * 5 + (fwd ? kx : 4 - kx)];
-            (fwd ? img : dimg)[fwd ? t : t - n] = __float2bfloat16_rn(v);
+            if (co < a.cout && ci < a.cin)
+                v = a.w[((size_t(co) * a.cin + ci) * 5 + (fwd ? 4 - s : s)) * 5 + (fwd ? kx : 4 - kx)];
+            (fwd ? a.img : a.dimg)[fwd ? t : t - n] = __float2bfloat16_rn(v);
+        }
+    }
+
+    // FP32 planes [batch][c][plane] as bf16 chunk planes [batch][npad/8][plane][8], zero from channel c on.
+    __global__ void chunk_kernel(const float* __restrict__ x, int c, int npad, size_t plane, size_t n, uint4* __restrict__ out)
+    {
+        for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < n; t += size_t(gridDim.x) * blockDim.x)
+        {
+            const size_t s = t % plane, r = t / plane;
+            const int q = int(r % (npad / 8));
+            const float* p = x + (r / (npad / 8)) * c * plane + s;
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = 8 * q + e < c ? p[(8 * q + e) * plane] : 0.f;
+            out[t] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                pack_bf16x2(v[6], v[7]));
         }
     }
 
@@ -1464,16 +1492,87 @@ extern "C" int amb_conv5x5_param_grads(const void* x, const void* dz, int batch,
                        scratch, scratch_bytes, error, stream);
 }
 
+extern "C" int amb_conv5x5_stack_images(int layers, const float* const* w, const int* cout, const int* cin,
+                                        const int* cin_pad, const int* npad, void* const* img, void* const* dimg,
+                                        void* stream)
+{
+    if (layers < 1 || !w || !cout || !cin || !cin_pad || !npad || !img || !dimg)
+        return fail_invalid("amb_conv5x5_images: bad arguments");
+    cudaError_t e = cudaSuccess;
+    for (int l0 = 0; l0 < layers && e == cudaSuccess; l0 += kImageLayers)
+    {
+        ImageArgs a{};
+        const int count = std::min(kImageLayers, layers - l0);
+        int most = 0;
+        for (int i = 0; i < count; ++i)
+        {
+            const int l = l0 + i;
+            if (!w[l] || (!img[l] && !dimg[l]) || cin[l] < 1 || cout[l] < 1 || cin[l] > cin_pad[l] || cout[l] > npad[l] ||
+                cin_pad[l] % 8 || npad[l] % 8)
+                return fail_invalid("amb_conv5x5_images: bad arguments");
+            a.layer[i] = {w[l], static_cast<__nv_bfloat16*>(img[l]), static_cast<__nv_bfloat16*>(dimg[l]), cout[l], cin[l],
+                          cin_pad[l], npad[l]};
+            most = std::max(most, 2 * 25 * cin_pad[l] * npad[l]);
+        }
+        weight_images_kernel<<<dim3((most + 255) / 256, count), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+        e = cudaGetLastError();
+    }
+    return e == cudaSuccess ? AMB_OK : fail_cuda("amb_conv5x5_images", e);
+}
+
 extern "C" int amb_conv5x5_images(const float* w, int cout, int cin, int cin_pad, int npad, void* img, void* dimg,
                                   void* stream)
 {
-    if (!w || (!img && !dimg) || cin < 1 || cout < 1 || cin > cin_pad || cout > npad || cin_pad % 8 || npad % 8)
-        return fail_invalid("amb_conv5x5_images: bad arguments");
-    const int n = 2 * 25 * cin_pad * npad;
-    weight_images_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        w, cout, cin, cin_pad, npad, static_cast<__nv_bfloat16*>(img), static_cast<__nv_bfloat16*>(dimg));
+    return amb_conv5x5_stack_images(1, &w, &cout, &cin, &cin_pad, &npad, &img, &dimg, stream);
+}
+
+extern "C" int amb_conv5x5_stack_forward(const void* in, int batch, int nrows, int ncols, int layers, const int* cin,
+                                         const int* npad, int cout, const void* const* wimg, const float* const* bias,
+                                         void* const* out, void* const* pre, float* out_f32, int* error, void* stream)
+{
+    if (layers < 1 || !cin || !npad || !wimg || !bias || !out || !pre)
+        return fail_invalid("amb_conv5x5_stack_forward: bad arguments");
+    for (int l = 0; l < layers; ++l)
+    {
+        if (l && cin[l] != npad[l - 1])
+            return fail_invalid("amb_conv5x5_stack_forward: each layer's cin must be the npad before it");
+        const bool last = l == layers - 1;
+        const int rc = amb_conv5x5_forward(l ? out[l - 1] : in, batch, nrows, ncols, cin[l], wimg[l], bias[l], npad[l],
+                                           last ? cout : npad[l], last ? EPI_F32 : EPI_GELU, last ? nullptr : out[l],
+                                           last ? nullptr : pre[l], nullptr, last ? out_f32 : nullptr, error, stream);
+        if (rc != AMB_OK) return rc;
+    }
+    return AMB_OK;
+}
+
+extern "C" int amb_conv5x5_stack_backward(const float* dout, int batch, int nrows, int ncols, int layers, const int* cin,
+                                          const int* cin_used, const int* npad, const int* cout, const void* const* x,
+                                          const void* const* pre, const void* const* dimg, void* dz0, void* dz1,
+                                          float* const* gw, float* const* gb, float* scratch, size_t scratch_bytes,
+                                          int* error, void* stream)
+{
+    if (!dout || layers < 1 || !cin || !cin_used || !npad || !cout || !x || !pre || !dimg || !dz0 || (layers > 1 && !dz1) ||
+        !gw || !gb || !valid_geometry(batch, nrows, ncols) || (npad[layers - 1] != 16 && npad[layers - 1] != 32) ||
+        cout[layers - 1] < 1 || cout[layers - 1] > npad[layers - 1] || (reinterpret_cast<uintptr_t>(dz0) & 15))
+        return fail_invalid("amb_conv5x5_stack_backward: bad arguments");
+    const size_t plane = size_t(nrows) * ncols, n = plane * batch * (npad[layers - 1] / 8);
+    const int grid = int(std::min<size_t>((n + 255) / 256, size_t(sm_count()) * 16));
+    chunk_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(dout, cout[layers - 1], npad[layers - 1], plane, n,
+                                                                      static_cast<uint4*>(dz0));
     cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? AMB_OK : fail_cuda("amb_conv5x5_images", e);
+    if (e != cudaSuccess) return fail_cuda("amb_conv5x5_stack_backward", e);
+    void *dz = dz0, *prev = dz1;
+    for (int l = layers - 1; l >= 0; --l)
+    {
+        int rc = amb_conv5x5_param_grads(x[l], dz, batch, nrows, ncols, cin[l], npad[l], cin_used[l], cout[l], gw[l], gb[l],
+                                         scratch, scratch_bytes, error, stream);
+        if (rc == AMB_OK && l > 0)
+            rc = amb_conv5x5_forward(dz, batch, nrows, ncols, npad[l], dimg[l], nullptr, cin[l], cin[l], EPI_GELU_BWD, prev,
+                                     nullptr, pre[l - 1], nullptr, error, stream);
+        if (rc != AMB_OK) return rc;
+        std::swap(dz, prev);
+    }
+    return AMB_OK;
 }
 
 extern "C" int amb_learned_input(const float* phi, const float* params, int batch, int nrows, int ncols, void* x,

@@ -353,6 +353,22 @@ int amb_conv5x5_param_grads(const void* x, const void* dz, int batch, int nrows,
  * and npad output channels, dimg for its data gradient (npad input, cin_pad output); either may be NULL. */
 int amb_conv5x5_images(const float* w, int cout, int cin, int cin_pad, int npad, void* img, void* dimg, void* stream);
 
+/* The same for a stack of layers in one call each. Arrays are host arrays of one value per layer.
+ * images: one launch. forward: GELU after all layers but the last, whose `cout` channels go to out_f32; out[l] (and, if
+ * not NULL, pre[l]) of all layers but the last, out[l] the input of layer l + 1. backward: the gradients gw and gb (NULL
+ * entries: not formed) for dout [batch][cout of the last][nrows][ncols], given the layers' inputs x and
+ * pre-activations pre; dz0 and dz1 hold one activation of the widest layer each; scratch: the most that
+ * amb_conv5x5_wgrad_scratch_bytes gives for a layer. */
+int amb_conv5x5_stack_images(int layers, const float* const* w, const int* cout, const int* cin, const int* cin_pad,
+                             const int* npad, void* const* img, void* const* dimg, void* stream);
+int amb_conv5x5_stack_forward(const void* in, int batch, int nrows, int ncols, int layers, const int* cin,
+                              const int* npad, int cout, const void* const* wimg, const float* const* bias,
+                              void* const* out, void* const* pre, float* out_f32, int* error, void* stream);
+int amb_conv5x5_stack_backward(const float* dout, int batch, int nrows, int ncols, int layers, const int* cin,
+                               const int* cin_used, const int* npad, const int* cout, const void* const* x,
+                               const void* const* pre, const void* const* dimg, void* dz0, void* dz1, float* const* gw,
+                               float* const* gb, float* scratch, size_t scratch_bytes, int* error, void* stream);
+
 /* Network input planes (16 channels, 2 chunks): bf16(phi), 256*(phi - bf16(phi)), zeta/4,
  * lambda, 10*T, zeros. phi: [batch][nrows][ncols] FP32; params: [batch][3] = (zeta, lambda, T). */
 int amb_learned_input(const float* phi, const float* params, int batch, int nrows, int ncols, void* x, void* stream);

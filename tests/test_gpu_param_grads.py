@@ -44,3 +44,48 @@ def test_images(cin_used, cin, cout, npad):
                                       torch.cuda.current_stream().cuda_stream) == 0
     assert torch.equal(img, L.weight_image(w, cin, npad).reshape(-1))
     assert torch.equal(dimg, L.dgrad_image(w, cin, npad).reshape(-1))
+
+
+@pytest.mark.parametrize("layers", [2, 3, 9])
+@pytest.mark.parametrize("shape", [(1, 3, 128), (3, 13, 256)])
+def test_stack_equals_the_layers(shape, layers):
+    """One call for all layers: bitwise the layers' own calls (images of more layers than one launch takes,
+    activations that take turns, gradients handed down through two buffers)."""
+    import torch
+    from activemodelbplus import learned as L
+    from activemodelbplus.integrator import _native as N
+    B, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(layers)
+    net = L.FluxNet(seed=5, layers=layers)
+    for b in net.biases[:-1]:
+        b.normal_(0, 0.1, generator=g)
+    x = torch.randn(B, 2, H, W, 8, device="cuda", generator=g).to(torch.bfloat16)
+    dflux = torch.randn(B, 2, H, W, device="cuda", generator=g)
+    flux = net.forward(x, train=True)
+    gw, gb = net.backward(dflux)
+    assert torch.equal(net.forward(x), flux)
+    img = [L.weight_image(w, net.cin[l], net.npad[l]) for l, w in enumerate(net.weights)]
+    dimg = [None] + [L.dgrad_image(net.weights[l], net.cin[l], net.npad[l]) for l in range(1, layers)]
+    acts, pres = [x], []
+    for l in range(layers - 1):
+        out = torch.empty(B, 4, H, W, 8, dtype=torch.bfloat16, device="cuda")
+        pres.append(torch.empty_like(out))
+        L.conv_forward(acts[-1], img[l], net.biases[l], cin=net.cin[l], npad=32, epilogue=N.AMB_EPI_GELU, out=out, pre=pres[-1])
+        acts.append(out)
+    want = torch.empty_like(flux)
+    L.conv_forward(acts[-1], img[-1], net.biases[-1], cin=32, npad=16, cout=2, epilogue=N.AMB_EPI_F32, out_f32=want)
+    assert torch.equal(flux, want)
+    dz = L.to_chunks(dflux, 16)
+    for l in range(layers - 1, -1, -1):
+        rw, rb = L.param_grads(acts[l], dz, cin=net.cin[l], npad=net.npad[l], cin_used=net.cin_used[l], cout=net.cout[l],
+                               scratch=L._Scratch())
+        assert torch.equal(gw[l], rw)
+        if l == layers - 1:
+            assert torch.allclose(gb[l][:2], dflux.sum(dim=(0, 2, 3)), rtol=1e-5, atol=1e-3) and not gb[l][2:].any()
+        else:
+            assert torch.equal(gb[l], rb)
+        if l:
+            prev = torch.empty(B, 4, H, W, 8, dtype=torch.bfloat16, device="cuda")
+            L.conv_forward(dz, dimg[l], None, cin=net.npad[l], npad=32, epilogue=N.AMB_EPI_GELU_BWD, out=prev, gate=pres[l - 1])
+            dz = prev
+    net.check_error()
