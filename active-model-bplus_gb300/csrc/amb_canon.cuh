@@ -1,6 +1,6 @@
 // The step's arithmetic, defined once for every kernel that evaluates it.
 //
-// Every FP32/FP64 step kernel (the shared-memory tile kernel, the warp-pair sliding kernel)
+// Every FP32/FP64 step kernel (tiles, sliding strips, grid-wide phases)
 // evaluates the same operations in the same order at every site,
 // each rounded exactly once as written here (explicit round-to-nearest intrinsics: the
 // compiler may not contract or reorder them), from the same constants (computed once on the

@@ -279,7 +279,7 @@ namespace amb
             uint2 rnext[R];
 
             // Output rows don't wrap; a row past the segment's last is computed from rows in range and not stored.
-            __device__ __forceinline__ int at(int j) const { return R == 1 ? min(grow, ny - 1) : min(grow + j, ny - 1); }
+            __device__ __forceinline__ int at(int j) const { return min(grow + j, ny - 1); }
             __device__ __forceinline__ void ahead()
             {
 #pragma unroll

@@ -293,7 +293,7 @@ def fp64_path(w, stencil, model, field, nsteps: int = 20):
     sec = e0.elapsed_time(e1) / 1e3
     sites = w["ny"] * w["nx"]
     return {"value": nsteps * sites / sec / 1e9, "unit": UNIT, "dtype": "f64",
-            "sample": f"{nsteps} steps of the {w['ny']}x{w['nx']} workload, tile kernel (512-thread CTAs), CUDA events"}
+            "sample": f"{nsteps} steps of the {w['ny']}x{w['nx']} workload, CUDA events"}
 
 
 def reference_gpu_baseline(w, nsteps: int = 20):
