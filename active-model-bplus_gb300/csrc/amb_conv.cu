@@ -1154,6 +1154,30 @@ namespace
         return (long long)__float2int_rn(q);  // |q| <= 1e9 < 2^31: the same value as a 64-bit conversion
     }
 
+    // One site's new fixed-point value from its four face increments, with the checks that fail a span.
+    __device__ __forceinline__ int updated_q(int q0, long long dq, bool finite, long long bound, bool* bad)
+    {
+        long long q = (long long)q0 - dq;
+        if (!finite || q > bound || q < -bound)
+        {
+            *bad = true;
+            q = q > bound ? bound : (q < -bound ? -bound : q);
+        }
+        return int32_t(q);
+    }
+
+    // q * 2^-24 rounded once to FP32: rounding q to FP32 and scaling by a power of two gives the same value
+    // (|q| <= 2e9, so the scaled value is a normal number or zero)
+    __device__ __forceinline__ float field_of(int q) { return __fmul_rn(__int2float_rn(q), 1.0f / 16777216.0f); }
+
+    // Channel chunk 0 of the next network input, as learned_input_kernel forms it.
+    __device__ __forceinline__ uint4 input_chunk(float f, float p0, float p1, float p2)
+    {
+        const __nv_bfloat16 hi = __float2bfloat16_rn(f);
+        const float lo = (f - __bfloat162float(hi)) * 256.f;
+        return make_uint4(pack_bf16x2(__bfloat162float(hi), lo), pack_bf16x2(p0 * 0.25f, p1), pack_bf16x2(p2 * 10.f, 0.f), 0u);
+    }
+
     // phi_q -= sum of integer face increments (each face computed identically by the two
     // sites that share it, so the sum over all sites is unchanged: exact conservation).
     __global__ void learned_update_kernel(const float* __restrict__ flux, const float* __restrict__ extra,
@@ -1184,25 +1208,71 @@ namespace
                            face_q(fx, ex, xx, noise_mag, scale_x, r, cm, 0, 1, nrows, ncols) +
                            face_q(fy, ey, xy, noise_mag, scale_y, r, c, 1, 0, nrows, ncols) -
                            face_q(fy, ey, xy, noise_mag, scale_y, rm, c, 1, 0, nrows, ncols);
-            long long q = (long long)phi_q[i] - dq;
-            bool bad = !isfinite(fx[i]) || !isfinite(fy[i]) || q > bound || q < -bound;
-            if (extra) bad = bad || !isfinite(ex[i]) || !isfinite(ey[i]);
-            if (bad)
-            {
-                atomicOr(flag, 1);
-                q = q > bound ? bound : (q < -bound ? -bound : q);
-            }
-            phi_q[i] = int32_t(q);
-            // q * 2^-24 rounded once to FP32: rounding q to FP32 and scaling by a power of two gives the
-            // same value (|q| <= 2e9, so the scaled value is a normal number or zero)
-            const float f = __fmul_rn(__int2float_rn(int(q)), 1.0f / 16777216.0f);
+            bool bad = false;
+            const bool finite = isfinite(fx[i]) && isfinite(fy[i]) && (!extra || (isfinite(ex[i]) && isfinite(ey[i])));
+            const int q = updated_q(phi_q[i], dq, finite, bound, &bad);
+            if (bad) atomicOr(flag, 1);
+            phi_q[i] = q;
+            const float f = field_of(q);
             phi_f[i] = f;
-            if (x_next)  // channel chunk 0 of the next network input, as learned_input_kernel forms it
+            if (x_next) x_next[i] = input_chunk(f, params[0], params[1], params[2]);
+        }
+    }
+
+    // The same on four columns per thread, for rows of whole aligned 16-byte quads and no per-site noise: a quarter of
+    // the threads, 13 faces instead of 16 and wide accesses (a macro step at
+    // 512^2: 82.6 -> 80.0 us, at 768^2 156.4 -> 147.7).
+    __global__ void learned_update_quad_kernel(const float* __restrict__ flux, const float* __restrict__ extra, int nrows,
+                                               int ncols, float scale_y, float scale_x, int32_t* __restrict__ phi_q,
+                                               float* __restrict__ phi_f, long long bound, int* __restrict__ flag,
+                                               int64_t* __restrict__ advance, const float* __restrict__ params,
+                                               uint4* __restrict__ x_next)
+    {
+        if (advance && blockIdx.x == 0 && threadIdx.x == 0) *advance += 1;
+        const size_t plane = size_t(nrows) * ncols;
+        const int quads = ncols / 4;
+        const size_t n = size_t(nrows) * quads;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const auto load = [](const float* p, size_t i) { return *reinterpret_cast<const float4*>(p + i); };
+        const auto face = [&](float f, float e, float scale) {
+            const float q = __fmul_rn(scale, extra ? __fadd_rn(f, e) : f);
+            return (long long)__float2int_rn(q > 1e9f ? 1e9f : (q < -1e9f ? -1e9f : q));
+        };
+        for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < n; t += size_t(gridDim.x) * blockDim.x)
+        {
+            const int r = int(t / quads), c = int(t - size_t(r) * quads) * 4;
+            const size_t row = size_t(r) * ncols, up = size_t(r == 0 ? nrows - 1 : r - 1) * ncols;
+            const size_t left = row + (c == 0 ? ncols - 1 : c - 1);
+            const float4 fy = load(flux, row + c), fx = load(flux + plane, row + c), fu = load(flux, up + c);
+            const float4 ey = extra ? load(extra, row + c) : zero, ex = extra ? load(extra + plane, row + c) : zero,
+                         eu = extra ? load(extra, up + c) : zero;
+            const float fl = flux[plane + left], el = extra ? extra[plane + left] : 0.f;
+            const int4 q0 = *reinterpret_cast<const int4*>(phi_q + row + c);
+            const float vy[4] = {fy.x, fy.y, fy.z, fy.w}, vx[4] = {fx.x, fx.y, fx.z, fx.w}, vu[4] = {fu.x, fu.y, fu.z, fu.w};
+            const float wy[4] = {ey.x, ey.y, ey.z, ey.w}, wx[4] = {ex.x, ex.y, ex.z, ex.w}, wu[4] = {eu.x, eu.y, eu.z, eu.w};
+            const int qs[4] = {q0.x, q0.y, q0.z, q0.w};
+            long long before = face(fl, el, scale_x);
+            int q[4];
+            float f[4];
+            bool bad = false;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
             {
-                const __nv_bfloat16 hi = __float2bfloat16_rn(f);
-                const float lo = (f - __bfloat162float(hi)) * 256.f;
-                x_next[i] = make_uint4(pack_bf16x2(__bfloat162float(hi), lo), pack_bf16x2(params[0] * 0.25f, params[1]),
-                                       pack_bf16x2(params[2] * 10.f, 0.f), 0u);
+                const long long here = face(vx[k], wx[k], scale_x);
+                const long long dq = here - before + face(vy[k], wy[k], scale_y) - face(vu[k], wu[k], scale_y);
+                before = here;
+                const bool finite = isfinite(vx[k]) && isfinite(vy[k]) && isfinite(wx[k]) && isfinite(wy[k]);
+                q[k] = updated_q(qs[k], dq, finite, bound, &bad);
+                f[k] = field_of(q[k]);
+            }
+            if (bad) atomicOr(flag, 1);
+            *reinterpret_cast<int4*>(phi_q + row + c) = make_int4(q[0], q[1], q[2], q[3]);
+            *reinterpret_cast<float4*>(phi_f + row + c) = make_float4(f[0], f[1], f[2], f[3]);
+            if (x_next)
+            {
+                const float p0 = params[0], p1 = params[1], p2 = params[2];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x_next[row + c + k] = input_chunk(f[k], p0, p1, p2);
             }
         }
     }
@@ -1608,7 +1678,17 @@ static int learned_update_launch(const float* flux, const float* extra, int nrow
     const double fix = 16777216.0;
     const double qb = std::min(bound * fix, 2.0e9);
     const bool noisy = xi && noise_mag > 0;
-    learned_update_kernel<<<grid, 256, 0, s>>>(flux, extra, noisy ? xi : nullptr, nrows, ncols,
+    const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    if (!noisy && ncols % 4 == 0 && al16(flux) && al16(extra) && al16(phi_q) && al16(phi_f))
+    {
+        const size_t quads = size_t(nrows) * (ncols / 4);
+        const int blocks = int(std::min<size_t>((quads + 127) / 128, size_t(sm_count()) * 16));
+        learned_update_quad_kernel<<<blocks, 128, 0, s>>>(flux, extra, nrows, ncols, float(dt_macro / dy * fix),
+                                                          float(dt_macro / dx * fix), phi_q, phi_f, (long long)qb, flag,
+                                                          step_to_advance, params, static_cast<uint4*>(x_next));
+    }
+    else
+        learned_update_kernel<<<grid, 256, 0, s>>>(flux, extra, noisy ? xi : nullptr, nrows, ncols,
                                                float(dt_macro / dy * fix), float(dt_macro / dx * fix),
                                                noisy ? float(noise_mag) : 0.f, phi_q, phi_f, (long long)qb, flag,
                                                step_to_advance, params, static_cast<uint4*>(x_next));
