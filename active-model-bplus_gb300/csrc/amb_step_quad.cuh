@@ -12,7 +12,7 @@
 // tile count match the SMs is therefore best where it fits (256^2: 7 or 14 rows, 3.4 us per step;
 // two or three tiles per SM 4.8 and 6.6), several CTAs of 256 threads otherwise. us per step, f32c,
 // T = 0.05, autotuned, this kernel and the one-column-per-thread tile kernel before it: 256^2 3.4 (6.3),
-// 512^2 5.9 (8.7), 768^2 9.2 (15.4), 1024^2 16.2 (24.6), 250 x 333 5.1 (6.7); from 1536^2 on the sliding
+// 512^2 5.9 (8.7), 768^2 9.2 (15.4), 1024^2 16.2 (24.6), 250 x 333 4.6 (6.7); from 1536^2 on the sliding
 // kernel, with less halo work, is the faster (28.8 there).
 //
 // The noise of a step depends on no field, so it is drawn into the arrays that J1 later replaces:
@@ -137,20 +137,26 @@ namespace amb
             }
             else
             {
-                constexpr int W = G::PW;
-                for (int t = threadIdx.x; t < rows * W; t += 8 * NT)
+                // A thread walks down a run of rows of one column, so that a site costs a load, a store and a step of
+                // the row (index arithmetic per site instead: 250 x 333 5.06 us per step, 4.57 so; 683 x 1801 29.6 and
+                // 27.2). Aligned quads shifted between lanes were slower (6.1), as were other batches than 8 rows.
+                constexpr int W = G::PW, NG = NT / W, B = 8;
+                const int run = (rows + NG - 1) / NG, j = threadIdx.x % W, g = threadIdx.x / W;
+                const int hi = g < NG ? min(rows, (g + 1) * run) : 0;
+                int gr = wrap_index(r0 + g * run - 9, ny);
+                const float* col = in + wrap_index(c0 + j - G::P0, nx);
+                for (int i = g * run; i < hi; i += B)
                 {
-                    float v[8];  // all loads of a batch before its stores
+                    float v[B];  // all loads of a batch before its stores
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
+                    for (int q = 0; q < B; ++q)
                     {
-                        const int e = t + q * NT, i = e / W, j = e - i * W;
-                        if (e < rows * W)
-                            v[q] = __ldcg(in + size_t(wrap_index(r0 + i - 9, ny)) * nx + wrap_index(c0 + j - G::P0, nx));
+                        if (i + q < hi) v[q] = __ldcg(col + size_t(gr) * nx);
+                        gr = gr + 1 == ny ? 0 : gr + 1;
                     }
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (t + q * NT < rows * W) a.phi[t + q * NT] = v[q];
+                    for (int q = 0; q < B; ++q)
+                        if (i + q < hi) a.phi[(i + q) * W + j] = v[q];
                 }
             }
         }
