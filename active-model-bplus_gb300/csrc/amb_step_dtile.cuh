@@ -9,8 +9,8 @@
 // div J side by side. An item is a column and a run of rows whose row sums are carried. The noise is
 // drawn into the arrays that J1 replaces, for the next step while the barrier completes.
 //
-// us per step at T = 0.05, this kernel and the three-phase kernel: 64^2 6.4 (12.5), 48 x 100 7.0 (12.7),
-// 128^2 9.3 (13.2), 200 x 300 18.8 (20.1).
+// us per step at T = 0.05, this kernel and the three-phase kernel: 64^2 6.1 (12.5), 48 x 100 6.7 (12.7),
+// 128^2 9.0 (13.2), 200 x 300 18.5 (20.1).
 #pragma once
 
 #include "amb_step_phase.cuh"
@@ -109,24 +109,32 @@ namespace amb
             }
         }
 
-        // One step of the CTA's tile: halo load, stages, update.
-        __device__ __forceinline__ void step(const Arrays& a, const Shape& t, const phase::Coef& k, const double* in,
-                                             double* out, int ny, int nx, int noise_mode, int r0, int c0)
+        // Where site e of the tile with its halo lies in the field.
+        __device__ __forceinline__ size_t halo_site(const Arrays& a, int e, int ny, int nx, int r0, int c0)
         {
-            const int ty = t.ty, tx = t.tx;
-            for (int e = threadIdx.x; e < (ty + 18) * a.pw; e += 4 * kThreads)
+            const int i = e / a.pw, j = e - i * a.pw;
+            return size_t(wrap_index(r0 + i - 9, ny)) * nx + wrap_index(c0 + j - 9, nx);
+        }
+
+        // One step of the CTA's tile: halo load, stages, update. first: where this thread's first four sites lie,
+        // formed once for all steps (the division and the wrap-arounds delayed the loads of each).
+        __device__ __forceinline__ void step(const Arrays& a, const Shape& t, const phase::Coef& k, const double* in,
+                                             double* out, int ny, int nx, int noise_mode, int r0, int c0,
+                                             const size_t (&first)[4])
+        {
+            const int ty = t.ty, tx = t.tx, sites = (ty + 18) * a.pw;
+            for (int e = threadIdx.x; e < sites; e += 4 * kThreads)
             {
                 double v[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                 {
-                    const int f = e + q * kThreads, i = f / a.pw, j = f - i * a.pw;
-                    if (f < (ty + 18) * a.pw)
-                        v[q] = __ldcg(in + size_t(wrap_index(r0 + i - 9, ny)) * nx + wrap_index(c0 + j - 9, nx));
+                    const int f = e + q * kThreads;
+                    if (f < sites) v[q] = __ldcg(in + (e < kThreads ? first[q] : halo_site(a, f, ny, nx, r0, c0)));
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (e + q * kThreads < (ty + 18) * a.pw) a.phi[e + q * kThreads] = v[q];
+                    if (e + q * kThreads < sites) a.phi[e + q * kThreads] = v[q];
             }
             __syncthreads();
 
@@ -272,11 +280,14 @@ namespace amb
             const size_t plane = size_t(ny) * nx;
             StepParams p = p0;
             const auto noise_of = [&](int s) { return injected ? injected + size_t(s) * 2 * plane : nullptr; };
+            size_t first[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) first[q] = halo_site(a, threadIdx.x + q * kThreads, ny, nx, r0, c0);
             draw(a, t, p, noise_mode, noise_of(0), r0, c0);
             unsigned target = 0;
             for (int s = 0; s < nsteps; ++s)
             {
-                step(a, t, k, (s & 1) ? buf1 : buf0, (s & 1) ? buf0 : buf1, ny, nx, noise_mode, r0, c0);
+                step(a, t, k, (s & 1) ? buf1 : buf0, (s & 1) ? buf0 : buf1, ny, nx, noise_mode, r0, c0, first);
                 if (s + 1 == nsteps) break;
                 target += gridDim.x;
                 if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
