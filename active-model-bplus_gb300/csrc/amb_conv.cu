@@ -38,14 +38,19 @@
 // instruction per x tap and 16 sites accumulates every (X row, dZ row) pair, of which the diagonals
 // ky = X row - dZ row are the taps: the other pairs (3 of 8) are not read. Both operands MN-major. Against
 // five y taps as separate 128 x 32 instructions, each of which reads the whole A tile (33 of its 41 cycles),
-// this takes a third of the tensor time. A persistent CTA keeps its x taps' accumulators in TMEM over all its
-// row blocks (double-buffered bulk copies), sums the diagonals once at the end and writes one partial;
+// this takes a third of the tensor time. A persistent CTA works through its row blocks (double-buffered bulk
+// copies) and keeps its x taps' accumulators in TMEM over chains of kChain blocks; after each chain the epilogue
+// warps add the diagonals to FP32 sums in their registers, while the next blocks arrive. It writes one partial;
 // a second kernel reduces the partials in a fixed order (deterministic gradients). The same CTAs sum dZ
 // over the sites while it is staged (bias gradients).
-// Measured for 16 x 128^2 sites, 32 x 32 channels: 25 us and 3.6 us for the reduction (one 128 x 32
-// instruction per tap, 256 partials: 80 and 17 us). 9 us of it are instructions, the rest the copies, which
-// the copy engine takes one by one (dZ rows that follow one another in memory go as one), and the
-// epilogue.
+// The tensor core truncates each addition to an accumulator, so a chain's error grows with its length. Largest
+// error over the largest gradient, values of mean 0.5, 32 x 32 channels, chains of 4 / 8 / 16 blocks / all blocks of
+// the CTA: 16 x 128^2 sites 0.6e-6 / 1.1e-6 / 2.0e-6 / 2.4e-6, 16 x 512^2 0.7e-6 / 1.2e-6 / 2.2e-6 / 45e-6 (partials of
+// eight rows, before the CTAs were persistent: 1.7e-6 and 3.9e-6).
+// Measured for 16 x 128^2 sites, 32 x 32 channels, with the reduction: 32.8 us (one chain 33.0; one 128 x 32
+// instruction per tap, 256 partials: 107); 16 x 512^2: 520 us (one chain 513). 9 us of the 32.8 are instructions, the
+// rest the copies, which the copy engine takes one by one (dZ rows that follow one another in memory go as
+// one), and the epilogue.
 #include "amb_gb300.h"
 #include "amb_kernels.h"
 #include "amb_tc.cuh"
@@ -123,6 +128,9 @@ namespace
         return c;
     }
 
+    // Row blocks (of eight instructions each) that an accumulator takes before it is added to the FP32 sums.
+    constexpr int kChain = 8;
+
     // wgrad geometry for Cin = 8 CC and NPAD gradient channels
     template <int CC, int NPAD>
     struct Wg
@@ -135,12 +143,15 @@ namespace
         static constexpr int GROUPS = (5 + KPC - 1) / KPC;
         static constexpr uint32_t XB = (uint32_t(XR) * CC * kRowPlane + 127u) & ~127u;
         static constexpr uint32_t STAGE = XB + uint32_t(ZR) * NQ * kTile * 16u;
-        static constexpr int NST = 2 * STAGE + 1024u <= kSmemLimit ? 2 : 1;
-        static constexpr uint32_t BARS = NST * STAGE;
-        static constexpr uint32_t SMEM = BARS + 128u + 4u * 32u * 4u;
         static constexpr int ROW = NPAD + 4;         // floats of an accumulator row in shared memory
+        static constexpr uint32_t ACC = 128u * ROW * 4u;  // one tap of all accumulator rows
+        static constexpr int NST = 2 * STAGE + ACC + 1024u <= kSmemLimit ? 2 : 1;
+        static constexpr uint32_t BARS = NST * STAGE;
+        static constexpr uint32_t ACCS = BARS + 128u + 4u * 32u * 4u;
+        static constexpr uint32_t SMEM = ACCS + ACC;
         static constexpr int PART = KPC * 5 * CIN * NPAD;  // floats of one CTA's partial
-        static_assert(KPC * 5 * CIN * ROW * 4 <= int(NST * STAGE), "accumulators fit where the stages were");
+        static constexpr int SUMS = (CIN * NPAD + 511) / 512;  // quads of a tap's gradients per epilogue thread
+        static_assert(SMEM <= kSmemLimit, "shared memory");
     };
 
     __device__ __forceinline__ void give_up(int* error, volatile int* abort, int code)
@@ -557,7 +568,8 @@ namespace
         uint64_t* full = reinterpret_cast<uint64_t*>(smem + G::BARS);
         uint64_t* empty = full + 2;
         uint64_t* done = empty + 2;
-        uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+        uint64_t* drained = done + 1;
+        uint32_t* tslot = reinterpret_cast<uint32_t*>(drained + 1);
         volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
         float* bsum = reinterpret_cast<float*>(smem + G::BARS + 128);
 
@@ -586,6 +598,9 @@ namespace
             k.right = k.c0 + kTile == a.ncols ? 2 : 0;
             return k;
         };
+        // chains of accumulators: the first and the last block of each
+        const auto starts = [&](int i) { return i % kChain == 0; };
+        const auto ends = [&](int i) { return i % kChain == kChain - 1 || i == mine - 1; };
 
         if (threadIdx.x == 0)
         {
@@ -594,7 +609,8 @@ namespace
                 mbar_init(&full[i], 1 + 4);   // the loader and the four helper warps
                 mbar_init(&empty[i], 1 + 4);  // the MMAs' completion and the helper warps
             }
-            mbar_init(done, 1);
+            mbar_init(done, 1);     // the MMAs of a chain
+            mbar_init(drained, 4);  // the epilogue warps have read its accumulators
             *abort = 0;
             fence_mbar_init();
         }
@@ -663,11 +679,13 @@ namespace
                 constexpr int N0 = G::COLS < 256 ? G::COLS : 256, N1 = G::COLS - N0;
                 const uint32_t id0 = idesc_bf16(128, N0, true, true), id1 = idesc_bf16(128, N1 > 0 ? N1 : 16, true, true);
                 const uint32_t sa = smem_u32(smem);
-                bool ok = true, issued = false;
+                bool ok = true, open = false;
+                int chains = 0;  // completed or committed ones; open: one more has instructions issued
                 for (int i = 0; ok && i < mine; ++i)
                 {
                     const int st = i % G::NST;
-                    if (!mbar_wait(&full[st], (i / G::NST) & 1, abort))
+                    if (!mbar_wait(&full[st], (i / G::NST) & 1, abort) ||
+                        (starts(i) && chains > 0 && !mbar_wait(drained, (chains - 1) & 1, abort)))
                     {
                         ok = false;
                         break;
@@ -679,21 +697,28 @@ namespace
                         for (int ks = 0; ks < kTile / 16; ++ks)
                         {
                             const uint64_t ad = smem_desc(xa + uint32_t(ks * 16 + kx0 + kxi) * 16u, 128, kRowPlane);
-                            const uint32_t d = tbase + uint32_t(kxi * G::COLS), acc = (i | ks) ? 1u : 0u;
+                            const uint32_t d = tbase + uint32_t(kxi * G::COLS), acc = starts(i) && ks == 0 ? 0u : 1u;
                             mma_bf16(d, ad, smem_desc(za + ks * 256, 128, kTile * 16), id0, acc);
                             if constexpr (N1 > 0)
                                 mma_bf16(d + N0, ad, smem_desc(za + (N0 / 8) * (kTile * 16) + ks * 256, 128, kTile * 16),
                                          id1, acc);
                         }
                     mma_commit(&empty[st]);
-                    issued = true;
+                    open = true;
+                    if (ends(i))
+                    {
+                        mma_commit(done);
+                        ++chains;
+                        open = false;
+                    }
                 }
                 if (!ok) give_up(a.error, abort, 5);
-                if (issued || ok)
+                if (open)
                 {
                     mma_commit(done);
-                    if (!mbar_wait(done, 0, nullptr)) give_up(a.error, abort, 6);
+                    ++chains;
                 }
+                if (chains > 0 && !mbar_wait(done, (chains - 1) & 1, nullptr)) give_up(a.error, abort, 6);
             }
         }
         else
@@ -751,23 +776,19 @@ namespace
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[st]);
             };
-            for (int i = 0; ok && i < mine + G::NST - 1; ++i)
-            {
-                if (i < mine) prepare(i);
-                if (ok && i >= G::NST - 1) finish(i - (G::NST - 1));
-            }
-            if (!ok && lane == 0) give_up(a.error, abort, 7);
-            ok = __all_sync(0xffffffffu, mbar_wait(done, 0, abort) && ok);
-            if (!ok && lane == 0) give_up(a.error, abort, 8);
-            tc_fence_after();
-
-            // The diagonals, summed over the X rows of the block in shared memory (where the stages were).
-            // The lane's accumulator row is X row xr, channel ci; tap ky is dZ row xr - ky + 4 of the block.
-            float* acc = reinterpret_cast<float*>(smem);
+            // A finished chain: the diagonals of its accumulators, summed over the X rows of a block through shared
+            // memory and added to the thread's share of the gradients. The lane's accumulator row is X row xr,
+            // channel ci; tap ky is dZ row xr - ky + 4 of the block. All four warps come here for every chain,
+            // whatever their waits gave, so that the block barriers match.
+            float4 sum[G::KPC][5][G::SUMS];
+#pragma unroll
+            for (int kxi = 0; kxi < G::KPC; ++kxi)
+#pragma unroll
+                for (int ky = 0; ky < 5; ++ky)
+#pragma unroll
+                    for (int f = 0; f < G::SUMS; ++f) sum[kxi][ky][f] = make_float4(0.f, 0.f, 0.f, 0.f);
+            float* acc = reinterpret_cast<float*>(smem + G::ACCS);
             const auto sync4 = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-            sync4();
-            for (int e = t; e < G::KPC * 5 * G::CIN * G::ROW; e += 128) acc[e] = 0.f;
-            sync4();
             const int q4 = warp & 3;
             const uint32_t lanes = uint32_t(q4 * 32) << 16;
             const auto load = [&](int kxi, int zr, float (&v)[32]) {  // the NPAD channels of dZ row zr
@@ -776,51 +797,74 @@ namespace
                     tmem_ld8(tbase + lanes + uint32_t(kxi * G::COLS + (q * G::ZR + zr) * 8), v + 8 * q);
                 tmem_wait_ld();
             };
-            const auto add = [&](int kxi, int ky, int ci, const float (&v)[32]) {
-                float* row = acc + ((kxi * 5 + ky) * G::CIN + ci) * G::ROW;
+            const auto drain = [&](int chain) {
+                ok = __all_sync(0xffffffffu, ok && mbar_wait(done, chain & 1, abort));
+                if (!ok && lane == 0) give_up(a.error, abort, 8);
+                tc_fence_after();
 #pragma unroll
-                for (int n = 0; n < NPAD; n += 4)
+                for (int kxi = 0; kxi < G::KPC; ++kxi)
                 {
-                    float4 w = *reinterpret_cast<float4*>(row + n);
-                    w.x += v[n]; w.y += v[n + 1]; w.z += v[n + 2]; w.w += v[n + 3];
-                    *reinterpret_cast<float4*>(row + n) = w;
-                }
-            };
-            if constexpr (CC == 4)  // one X row per warp: in each turn every warp adds to a tap of its own
-                for (int turn = 0; turn < 5; ++turn)
-                {
-                    const int ky = (q4 + turn) % 5;
-                    for (int kxi = 0; ok && mine > 0 && kxi < nkx; ++kxi)
+                    if (kxi >= nkx) continue;
+#pragma unroll
+                    for (int ky = 0; ky < 5; ++ky)
                     {
                         float v[32];
-                        load(kxi, q4 - ky + 4, v);
-                        add(kxi, ky, lane, v);
-                    }
-                    sync4();
-                }
-            else  // two X rows per warp, the warps one after the other
-                for (int turn = 0; turn < 4; ++turn)
-                {
-                    for (int kxi = 0; ok && mine > 0 && turn == q4 && kxi < nkx; ++kxi)
-                        for (int ky = 0; ky < 5; ++ky)
+                        load(kxi, q4 * (G::XR / 4) - ky + 4, v);
+                        if constexpr (CC == 2)  // two X rows per warp: the upper lanes' dZ row is the next one
                         {
-                            float v0[32], v1[32];
-                            load(kxi, 2 * q4 - ky + 4, v0);
-                            load(kxi, 2 * q4 - ky + 5, v1);
-                            if (lane < 16) add(kxi, ky, lane, v0);
-                            __syncwarp();
-                            if (lane >= 16) add(kxi, ky, lane - 16, v1);
-                            __syncwarp();
+                            float w[32];
+                            load(kxi, 2 * q4 - ky + 5, w);
+#pragma unroll
+                            for (int n = 0; n < NPAD; ++n) v[n] = lane < 16 ? v[n] : w[n];
                         }
-                    sync4();
+                        sync4();  // the tap before is read
+#pragma unroll
+                        for (int n = 0; n < NPAD; n += 4)
+                            *reinterpret_cast<float4*>(acc + (q4 * 32 + lane) * G::ROW + n) =
+                                make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
+                        sync4();
+#pragma unroll
+                        for (int f = 0; f < G::SUMS; ++f)
+                        {
+                            const int e = t + f * 128, ci = e / (NPAD / 4), n = e % (NPAD / 4) * 4;
+                            if (G::CIN * NPAD % 512 != 0 && ci >= G::CIN) continue;
+                            float4 s = *reinterpret_cast<const float4*>(acc + ci * G::ROW + n);
+#pragma unroll
+                            for (int xr = 1; xr < G::XR; ++xr)
+                            {
+                                const float4 u = *reinterpret_cast<const float4*>(acc + (xr * G::CIN + ci) * G::ROW + n);
+                                s.x += u.x; s.y += u.y; s.z += u.z; s.w += u.w;
+                            }
+                            float4& g = sum[kxi][ky][f];
+                            g.x += s.x; g.y += s.y; g.z += s.z; g.w += s.w;
+                        }
+                    }
                 }
-            float* part = a.partial + size_t(blockIdx.x) * G::PART;
-            for (int e = t; e < nkx * 5 * G::CIN * (NPAD / 4); e += 128)
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(drained);
+            };
+            int chain = 0;
+            for (int i = 0; i < mine + G::NST - 1; ++i)
             {
-                const int row = e / (NPAD / 4), n = (e - row * (NPAD / 4)) * 4;
-                *reinterpret_cast<float4*>(part + size_t(row) * NPAD + n) =
-                    *reinterpret_cast<const float4*>(acc + row * G::ROW + n);
+                const int j = i - (G::NST - 1);
+                if (i < mine && ok) prepare(i);
+                if (j >= 0 && ok) finish(j);
+                if (!ok && lane == 0) give_up(a.error, abort, 7);
+                if (j >= 0 && ends(j)) drain(chain++);
             }
+            float* part = a.partial + size_t(blockIdx.x) * G::PART;
+#pragma unroll
+            for (int kxi = 0; kxi < G::KPC; ++kxi)
+#pragma unroll
+                for (int ky = 0; ky < 5; ++ky)
+#pragma unroll
+                    for (int f = 0; f < G::SUMS; ++f)
+                    {
+                        const int e = t + f * 128;
+                        if (kxi < nkx && e < G::CIN * NPAD / 4)
+                            *reinterpret_cast<float4*>(part + size_t((kxi * 5 + ky) * G::CIN) * NPAD + e * 4) = sum[kxi][ky][f];
+                    }
             if (bias)
             {
 #pragma unroll

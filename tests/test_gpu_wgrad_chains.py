@@ -1,0 +1,29 @@
+"""Weight and bias gradients where a CTA sums many row blocks: what one accumulator of the tensor core takes
+is bounded, however large the batch."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cin,npad", [(32, 32), (16, 32), (32, 16), (16, 16)])
+def test_error_does_not_grow_with_the_batch(cin, npad):
+    """Against FP64 sums, values of one sign, some hundred row blocks per CTA: 2e-5 of the largest gradient, what
+    64 truncated FP32 additions per accumulator (64 * 2^-23) and a few hundred rounded ones between them can
+    leave (128 instead of 64, half the bound's first part again)."""
+    import torch
+    from activemodelbplus import learned as L
+    B, H, W = 16, 512, 512
+    g = torch.Generator(device="cuda").manual_seed(cin + npad)
+    x = (0.5 + torch.randn(B, cin // 8, H, W, 8, device="cuda", generator=g)).to(torch.bfloat16)
+    dz = (0.5 + torch.randn(B, npad // 8, H, W, 8, device="cuda", generator=g)).to(torch.bfloat16)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gw, gb = L.param_grads(x, dz, cin=cin, npad=npad, cin_used=cin, cout=npad, scratch=L._Scratch(), error=err)
+    assert int(err.item()) == 0
+    rows = [t.double().permute(0, 1, 4, 2, 3).reshape(B, -1, H, W) for t in (x, dz)]
+    zs = rows[1].reshape(B, npad, H * W)
+    for ky, kx in ((0, 0), (1, 2), (4, 4)):
+        xs = torch.roll(rows[0], (2 - ky, 2 - kx), (2, 3)).reshape(B, cin, H * W)
+        want = torch.einsum("bin,bon->oi", xs, zs)
+        assert (gw[:, :, ky, kx].double() - want).abs().max() <= 2e-5 * want.abs().max()
+    want = zs.sum(dim=(0, 2))
+    assert (gb.double() - want).abs().max() <= 2e-5 * want.abs().max()
