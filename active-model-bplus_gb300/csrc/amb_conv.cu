@@ -62,6 +62,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 namespace
 {
@@ -578,29 +579,32 @@ namespace
         while (int(blockIdx.x) >= a.first[group + 1]) ++group;
         const int kx0 = group * G::KPC, nkx = min(G::KPC, 5 - kx0);
         const int cta = blockIdx.x - a.first[group], nctas = a.first[group + 1] - a.first[group];
-        const int nwin = a.ncols / kTile, nblk = (a.nrows + G::XR - 1) / G::XR;
-        const int total = a.batch * nwin * nblk;
-        const int mine = cta < total ? (total - cta + nctas - 1) / nctas : 0;  // row blocks of this CTA
+        // Row blocks: those of XR rows first, then, where the rows are no multiple of it, each image's last, whose
+        // missing X rows are zeros. Those are chains of their own, of which only the rows there are count: a zero row
+        // times an infinite gradient is no zero.
+        const int nwin = a.ncols / kTile, nblk = a.nrows / G::XR, rest = a.nrows - nblk * G::XR;
+        const int whole = a.batch * nwin * nblk, total = whole + (rest ? a.batch * nwin : 0);
+        const auto dealt = [&](int n) { return cta < n ? int(unsigned(n - cta + nctas - 1) / unsigned(nctas)) : 0; };
+        const int mine = dealt(total), mine_whole = dealt(whole);  // row blocks of this CTA
 
         struct Block
         {
             int b, c0, r0, rows, left, right;  // image, first column, first X row, X rows, wrapped sites
         };
         const auto block = [&](int i) {
-            int t = cta + i * nctas;
+            const bool full = i < mine_whole;
+            const unsigned t = cta + i * nctas - (full ? 0 : whole), n = full ? nblk : 1, u = t / n, v = u / unsigned(nwin);
             Block k;
-            k.r0 = t % nblk * G::XR;
-            t /= nblk;
-            k.c0 = t % nwin * kTile;
-            k.b = t / nwin;
-            k.rows = min(G::XR, a.nrows - k.r0);
+            k.rows = full ? G::XR : rest;
+            k.r0 = int(full ? t - u * n : nblk) * G::XR;
+            k.c0 = int(u - v * nwin) * kTile;
+            k.b = int(v);
             k.left = k.c0 == 0 ? 2 : 0;
             k.right = k.c0 + kTile == a.ncols ? 2 : 0;
             return k;
         };
-        // chains of accumulators: the first and the last block of each
-        const auto starts = [&](int i) { return i % kChain == 0; };
-        const auto ends = [&](int i) { return i % kChain == kChain - 1 || i == mine - 1; };
+        // The last block of a chain, given the blocks that the chain has before it.
+        const auto ends = [&](int i, int before) { return before == kChain - 1 || i == mine_whole - 1 || i == mine - 1; };
 
         if (threadIdx.x == 0)
         {
@@ -680,36 +684,37 @@ namespace
                 const uint32_t id0 = idesc_bf16(128, N0, true, true), id1 = idesc_bf16(128, N1 > 0 ? N1 : 16, true, true);
                 const uint32_t sa = smem_u32(smem);
                 bool ok = true, open = false;
-                int chains = 0;  // completed or committed ones; open: one more has instructions issued
+                int chains = 0, before = 0;  // chains committed, blocks of the next one; open: it has instructions issued
                 for (int i = 0; ok && i < mine; ++i)
                 {
                     const int st = i % G::NST;
                     if (!mbar_wait(&full[st], (i / G::NST) & 1, abort) ||
-                        (starts(i) && chains > 0 && !mbar_wait(drained, (chains - 1) & 1, abort)))
+                        (before == 0 && chains > 0 && !mbar_wait(drained, (chains - 1) & 1, abort)))
                     {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
+                    const bool first = before == 0;
                     const uint32_t xa = sa + st * G::STAGE, za = xa + G::XB;
                     for (int kxi = 0; kxi < nkx; ++kxi)
 #pragma unroll
                         for (int ks = 0; ks < kTile / 16; ++ks)
                         {
                             const uint64_t ad = smem_desc(xa + uint32_t(ks * 16 + kx0 + kxi) * 16u, 128, kRowPlane);
-                            const uint32_t d = tbase + uint32_t(kxi * G::COLS), acc = starts(i) && ks == 0 ? 0u : 1u;
+                            const uint32_t d = tbase + uint32_t(kxi * G::COLS), acc = first && ks == 0 ? 0u : 1u;
                             mma_bf16(d, ad, smem_desc(za + ks * 256, 128, kTile * 16), id0, acc);
                             if constexpr (N1 > 0)
                                 mma_bf16(d + N0, ad, smem_desc(za + (N0 / 8) * (kTile * 16) + ks * 256, 128, kTile * 16),
                                          id1, acc);
                         }
                     mma_commit(&empty[st]);
-                    open = true;
-                    if (ends(i))
+                    open = !ends(i, before++);
+                    if (!open)
                     {
                         mma_commit(done);
                         ++chains;
-                        open = false;
+                        before = 0;
                     }
                 }
                 if (!ok) give_up(a.error, abort, 5);
@@ -797,7 +802,7 @@ namespace
                     tmem_ld8(tbase + lanes + uint32_t(kxi * G::COLS + (q * G::ZR + zr) * 8), v + 8 * q);
                 tmem_wait_ld();
             };
-            const auto drain = [&](int chain) {
+            const auto drain = [&](int chain, auto whole_blocks) {
                 ok = __all_sync(0xffffffffu, ok && mbar_wait(done, chain & 1, abort));
                 if (!ok && lane == 0) give_up(a.error, abort, 8);
                 tc_fence_after();
@@ -817,11 +822,17 @@ namespace
 #pragma unroll
                             for (int n = 0; n < NPAD; ++n) v[n] = lane < 16 ? v[n] : w[n];
                         }
+                        if constexpr (!decltype(whole_blocks)::value)
+                        {
+                            const bool counts = (q4 * 32 + lane) / G::CIN < rest;  // not a row past the image
+#pragma unroll
+                            for (int n = 0; n < NPAD; ++n) v[n] = counts ? v[n] : 0.f;
+                        }
                         sync4();  // the tap before is read
+                        float* row = acc + (q4 * 32 + lane) * G::ROW;
 #pragma unroll
                         for (int n = 0; n < NPAD; n += 4)
-                            *reinterpret_cast<float4*>(acc + (q4 * 32 + lane) * G::ROW + n) =
-                                make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
+                            *reinterpret_cast<float4*>(row + n) = make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
                         sync4();
 #pragma unroll
                         for (int f = 0; f < G::SUMS; ++f)
@@ -844,14 +855,17 @@ namespace
                 __syncwarp();
                 if (lane == 0) mbar_arrive(drained);
             };
-            int chain = 0;
+            int chain = 0, before = 0;
             for (int i = 0; i < mine + G::NST - 1; ++i)
             {
                 const int j = i - (G::NST - 1);
                 if (i < mine && ok) prepare(i);
                 if (j >= 0 && ok) finish(j);
                 if (!ok && lane == 0) give_up(a.error, abort, 7);
-                if (j >= 0 && ends(j)) drain(chain++);
+                if (j < 0 || !ends(j, before++)) continue;
+                if (j < mine_whole) drain(chain++, std::true_type{});
+                else drain(chain++, std::false_type{});
+                before = 0;
             }
             float* part = a.partial + size_t(blockIdx.x) * G::PART;
 #pragma unroll

@@ -27,3 +27,25 @@ def test_error_does_not_grow_with_the_batch(cin, npad):
         assert (gw[:, :, ky, kx].double() - want).abs().max() <= 2e-5 * want.abs().max()
     want = zs.sum(dim=(0, 2))
     assert (gb.double() - want).abs().max() <= 2e-5 * want.abs().max()
+
+
+# row counts with and without a remainder of 4 and of 8, fewer rows than a block, several blocks per CTA
+@pytest.mark.parametrize("shape", [(1, 3, 128), (1, 12, 128), (2, 13, 128), (2, 14, 256), (3, 130, 384)])
+@pytest.mark.parametrize("cin,npad", [(32, 32), (16, 32), (32, 16), (16, 16)])
+def test_an_infinite_gradient_stays_infinite(shape, cin, npad):
+    """One infinite gradient beside positive inputs: its channel's weight gradients are all +inf (each tap and
+    input channel has that one infinite term), no other channel changes."""
+    import torch
+    from activemodelbplus import learned as L
+    B, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = (0.5 + torch.rand(B, cin // 8, H, W, 8, device="cuda", generator=g)).to(torch.bfloat16)
+    dz = torch.randn(B, npad // 8, H, W, 8, device="cuda", generator=g).to(torch.bfloat16)
+    clean = L.conv_wgrad(x, dz, cin=cin, npad=npad)
+    other = [c for c in range(npad) if c != 11]
+    for b, row, col in ((0, 0, 40), (B - 1, 1, 0), (0, H // 2, W - 1), (B - 1, H - 1, 127), (0, H - 2, 5)):
+        z = dz.clone()
+        z[b, 1, row, col, 3] = float("inf")  # channel 11
+        dw = L.conv_wgrad(x, z, cin=cin, npad=npad)
+        assert bool((dw[:, :, 11] == float("inf")).all())
+        assert torch.equal(dw[:, :, other], clean[:, :, other])
