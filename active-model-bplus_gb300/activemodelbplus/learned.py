@@ -25,6 +25,7 @@ the residuals stay below tol/4.
 """
 from __future__ import annotations
 
+import copy
 import ctypes
 import math
 
@@ -664,7 +665,8 @@ class LearnedStepper:
     """Advance one field by K Euler steps per network evaluation, with plain fallback.
 
     Args:
-        net: trained :class:`FluxNet` (captured as it is when the first macro step runs).
+        net: trained :class:`FluxNet`. With ``use_graph`` its weights and biases are taken as they are when the
+            first macro step or check runs, for all later ones; without, as they are at each step.
         field: initial field (ny, nx), ncols % 128 == 0.
         stencil, model: as for :class:`Integrator` (dx = dy = 1 is what the network saw).
         K: Euler steps per macro step (the K the network was trained for).
@@ -734,6 +736,7 @@ class LearnedStepper:
         self._wres = lowpass_weights(self.shape, residual_sigma, dev) if residual_sigma > 0 else None
         self.use_graph = bool(use_graph)
         self._graph = None
+        self._frozen = None
         quiet = Model(self.model)
         quiet.T = 0.0
         self._plain = Integrator(host, self.stencil, self.model, precision=plain_precision, seed=self.seed ^ 0x5EED)
@@ -751,22 +754,37 @@ class LearnedStepper:
         """Exact sum of the fixed-point field (integer)."""
         return int(self.phi_q.to(dtype=_torch().int64).sum().item())
 
+    def _network(self) -> FluxNet:
+        """The network of the macro steps and of their checks: a captured macro step reads the operand images and
+        biases that it was captured with, so with use_graph both use a snapshot (refresh() builds images in new
+        buffers, the biases are cloned); a later change of ``net`` reaches neither."""
+        if not self.use_graph:
+            return self.net
+        if self._frozen is None:
+            self.net.refresh()
+            net = copy.copy(self.net)
+            net.biases = [b.clone() for b in net.biases]
+            net._saved, net._scratch = None, _Scratch()
+            self._frozen = net
+        return self._frozen
+
     def _apply(self, noisy: bool) -> None:
         """Network flux, plus (one spectral pass) the linear part and the filtered noise flux,
         then the exactly conservative fixed-point update. In a captured macro step the spectral pass
         is a branch beside the network's, which leaves room for it (one CTA per SM, and the SMs idle
         between layers); its buffers are the stepper's own, so nothing is allocated on the branch."""
         torch = _torch()
+        net = self._network()
         noisy = noisy and self.model.T > 0
         if torch.cuda.is_current_stream_capturing() and not (noisy and self._g is not None and not self.spectral_noise):
             here, branch = torch.cuda.current_stream(), torch.cuda.Stream()
             branch.wait_stream(here)
             with torch.cuda.stream(branch):
                 xi_direct, mag = self._spectral(noisy)
-            net_flux = self.net.forward(self._x)
+            net_flux = net.forward(self._x)
             here.wait_stream(branch)
         else:
-            net_flux = self.net.forward(self._x)
+            net_flux = net.forward(self._x)
             xi_direct, mag = self._spectral(noisy)
         _check(N.lib().amb_learned_update_input(
             _ptr(net_flux), _ptr(self._extra), *self.shape, self.dtk, self.stencil.dx, self.stencil.dy,
@@ -802,11 +820,11 @@ class LearnedStepper:
     def _macro_step(self) -> None:
         """One learned macro step (network, noise, fixed-point update, step counter).
         With use_graph the sequence is captured into a CUDA graph on first use and
-        replayed afterwards (the network's weights are fixed from then on)."""
+        replayed afterwards (the network is fixed from then on, see _network)."""
         torch = _torch()
         noisy = self.model.T > 0
         if self.use_graph and self._graph is None:
-            self.net.refresh()
+            self._network()
             saved = (self.phi_q.clone(), self.step_dev.clone(), self.flag.clone())
             side = torch.cuda.Stream()
             side.wait_stream(torch.cuda.current_stream())
@@ -822,7 +840,6 @@ class LearnedStepper:
             with torch.cuda.graph(g):  # records only; the state changes at replay
                 self._apply(noisy=noisy)
             self._graph = g
-            self._held = (self.net._images, list(self.net.biases))  # what the captured kernels read
         if self._graph is not None:
             self._graph.replay()
         else:
@@ -853,8 +870,9 @@ class LearnedStepper:
             sim._residual.zero_()
         sim._launch(self.K)
         dplain = sim.field_tensor.float() - start
-        flux = self.net.forward(network_input(start.unsqueeze(0), self.params))
-        if getattr(self.net, "linear_split", False):
+        net = self._network()
+        flux = net.forward(network_input(start.unsqueeze(0), self.params))
+        if getattr(net, "linear_split", False):
             flux = flux + self._linear.flux(start.unsqueeze(0))
         dpred = -self.dtk * divergence(flux, self.stencil.dx, self.stencil.dy)[0]
         if self._wres is not None:
