@@ -188,7 +188,7 @@ class Integrator:
             warps)}; for kernel="tile" {"pairs_per_cta": g (256-thread groups per CTA),
             "persistent": bool (all steps of a run() in one launch), "tile_rows": 32 or 28
             (output tile height), and for FP32 storage "seg_rows": 1 to 64 (output tile height, 0:
-            tile_rows) and "tile_cols": 32 or 64}; e.g. a configuration the autotuner reported.
+            tile_rows, more runs as 64) and "tile_cols": 32 or 64}; e.g. a configuration the autotuner reported.
     """
 
     def __init__(self, field, stencil, model, *, precision: str = "f64", seed: int | None = None,
@@ -240,10 +240,13 @@ class Integrator:
                 raise ValueError('launch= applies to kernel="sliding" (FP32 storage) or kernel="tile"')
             if int(launch.get("tile_rows", 32)) not in (28, 32):
                 raise ValueError("tile_rows must be 32 or 28")
+            tile_cols = int(launch.get("tile_cols", 32))
+            if tile_cols not in (32, 64) or (tile_cols == 64 and (kernel != "tile" or precision == "f64")):
+                raise ValueError('tile_cols must be 32 or, with kernel="tile" and FP32 storage, 64')
             flags = ((N.AMB_FLAG_PERSISTENT if launch.get("persistent", False) else 0)
                      | (N.AMB_FLAG_FUSED if launch.get("fused", False) else 0)
                      | (N.AMB_FLAG_TILE_ROWS_28 if int(launch.get("tile_rows", 32)) == 28 else 0)
-                     | (N.AMB_FLAG_TILE_COLS_64 if int(launch.get("tile_cols", 32)) == 64 else 0))
+                     | (N.AMB_FLAG_TILE_COLS_64 if tile_cols == 64 else 0))
             self._launch_cfg = N.amb_kernel_config(_KERNELS[kernel], int(launch.get("seg_rows", 0)),
                                                    int(launch.get("pairs_per_cta", 0)), flags)
         self._tuned = None

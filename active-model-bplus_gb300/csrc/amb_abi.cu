@@ -164,6 +164,8 @@ namespace
             return fail(AMB_ERR_INVALID, "kernel config: seg_rows >= 0, pairs_per_cta in {0, 1, 2, 4}");
         if (cfg.flags & ~(AMB_FLAG_PERSISTENT | AMB_FLAG_FUSED | AMB_FLAG_TILE_ROWS_28 | AMB_FLAG_TILE_COLS_64))
             return fail(AMB_ERR_INVALID, "kernel config: unknown flags");
+        if ((cfg.flags & AMB_FLAG_TILE_COLS_64) && (cfg.kernel != AMB_KERNEL_TILE || max_kernel == AMB_KERNEL_TILE))
+            return fail(AMB_ERR_INVALID, "kernel config: AMB_FLAG_TILE_COLS_64 is the FP32 tile kernel's");
         return AMB_OK;
     }
 }

@@ -82,7 +82,7 @@ typedef struct amb_model
 
 /* Explicit kernel configuration for amb_step_f32_ex / amb_step_f64_ex (zeros mean defaults).
  * seg_rows: rows per warp-pair task of the sliding kernel; output rows per tile of the FP32 tile
- *   kernel (1 to 64; 0: 32, or 28 with AMB_FLAG_TILE_ROWS_28).
+ *   kernel (1 to 64, more runs as 64; 0: 32, or 28 with AMB_FLAG_TILE_ROWS_28); not used by the FP64 tile kernel.
  * pairs_per_cta: sliding kernel: warp pairs per CTA (1, 2 or 4); tile kernel: groups of 256
  *   threads per CTA (1, 2 or 4; FP32: 4 runs as 2).
  * flags: AMB_FLAG_PERSISTENT (tile kernel): all nsteps of the call in one cooperative launch,
@@ -94,8 +94,8 @@ typedef struct amb_model
  *   AMB_FLAG_TILE_ROWS_28 (tile kernel): output tiles of 28 rows x 32 columns instead of 32 x 32
  *   (balances small grids over the SMs: 512 x 512 is 304 tiles, two per SM). Bitwise the same
  *   results.
- *   AMB_FLAG_TILE_COLS_64 (FP32 tile kernel): 64 output columns per tile instead of 32. Bitwise the
- *   same results. */
+ *   AMB_FLAG_TILE_COLS_64 (FP32 storage and AMB_KERNEL_TILE only, refused elsewhere): 64 output
+ *   columns per tile instead of 32. Bitwise the same results. */
 typedef struct amb_kernel_config
 {
     int kernel;
