@@ -961,13 +961,12 @@ namespace
             const float4 v = sums[i][el];
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
-        if (a.dw) *reinterpret_cast<float4*>(a.dw + (size_t(tap) * a.cin + ci) * a.npad + n * 4) = s;
+        const float v[4] = {s.x, s.y, s.z, s.w};
+        if (a.dw)  // a caller's array, aligned to its floats only
+            for (int q = 0; q < 4; ++q) a.dw[(size_t(tap) * a.cin + ci) * a.npad + n * 4 + q] = v[q];
         if (a.gw && ci < a.cin_used)
-        {
-            const float v[4] = {s.x, s.y, s.z, s.w};
             for (int q = 0; q < 4; ++q)
                 if (n * 4 + q < a.cout) a.gw[(size_t(n * 4 + q) * a.cin_used + ci) * 25 + tap] = v[q];
-        }
     }
 
     // Operand images of the layers' weights w [cout][cin][5][5], one layer per blockIdx.y: the forward
@@ -1554,8 +1553,8 @@ namespace
             (npad != 16 && npad != 32) || cin_used < 1 || cin_used > cin || cout < 1 || cout > npad)
             return fail_invalid("weight gradient: need ncols % 128 == 0, nrows >= 3, cin and npad in {16, 32}");
         const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-        if (!al16(x) || !al16(dz) || !al16(scratch) || (dw && !al16(dw)))
-            return fail_invalid("weight gradient: buffers must be 16-byte aligned");
+        if (!al16(x) || !al16(dz) || !al16(scratch))
+            return fail_invalid("weight gradient: x, dz and scratch must be 16-byte aligned");
         const WgradPlan plan = wgrad_plan(batch, nrows, ncols, cin, npad);
         if (scratch_bytes < plan.bytes(npad))
             return fail_invalid("weight gradient: scratch too small (see amb_conv5x5_wgrad_scratch_bytes)");

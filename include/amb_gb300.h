@@ -338,7 +338,7 @@ int amb_conv5x5_forward(const void* in, int batch, int nrows, int ncols, int cin
 /* Weight gradient: dw[tap][ci][co] (FP32, 25*cin*npad) = sum over batch and sites of
  * x[b][ci][(r+ky-2) mod nrows][(c+kx-2) mod ncols] * dz[b][co][r][c]. x: [batch][cin/8][...][8],
  * dz: [batch][npad/8][...][8]. Deterministic (fixed reduction order); scratch must hold
- * amb_conv5x5_wgrad_scratch_bytes(...) bytes. */
+ * amb_conv5x5_wgrad_scratch_bytes(...) bytes. x, dz and scratch: 16-byte aligned. */
 size_t amb_conv5x5_wgrad_scratch_bytes(int batch, int nrows, int ncols, int cin, int npad);
 int amb_conv5x5_wgrad(const void* x, const void* dz, int batch, int nrows, int ncols, int cin, int npad, float* dw,
                       float* scratch, size_t scratch_bytes, int* error, void* stream);

@@ -49,3 +49,22 @@ def test_an_infinite_gradient_stays_infinite(shape, cin, npad):
         dw = L.conv_wgrad(x, z, cin=cin, npad=npad)
         assert bool((dw[:, :, 11] == float("inf")).all())
         assert torch.equal(dw[:, :, other], clean[:, :, other])
+
+
+def test_gradients_at_any_float():
+    """The caller's gradient arrays need no more than a float's alignment."""
+    import torch
+    from activemodelbplus import learned as L
+    from activemodelbplus.integrator import _native as N
+    lib, stream = N.lib(), torch.cuda.current_stream().cuda_stream
+    x, dz = (torch.randn(1, 4, 8, 128, 8, device="cuda").to(torch.bfloat16) for _ in range(2))
+    nbytes = lib.amb_conv5x5_wgrad_scratch_bytes(1, 8, 128, 32, 32)
+    scratch = torch.empty(nbytes // 4, device="cuda")
+    dw, gw, gb = torch.zeros(25 * 1024 + 3, device="cuda"), torch.zeros(25 * 1024 + 1, device="cuda"), torch.zeros(33, device="cuda")
+    for at in (1, 2, 3):
+        assert lib.amb_conv5x5_wgrad(x.data_ptr(), dz.data_ptr(), 1, 8, 128, 32, 32, dw[at:].data_ptr(), scratch.data_ptr(),
+                                     nbytes, None, stream) == 0, N.last_error()
+        assert torch.equal(dw[at:at + 25 * 1024].reshape(25, 32, 32), L.conv_wgrad(x, dz, cin=32, npad=32))
+    assert lib.amb_conv5x5_param_grads(x.data_ptr(), dz.data_ptr(), 1, 8, 128, 32, 32, 32, 32, gw[1:].data_ptr(),
+                                       gb[1:].data_ptr(), scratch.data_ptr(), nbytes, None, stream) == 0, N.last_error()
+    assert torch.equal(gw[1:].reshape(32, 32, 5, 5), L.wgrad_to_weights(L.conv_wgrad(x, dz, cin=32, npad=32), 32, 32))
