@@ -23,11 +23,25 @@ namespace
     constexpr int kBinEdges = 2048;    // most edges binned in shared memory
 
     // The exact bin of k: l with edges[l-1] < k <= edges[l] (np.digitize right=True; nedges if beyond), from
-    // any starting guess.
+    // a guess a few bins away.
     __device__ __forceinline__ int exact_bin(double k, const double* __restrict__ edges, int nedges, int l)
     {
         while (l < nedges && edges[l] < k) ++l;
         while (l > 0 && !(edges[l - 1] < k)) --l;
+        return l;
+    }
+
+    // The same by halving.
+    template <typename Real>
+    __device__ __forceinline__ int find_bin(Real k, const Real* __restrict__ edges, int nedges)
+    {
+        int l = 0;
+        for (int hi = nedges; l < hi;)
+        {
+            const int mid = (l + hi) >> 1;
+            if (edges[mid] < k) l = mid + 1;
+            else hi = mid;
+        }
         return l;
     }
 
@@ -50,6 +64,8 @@ namespace
     // 1024^2: 35 us, the packed transform's unpacking included, on top of 87 us for the transform (one
     // thread and two global atomics per mode, all in FP64: 94 us, after 172 us of complex transform
     // and 28 us of elementwise passes).
+    // Past kBinEdges edges each mode's bin is found by halving in FP64: at 1024^2 a call takes 350 us with 2100
+    // edges, 359 with 4096, 615 with 100000 (walking there from the first edge: 804, 1271, 23500).
     template <Spectrum MODE>
     __global__ void __launch_bounds__(256)
     radial_bin_kernel(const double* __restrict__ in, int ny, int nx, int64_t rs, int64_t cs, double scale, double dx,
@@ -144,30 +160,21 @@ namespace
                     int l = bins[h];
                     if (act)
                     {
-                        bool exact = !shared;
-                        if (shared)
+                        const float k = sqrtf(kx2f + ky2f[warp][h][i]);
+                        if (shared && k > 1e-18f && k < 1e18f)
                         {
-                            const float k = sqrtf(kx2f + ky2f[warp][h][i]);
-                            if (l < 0)
-                            {
-                                int hi = nedges;
-                                for (l = 0; l < hi;)
-                                {
-                                    const int mid = (l + hi) >> 1;
-                                    if (ef[mid] < k) l = mid + 1;
-                                    else hi = mid;
-                                }
-                            }
+                            if (l < 0) l = find_bin(k, ef, nedges);
                             else
                             {
                                 while (l < nedges && ef[l] < k) ++l;
                                 while (l > 0 && !(ef[l - 1] < k)) --l;
                             }
                             const float tol = 1e-6f * k;
-                            exact = !(k > 1e-18f && k < 1e18f) || (l < nedges && !(fabsf(ef[l] - k) > tol)) ||
-                                    (l > 0 && !(fabsf(ef[l - 1] - k) > tol));
+                            if ((l < nedges && !(fabsf(ef[l] - k) > tol)) || (l > 0 && !(fabsf(ef[l - 1] - k) > tol)))
+                                l = exact_bin(sqrt(kx2 + ky2s[warp][h][i]), edges, nedges, l);
                         }
-                        if (exact) l = exact_bin(sqrt(kx2 + ky2s[warp][h][i]), edges, nedges, max(l, 0));
+                        else  // more edges than shared memory takes, or out of FP32's range
+                            l = find_bin(sqrt(kx2 + ky2s[warp][h][i]), edges, nedges);
                         bins[h] = l;
                     }
                     const int bin = act ? l : -1;
