@@ -19,7 +19,13 @@ namespace amb
 {
     namespace dtile
     {
-        constexpr int kThreads = 512;
+        // Threads per CTA. 512 for the lowest time of one run. A CTA of 256 leaves half an SM's registers to a CTA of
+        // another run, so that runs on several streams share the GPU, at the same time for one run where a tile has
+        // few sites. us per step of one run, and per step and run with 8 at once: 64^2 6.65 and 3.7 (512: 6.69 and
+        // 6.1), 128^2 9.8 and 6.9 (9.5 and 9.0), 200^2 16.8 and 12.9 (15.0 and 14.5). One launch per step of the tile
+        // kernel: 64^2 and 128^2 47.7 and 6.4, 200^2 47.7 and 13.7.
+        constexpr int kThreads = 512, kThreadsSmall = 256;
+        constexpr double kSitesSmall = 110;  // most sites per SM for the small CTA
 
         struct Shape
         {
@@ -55,13 +61,14 @@ namespace amb
 
         // Deals the items of one list, W columns times the runs of L rows in H, to the CTA's warps; lists
         // given to the same Deal follow one another. f(column, first row, last row + 1).
+        template <int NT>
         struct Deal
         {
             int next = 0;
             template <typename F>
             __device__ __forceinline__ void operator()(int W, int H, int L, F&& f)
             {
-                const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kThreads / 32;
+                const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = NT / 32;
                 const int n = W * ((H + L - 1) / L), chunks = (n + 31) >> 5;
                 for (int c = (warp - next) & (warps - 1); c < chunks; c += warps)
                 {
@@ -78,12 +85,13 @@ namespace amb
 
         // xi of the tile's J1_y and J1_x into their arrays, one Philox call per quad of columns where the
         // quad is one of the noise's.
+        template <int NT>
         __device__ __forceinline__ void draw(const Arrays& a, const Shape& t, const StepParams& p, int noise_mode,
                                              const double* injected, int r0, int c0)
         {
             if (noise_mode == NOISE_OFF) return;
             const int ny = p.ny, nx = p.nx, qy = t.tx / 4, qx = qy + 2, n1 = qy * (t.ty + 8), n = n1 + qx * t.ty;
-            for (int e = threadIdx.x; e < n; e += kThreads)
+            for (int e = threadIdx.x; e < n; e += NT)
             {
                 const int comp = e >= n1, k = comp ? e - n1 : e, w = comp ? qx : qy;
                 const int i = k / w, j = k - i * w;
@@ -118,28 +126,29 @@ namespace amb
 
         // One step of the CTA's tile: halo load, stages, update. first: where this thread's first four sites lie,
         // formed once for all steps (the division and the wrap-arounds delayed the loads of each).
+        template <int NT>
         __device__ __forceinline__ void step(const Arrays& a, const Shape& t, const phase::Coef& k, const double* in,
                                              double* out, int ny, int nx, int noise_mode, int r0, int c0,
                                              const size_t (&first)[4])
         {
             const int ty = t.ty, tx = t.tx, sites = (ty + 18) * a.pw;
-            for (int e = threadIdx.x; e < sites; e += 4 * kThreads)
+            for (int e = threadIdx.x; e < sites; e += 4 * NT)
             {
                 double v[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                 {
-                    const int f = e + q * kThreads;
-                    if (f < sites) v[q] = __ldcg(in + (e < kThreads ? first[q] : halo_site(a, f, ny, nx, r0, c0)));
+                    const int f = e + q * NT;
+                    if (f < sites) v[q] = __ldcg(in + (e < NT ? first[q] : halo_site(a, f, ny, nx, r0, c0)));
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (e + q * kThreads < sites) a.phi[e + q * kThreads] = v[q];
+                    if (e + q * NT < sites) a.phi[e + q * NT] = v[q];
             }
             __syncthreads();
 
             // about one item per thread: runs as long as that allows
-            const auto run = [](int sites) { return max(1, sites / kThreads); };
+            const auto run = [](int sites) { return max(1, sites / NT); };
 
             // ---- stage A. walk(column, rows, f): f(row, site) down a run, tile coordinates
             const auto walk = [&](int j, int lo, int hi, auto&& f) {
@@ -161,7 +170,7 @@ namespace amb
                 walk(j, lo, hi, [&](int i, const SiteA<double>& s) { a.mup[(i + 8) * a.mw + j + 8] = s.mup; });
             };
             {
-                Deal deal;
+                Deal<NT> deal;
                 deal(tx + 4, ty + 4, run((tx + 4) * (ty + 4)), [&](int jj, int g0, int g1) {
                     const int j = jj - 2;
                     walk(j, g0 - 2, g1 - 2, [&](int i, const SiteA<double>& s) {
@@ -186,7 +195,7 @@ namespace amb
 
             // ---- stage B: J1_y, J1_x (over their noise), J2 (over J_c)
             {
-                Deal deal;
+                Deal<NT> deal;
                 const bool noisy = noise_mode != NOISE_OFF;
                 deal(tx + 2, ty + 2, run((tx + 2) * (ty + 2)), [&](int j, int g0, int g1) {
                     const double* s = a.mua + g0 * a.aw + j + 1;  // row g0 - 2 of the tile
@@ -222,7 +231,7 @@ namespace amb
 
             // ---- stage C: the three terms of div J (divTj over mu_a, DY8 over mu_p), then the update
             {
-                Deal deal;
+                Deal<NT> deal;
                 deal(tx, ty, run(tx * ty), [&](int j, int g0, int g1) {
                     const double *y = a.j2y + g0 * a.cw + j + 1, *x = a.j2x + g0 * a.cw + j + 1;
                     const auto smooth = [&] { return canon_smooth(y[-1], y[0], y[1], k); };
@@ -252,7 +261,7 @@ namespace amb
                 });
             }
             __syncthreads();
-            for (int e = threadIdx.x; e < tx * ty; e += kThreads)
+            for (int e = threadIdx.x; e < tx * ty; e += NT)
             {
                 const int i = e / tx, j = e - i * tx, gr = r0 + i, gc = c0 + j;
                 if (gr < ny && gc < nx)
@@ -263,14 +272,15 @@ namespace amb
 
         // nsteps steps; each CTA owns one tile; step s reads buf[s % 2] and writes buf[(s + 1) % 2]. If the grid
         // barrier gives up, the CTA fills its share of both buffers with NaN (caught by the finite check).
-        __global__ void __launch_bounds__(kThreads, 1)
+        template <int NT>
+        __global__ void __launch_bounds__(NT, kThreads / NT)
         step_dtile_kernel(double* buf0, double* buf1, unsigned* count, const StepParams p0, const phase::Coef coef,
                           const Shape t, int noise_mode, const double* injected, int nsteps)
         {
             extern __shared__ __align__(16) double smem_d[];
             __shared__ int ok;
             __shared__ __align__(16) unsigned char coef_smem[sizeof(phase::Coef)];
-            for (int i = threadIdx.x; i < int(sizeof(phase::Coef) / 4); i += kThreads)
+            for (int i = threadIdx.x; i < int(sizeof(phase::Coef) / 4); i += NT)
                 reinterpret_cast<uint32_t*>(coef_smem)[i] = reinterpret_cast<const uint32_t*>(&coef)[i];
             __syncthreads();
             const phase::Coef& k = *reinterpret_cast<const phase::Coef*>(coef_smem);
@@ -282,17 +292,17 @@ namespace amb
             const auto noise_of = [&](int s) { return injected ? injected + size_t(s) * 2 * plane : nullptr; };
             size_t first[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) first[q] = halo_site(a, threadIdx.x + q * kThreads, ny, nx, r0, c0);
-            draw(a, t, p, noise_mode, noise_of(0), r0, c0);
+            for (int q = 0; q < 4; ++q) first[q] = halo_site(a, threadIdx.x + q * NT, ny, nx, r0, c0);
+            draw<NT>(a, t, p, noise_mode, noise_of(0), r0, c0);
             unsigned target = 0;
             for (int s = 0; s < nsteps; ++s)
             {
-                step(a, t, k, (s & 1) ? buf1 : buf0, (s & 1) ? buf0 : buf1, ny, nx, noise_mode, r0, c0, first);
+                step<NT>(a, t, k, (s & 1) ? buf1 : buf0, (s & 1) ? buf0 : buf1, ny, nx, noise_mode, r0, c0, first);
                 if (s + 1 == nsteps) break;
                 target += gridDim.x;
                 if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
                 p.step = p0.step + s + 1;
-                draw(a, t, p, noise_mode, noise_of(s + 1), r0, c0);
+                draw<NT>(a, t, p, noise_mode, noise_of(s + 1), r0, c0);
                 if (threadIdx.x == 0)
                 {
                     int done = 0;
@@ -308,7 +318,7 @@ namespace amb
                 if (!ok)
                 {
                     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-                    for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < plane; i += size_t(gridDim.x) * kThreads)
+                    for (size_t i = blockIdx.x * size_t(NT) + threadIdx.x; i < plane; i += size_t(gridDim.x) * NT)
                         buf0[i] = buf1[i] = nan;
                     return;
                 }

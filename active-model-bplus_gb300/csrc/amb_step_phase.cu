@@ -46,10 +46,10 @@ namespace amb
     {
         // FP64 warp instructions of one step of a tile, as its lists are packed (runs of about one item per
         // thread), plus what the barriers and the halo load cost beside them.
-        double tile_cost(int ty, int tx)
+        double tile_cost(int ty, int tx, int threads)
         {
-            const auto list = [](int w, int h, double per_site, double per_run) {
-                const int l = std::max(1, w * h / dtile::kThreads), items = w * ((h + l - 1) / l);
+            const auto list = [=](int w, int h, double per_site, double per_run) {
+                const int l = std::max(1, w * h / threads), items = w * ((h + l - 1) / l);
                 return double((items + 31) / 32) * (l * per_site + per_run);
             };
             return list(tx + 4, ty + 4, 25, 4) + list(2 * tx, 6, 11, 2) + list(12, ty, 11, 2) + list(tx + 2, ty + 2, 9, 8)
@@ -61,9 +61,10 @@ namespace amb
         // 1 x 64 12.3). False above 400 sites per SM, where the halo costs more than two grid barriers (us per
         // step, tiles and phases: 128^2 9.0 and 13.2, 200 x 300 18.5 and 20.1, 256^2 19.9 and 20.0, 350^2 35.8
         // and 29.5).
-        bool tile_shape(int ny, int nx, int sms, dtile::Shape* best)
+        bool tile_shape(int ny, int nx, int sms, dtile::Shape* best, int* threads)
         {
             double least = 1e300;
+            *threads = double(ny) * nx > dtile::kSitesSmall * sms ? dtile::kThreads : dtile::kThreadsSmall;
             if (double(ny) * nx > 400.0 * sms) return false;
             for (int tx : {8, 12, 16, 24, 32, 48})
             {
@@ -71,7 +72,7 @@ namespace amb
                 if (down < 1) continue;
                 const dtile::Shape t{std::max(1, (ny + down - 1) / down), tx};
                 if (t.doubles() * sizeof(double) > kTileSmem) continue;
-                const double cost = tile_cost(t.ty, t.tx);
+                const double cost = tile_cost(t.ty, t.tx, *threads);
                 if (cost < least)
                 {
                     least = cost;
@@ -109,17 +110,22 @@ namespace amb
             }
         }
         dtile::Shape tile{};
-        const bool small = tile_shape(p.ny, p.nx, sms, &tile);
+        int threads = 0;
+        const bool small = tile_shape(p.ny, p.nx, sms, &tile, &threads);
+        const void* dtile_kernel = threads == dtile::kThreads
+                                       ? reinterpret_cast<const void*>(dtile::step_dtile_kernel<dtile::kThreads>)
+                                       : reinterpret_cast<const void*>(dtile::step_dtile_kernel<dtile::kThreadsSmall>);
         if (small)
         {
             static std::mutex attr_mutex;
-            static bool configured[64];
+            static bool configured[2][64];
+            bool* done = configured[threads == dtile::kThreads];
             std::lock_guard<std::mutex> lock(attr_mutex);
-            if (dev >= 64 || !configured[dev])
+            if (dev >= 64 || !done[dev])
             {
-                e = cudaFuncSetAttribute(dtile::step_dtile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileSmem));
+                e = cudaFuncSetAttribute(dtile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileSmem));
                 if (e != cudaSuccess) return e;
-                if (dev < 64) configured[dev] = true;
+                if (dev < 64) done[dev] = true;
             }
         }
         int band = 0;
@@ -141,8 +147,7 @@ namespace amb
                 const int tiles = ((p.ny + tile.ty - 1) / tile.ty) * ((p.nx + tile.tx - 1) / tile.tx);
                 unsigned* count = static_cast<unsigned*>(workspace);
                 void* args[] = {&in, &out, &count, &pp, const_cast<phase::Coef*>(&k), &tile, &noise_mode, &inj, &m};
-                e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(dtile::step_dtile_kernel), dim3(tiles),
-                                                dim3(dtile::kThreads), args, tile.doubles() * sizeof(double), stream);
+                e = cudaLaunchCooperativeKernel(dtile_kernel, dim3(tiles), dim3(threads), args, tile.doubles() * sizeof(double), stream);
                 if (e != cudaSuccess) return e;
                 done += n;
                 continue;
