@@ -14,9 +14,16 @@ namespace amb
         // Largest planes workspace. A band of at most this many bytes keeps the recomputed rows of a
         // band boundary (16 of phase 1, 8 of phase 2) below 1 % of the band at 4096 columns.
         constexpr size_t kWorkspaceCap = size_t(256) << 20;
-        // Sites x steps of one launch, about half a second of FP64 work, so that a long run stays a
-        // queue of launches.
-        constexpr double kLaunchWork = 4e9;
+        // Longest launch in seconds, and the steps that fit: a long run stays a queue of launches, between which
+        // another stream's kernels find the SMs free (300000 steps of 64^2 in 180 launches: 6.0 us per step, as in
+        // one). A step takes 6 us (tiles) or 12 us (phases) however small the grid, and 145 ps per site where the FP64
+        // pipe binds.
+        constexpr double kLaunchSeconds = 0.01;
+        int steps_per_launch(int ny, int nx, bool tiles)
+        {
+            const double step = std::max(tiles ? 6e-6 : 12e-6, double(ny) * nx * 145e-12);
+            return int(std::max(1.0, kLaunchSeconds / step));
+        }
         constexpr size_t kTileSmem = size_t(200) << 10;
 
         template <typename Real>
@@ -131,7 +138,7 @@ namespace amb
         int band = 0;
         workspace_bytes<double>(p.ny, p.nx, &band);
         const phase::Coef k(p);
-        const int chunk = int(std::max(1.0, std::min(double(nsteps), kLaunchWork / (double(p.ny) * p.nx))));
+        const int chunk = steps_per_launch(p.ny, p.nx, small);
         for (int done = 0; done < nsteps;)
         {
             const int n = std::min(chunk, nsteps - done);
