@@ -163,6 +163,10 @@ def _random_seed() -> int:
     return int.from_bytes(os.urandom(8), "little")
 
 
+# Largest workspace that an FP64 integrator keeps between runs (362^2): a lease costs some 5 us per run.
+_KEPT_WORKSPACE = 8 << 20
+
+
 class Integrator:
     """Explicit-Euler Active Model B+ integrator on one GPU
     (the reference's ``Integrator``, src/integrator.h:24-81, src/integrator.cc:105-123).
@@ -220,13 +224,13 @@ class Integrator:
         self._residual = (torch.zeros((self._ny, self._nx), dtype=torch.int16, device=self._device)
                           if precision == "f32c" else None)
         self._flag = torch.zeros(1, dtype=torch.int32, device=self._device)
-        self._workspace = None  # planes of the three-phase FP64 kernel; FP32: the grid barrier's counter
+        # FP32: the grid barrier's counter. FP64: the planes of the three-phase kernel, four times the field and up to
+        # 256 MiB: kept where small, else the bytes that each run takes and gives back; None: no room, tile kernel.
+        self._workspace = None
         if precision != "f64" or kernel != "tile":
-            try:
-                self._workspace = torch.empty(lib.amb_step_workspace_bytes(_PRECISIONS[precision], self._ny, self._nx),
-                                              dtype=torch.uint8, device=self._device)
-            except torch.cuda.OutOfMemoryError:
-                pass  # the tile kernel needs none
+            self._workspace = lib.amb_step_workspace_bytes(_PRECISIONS[precision], self._ny, self._nx)
+            if self._workspace <= _KEPT_WORKSPACE:
+                self._workspace = self._lease()
         self._timestep = 0
         self._terms_step = None
         self._terms_dev = None
@@ -329,13 +333,13 @@ class Integrator:
         if nsteps > 0:
             in_spare = ctypes.c_int(0)
             cur, other = self._buf[self._cur], self._buf[1 - self._cur]
+            ws = self._lease()
             if self._events is not None:
                 self._events[0].record()
-            if self._precision == "f64" and self._workspace is not None:
+            if self._precision == "f64" and ws is not None:
                 rc = lib.amb_step_f64_ws(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
                                          cur.data_ptr(), other.data_ptr(), self._timestep, nsteps, None,
-                                         self._workspace.data_ptr(), self._workspace.numel(), stream,
-                                         ctypes.byref(in_spare))
+                                         ws.data_ptr(), ws.numel(), stream, ctypes.byref(in_spare))
             elif self._precision == "f64":
                 rc = lib.amb_step_f64_ex(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny,
                                          self._nx, cur.data_ptr(), other.data_ptr(), self._timestep, nsteps, None,
@@ -348,9 +352,8 @@ class Integrator:
                     cfg = N.amb_kernel_config(_KERNELS[self._kernel], 0, 0, 0)
                 args = (ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx, cur.data_ptr(),
                         other.data_ptr(), res, self._timestep, nsteps, None, ctypes.byref(cfg))
-                if self._workspace is not None:
-                    rc = lib.amb_step_f32_ws(*args, self._workspace.data_ptr(), self._workspace.numel(), stream,
-                                             ctypes.byref(in_spare))
+                if ws is not None:
+                    rc = lib.amb_step_f32_ws(*args, ws.data_ptr(), ws.numel(), stream, ctypes.byref(in_spare))
                 else:
                     rc = lib.amb_step_f32_ex(*args, stream, ctypes.byref(in_spare))
             if self._events is not None:
@@ -359,6 +362,21 @@ class Integrator:
             if in_spare.value:
                 self._cur = 1 - self._cur
         self._timestep += nsteps
+
+    def _lease(self):
+        """The workspace of a run, or None: kernel="tile", a large one under capture (which runs single steps of the
+        tile kernel), no room (then no longer asked for). A large one comes from torch's allocator on the stream that
+        the run is queued on and goes back to it, so integrators that take turns share it."""
+        torch = _torch()
+        if not isinstance(self._workspace, int):
+            return self._workspace
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        try:
+            return torch.empty(self._workspace, dtype=torch.uint8, device=self._device)
+        except torch.cuda.OutOfMemoryError:
+            self._workspace = None
+            return None
 
     def _enqueue_finite_check(self) -> None:
         """OR a non-finite flag for the current field into ``self._flag`` (stream-ordered)."""
