@@ -167,6 +167,11 @@ def _random_seed() -> int:
 _KEPT_WORKSPACE = 8 << 20
 
 
+# Term planes (of the y component) that a current is the sum of, in the reference's order.
+_CURRENT_TERMS = {"passive": (2,), "lambda": (4,), "circulating": (6,), "random": (8,), "active": (6, 4),
+                  "deterministic": (6, 4, 2), "total": (6, 4, 2, 8)}
+
+
 class Integrator:
     """Explicit-Euler Active Model B+ integrator on one GPU
     (the reference's ``Integrator``, src/integrator.h:24-81, src/integrator.cc:105-123).
@@ -417,10 +422,21 @@ class Integrator:
         """Fresh host copies of both components, summed on the device in the reference's order
         (src/integrator.cu:406-465)."""
         terms = self._terms()
-        out = _torch().empty((2, self._ny, self._nx), dtype=terms.dtype, device=terms.device)
+        try:
+            out = _torch().empty((2, self._ny, self._nx), dtype=terms.dtype, device=terms.device)
+        except _torch().cuda.OutOfMemoryError:
+            return [self._sum_on_host([terms[k + c] for k in _CURRENT_TERMS[which]]) for c in range(2)]
         _check(N.lib().amb_current_from_terms(terms.data_ptr(), self._ny, self._nx, N.CURRENTS[which], out.data_ptr(),
                                               self._stream()))
         return [v.cpu().numpy() for v in out]
+
+    @staticmethod
+    def _sum_on_host(planes) -> np.ndarray:
+        """The sum of device planes in their order, where the device has no room for another plane."""
+        out = planes[0].cpu().numpy()
+        for p in planes[1:]:
+            out += p.cpu().numpy()
+        return out
 
     @property
     def current(self):
@@ -455,7 +471,10 @@ class Integrator:
     def chemical_potential(self) -> np.ndarray:
         """mu_p + mu_a (src/integrator.cu:385-388; not bound in the reference's module)."""
         t = self._terms()
-        return (t[0] + t[1]).cpu().numpy()
+        try:
+            return (t[0] + t[1]).cpu().numpy()
+        except _torch().cuda.OutOfMemoryError:
+            return self._sum_on_host([t[0], t[1]])
 
     @property
     def passive_chemical_potential(self) -> np.ndarray:

@@ -48,3 +48,20 @@ def test_a_run_without_room_takes_the_tile_kernel(room):
     sim.run(1)
     tile.run(3)
     assert torch.equal(sim.field_tensor, tile.field_tensor)
+
+
+def test_getters_need_ten_planes(room):
+    """Room for the term planes and no more: every current and potential, the same bits as with room."""
+    from activemodelbplus.integrator import _native as N
+    free, tight = _sim(), _sim()
+    names = ["current", "deterministic_current", "passive_current", "active_current", "lambda_current",
+             "circulating_current", "random_current", "chemical_potential", "passive_chemical_potential",
+             "active_chemical_potential"]
+    names = [n for n in names if hasattr(type(free), n)]
+    assert len(names) >= len(N.CURRENTS)
+    want = {n: getattr(free, n) for n in names}
+    del free
+    room(10.5)
+    for n in names:
+        got = getattr(tight, n)
+        assert np.array_equal(np.asarray(got), np.asarray(want[n])), n
