@@ -342,7 +342,8 @@ extern "C" int amb_current_from_terms(const double* terms, int nrows, int ncols,
     if (int rc = check_shape(nrows, ncols)) return rc;
     if (!terms || !out) return fail(AMB_ERR_INVALID, "terms and out must not be NULL");
     if (which < AMB_CURRENT_TOTAL || which > AMB_CURRENT_RANDOM) return fail(AMB_ERR_INVALID, "unknown current");
-    cudaError_t e = amb::launch_current(terms, size_t(nrows) * ncols, which, out, as_stream(stream));
+    const size_t n = size_t(nrows) * ncols;
+    cudaError_t e = amb::launch_current(terms, n, 0, 2 * n, which, out, as_stream(stream));
     return e == cudaSuccess ? AMB_OK : cuda_fail(e, "amb_current_from_terms");
 }
 
@@ -417,7 +418,7 @@ struct amb_integrator
     void* workspace = nullptr;  // step workspace, allocated at the first run if there is room
     bool workspace_tried = false;
     double* stage = nullptr;  // float64 staging plane for FP32 fields, allocated on first transfer
-    double* terms = nullptr;  // AMB_NTERMS planes and two of a current, allocated on first getter call
+    double* terms = nullptr;  // AMB_NTERMS planes, allocated on first getter call
     int* flag = nullptr;
 
     size_t n() const { return size_t(nrows) * ncols; }
@@ -472,7 +473,7 @@ namespace
         if (h->terms_timestep == h->timestep) return AMB_OK;
         if (!h->terms)
         {
-            cudaError_t e = cudaMalloc(&h->terms, h->n() * (AMB_NTERMS + 2) * sizeof(double));
+            cudaError_t e = cudaMalloc(&h->terms, h->n() * AMB_NTERMS * sizeof(double));
             if (e != cudaSuccess) return fail(AMB_ERR_NOMEM, "terms buffer: " + std::string(cudaGetErrorString(e)));
         }
         int rc = h->precision == AMB_F64
@@ -491,10 +492,18 @@ namespace
         return e == cudaSuccess ? AMB_OK : cuda_fail(e, "terms readback");
     }
 
-    int wait_read(amb_integrator* h)
+    // Waits for the copies queued by read_plane, whatever came after them.
+    int wait_read(amb_integrator* h, int rc)
     {
         cudaError_t e = cudaStreamSynchronize(h->stream);
-        return e == cudaSuccess ? AMB_OK : cuda_fail(e, "terms readback");
+        return rc ? rc : e == cudaSuccess ? AMB_OK : cuda_fail(e, "terms readback");
+    }
+
+    // A plane of doubles that holds nothing between calls: the field's other buffer, or, for FP32 fields, the
+    // staging plane that the field came through.
+    double* free_plane(amb_integrator* h)
+    {
+        return h->precision == AMB_F64 ? static_cast<double*>(h->buf[1 - h->cur]) : h->stage;
     }
 }
 
@@ -623,17 +632,14 @@ extern "C" int amb_integrator_get_chemical_potential(amb_integrator* h, int whic
     if (which < AMB_MU_TOTAL || which > AMB_MU_ACTIVE) return fail(AMB_ERR_INVALID, "unknown chemical potential");
     if (int rc = compute_terms(h)) return rc;
     const size_t n = h->n();
-    int rc = read_plane(h, h->terms + (which == AMB_MU_ACTIVE ? n : 0), host_out);
-    std::vector<double> active;
-    if (!rc && which == AMB_MU_TOTAL)
+    const double* from = h->terms + (which == AMB_MU_ACTIVE ? n : 0);
+    if (which == AMB_MU_TOTAL)
     {
-        active.resize(n);
-        rc = read_plane(h, h->terms + n, active.data());
+        cudaError_t e = amb::launch_sum(h->terms, h->terms + n, n, free_plane(h), h->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "chemical potential");
+        from = free_plane(h);
     }
-    if (!rc) rc = wait_read(h);
-    if (!rc)
-        for (size_t i = 0; i < active.size(); ++i) host_out[i] += active[i];
-    return rc;
+    return wait_read(h, read_plane(h, from, host_out));
 }
 
 extern "C" int amb_integrator_get_current(amb_integrator* h, int which, double* host_y, double* host_x)
@@ -642,11 +648,14 @@ extern "C" int amb_integrator_get_current(amb_integrator* h, int which, double* 
     if (which < AMB_CURRENT_TOTAL || which > AMB_CURRENT_RANDOM) return fail(AMB_ERR_INVALID, "unknown current");
     if (int rc = compute_terms(h)) return rc;
     const size_t n = h->n();
-    double* planes = h->terms + AMB_NTERMS * n;
-    int rc = amb_current_from_terms(h->terms, h->nrows, h->ncols, which, planes, h->stream);
-    if (!rc) rc = read_plane(h, planes, host_y);
-    if (!rc) rc = read_plane(h, planes + n, host_x);
-    return rc ? rc : wait_read(h);
+    double* host[2] = {host_y, host_x};
+    int rc = AMB_OK;
+    for (int c = 0; c < 2 && !rc; ++c)  // one component after the other through one plane
+    {
+        cudaError_t e = amb::launch_current(h->terms, n, c * n, n, which, free_plane(h), h->stream);
+        rc = e == cudaSuccess ? read_plane(h, free_plane(h), host[c]) : cuda_fail(e, "current");
+    }
+    return wait_read(h, rc);
 }
 
 extern "C" int amb_integrator_get_timestep(const amb_integrator* h, int64_t* out)

@@ -73,7 +73,10 @@ namespace amb
     cudaError_t launch_terms(const Real* phi, double* out, const StepParams& p, int noise_mode, const Real* injected,
                              cudaStream_t stream);
 
-    cudaError_t launch_current(const double* terms, size_t n, int which, double* out, cudaStream_t stream);
+    // Values [first, first + count) of a current (n of the y component, then n of the x component) from the term planes.
+    cudaError_t launch_current(const double* terms, size_t n, size_t first, size_t count, int which, double* out,
+                               cudaStream_t stream);
+    cudaError_t launch_sum(const double* a, const double* b, size_t n, double* out, cudaStream_t stream);
 
     int mass_partials(size_t n);
     template <typename Real>

@@ -111,11 +111,21 @@ namespace amb
         }
     }
 
-    // Both components of a current from the ten planes: the host reads two planes instead of ten.
-    __global__ void current_kernel(const double* __restrict__ terms, size_t n, int which, double* __restrict__ out)
+    // A current from the ten planes: the host reads two planes instead of ten.
+    __global__ void current_kernel(const double* __restrict__ terms, size_t n, size_t first, size_t count, int which,
+                                   double* __restrict__ out)
     {
-        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < 2 * n; i += (size_t)gridDim.x * blockDim.x)
-            out[i] = current_of(which, terms[2 * n + i], terms[4 * n + i], terms[6 * n + i], terms[8 * n + i]);
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
+        {
+            const double* t = terms + first + i;
+            out[i] = current_of(which, t[2 * n], t[4 * n], t[6 * n], t[8 * n]);
+        }
+    }
+
+    __global__ void sum_kernel(const double* __restrict__ a, const double* __restrict__ b, size_t n, double* __restrict__ out)
+    {
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+            out[i] = __dadd_rn(a[i], b[i]);
     }
 
     static int grid_for(size_t n, int block)
@@ -135,9 +145,16 @@ namespace amb
         return cudaGetLastError();
     }
 
-    cudaError_t launch_current(const double* terms, size_t n, int which, double* out, cudaStream_t stream)
+    cudaError_t launch_current(const double* terms, size_t n, size_t first, size_t count, int which, double* out,
+                               cudaStream_t stream)
     {
-        current_kernel<<<grid_for(2 * n, 256), 256, 0, stream>>>(terms, n, which, out);
+        current_kernel<<<grid_for(count, 256), 256, 0, stream>>>(terms, n, first, count, which, out);
+        return cudaGetLastError();
+    }
+
+    cudaError_t launch_sum(const double* a, const double* b, size_t n, double* out, cudaStream_t stream)
+    {
+        sum_kernel<<<grid_for(n, 256), 256, 0, stream>>>(a, b, n, out);
         return cudaGetLastError();
     }
 

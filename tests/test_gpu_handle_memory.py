@@ -1,0 +1,77 @@
+"""The C handle's getters: their sums, and what they hold on the device."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from activemodelbplus.integrator import _native as N
+
+pytestmark = pytest.mark.gpu
+STENCIL = N.amb_stencil(1e-3, 1, 1)
+MODEL = N.amb_model(-0.25, 0, 0.25, 1, -1, -4, 0.05)
+
+
+def _handle(field, precision, seed=7):
+    h = ctypes.c_void_p()
+    field = np.ascontiguousarray(field, dtype=np.float64)
+    rc = N.lib().amb_integrator_create(field.ctypes.data, *field.shape, ctypes.byref(STENCIL), ctypes.byref(MODEL), precision,
+                                       seed, ctypes.byref(h))
+    assert rc == 0, N.last_error()
+    return h
+
+
+def _used():
+    import torch
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def _current(h, which, shape):
+    out = np.empty((2,) + shape)
+    assert N.lib().amb_integrator_get_current(h, which, out[0].ctypes.data, out[1].ctypes.data) == 0, N.last_error()
+    return out
+
+
+def _potential(h, which, shape):
+    out = np.empty(shape)
+    assert N.lib().amb_integrator_get_chemical_potential(h, which, out.ctypes.data) == 0, N.last_error()
+    return out
+
+
+@pytest.mark.parametrize("precision", [N.AMB_F64, N.AMB_F32, N.AMB_F32C])
+@pytest.mark.parametrize("shape", [(1, 1), (33, 70)])
+def test_getters_leave_the_run_as_it_was(shape, precision):
+    """Every current and potential is the sum of its terms to the bit, and a run goes on as without them."""
+    lib, field = N.lib(), np.random.default_rng(1).normal(-0.4, 0.1, shape)
+    a, b = _handle(field, precision), _handle(field, precision)
+    for h in (a, b):
+        assert lib.amb_integrator_run(h, 3) == 0
+    t = {k: _current(a, w, shape) for k, w in N.CURRENTS.items()}
+    assert np.array_equal(t["active"], t["circulating"] + t["lambda"])
+    assert np.array_equal(t["deterministic"], t["active"] + t["passive"])
+    assert np.array_equal(t["total"], t["deterministic"] + t["random"])
+    assert np.array_equal(_potential(a, 0, shape), _potential(a, 1, shape) + _potential(a, 2, shape))
+    fields = []
+    for h in (a, b):
+        assert lib.amb_integrator_run(h, 4) == 0
+        out = np.empty(shape)
+        assert lib.amb_integrator_get_field(h, out.ctypes.data) == 0
+        fields.append(out)
+        lib.amb_integrator_destroy(h)
+    assert np.array_equal(*fields)
+
+
+@pytest.mark.parametrize("precision", [N.AMB_F64, N.AMB_F32C])
+def test_getters_allocate_the_term_planes_only(precision):
+    import torch
+    side, shape = 2048, (2048, 2048)
+    plane = side * side * 8
+    torch.cuda.empty_cache()
+    h = _handle(np.random.default_rng(2).normal(-0.4, 0.1, shape), precision)
+    assert N.lib().amb_integrator_run(h, 1) == 0
+    _current_before = _used()
+    _current(h, N.CURRENTS["total"], shape)
+    _potential(h, 0, shape)
+    assert _used() - _current_before < 10.5 * plane
+    N.lib().amb_integrator_destroy(h)
