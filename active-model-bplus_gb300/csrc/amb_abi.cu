@@ -420,6 +420,7 @@ struct amb_integrator
     double* stage = nullptr;  // float64 staging plane for FP32 fields, allocated on first transfer
     double* terms = nullptr;  // AMB_NTERMS planes, allocated on first getter call
     int* flag = nullptr;
+    std::mutex reading;  // getters share a plane for sums
 
     size_t n() const { return size_t(nrows) * ncols; }
     size_t elem() const { return precision == AMB_F64 ? sizeof(double) : sizeof(float); }
@@ -630,6 +631,7 @@ extern "C" int amb_integrator_get_chemical_potential(amb_integrator* h, int whic
 {
     if (!h || !host_out) return fail(AMB_ERR_INVALID, "NULL argument");
     if (which < AMB_MU_TOTAL || which > AMB_MU_ACTIVE) return fail(AMB_ERR_INVALID, "unknown chemical potential");
+    std::lock_guard<std::mutex> lock(h->reading);
     if (int rc = compute_terms(h)) return rc;
     const size_t n = h->n();
     const double* from = h->terms + (which == AMB_MU_ACTIVE ? n : 0);
@@ -646,6 +648,7 @@ extern "C" int amb_integrator_get_current(amb_integrator* h, int which, double* 
 {
     if (!h || !host_y || !host_x) return fail(AMB_ERR_INVALID, "NULL argument");
     if (which < AMB_CURRENT_TOTAL || which > AMB_CURRENT_RANDOM) return fail(AMB_ERR_INVALID, "unknown current");
+    std::lock_guard<std::mutex> lock(h->reading);
     if (int rc = compute_terms(h)) return rc;
     const size_t n = h->n();
     double* host[2] = {host_y, host_x};

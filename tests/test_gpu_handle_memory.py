@@ -1,5 +1,6 @@
-"""The C handle's getters: their sums, and what they hold on the device."""
+"""The C handle's getters: what they hold on the device, and several threads reading one handle."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -75,3 +76,24 @@ def test_getters_allocate_the_term_planes_only(precision):
     _potential(h, 0, shape)
     assert _used() - _current_before < 10.5 * plane
     N.lib().amb_integrator_destroy(h)
+
+
+def test_threads_read_one_handle():
+    """Getters of one state from several threads (every call its own arrays) give what one thread gets."""
+    shape, lib = (300, 400), N.lib()
+    h = _handle(np.random.default_rng(3).normal(-0.4, 0.1, shape), N.AMB_F64)
+    assert lib.amb_integrator_run(h, 2) == 0
+    want = [_current(h, w, shape) for w in range(7)]
+    bad = []
+
+    def work(w):
+        for _ in range(30):
+            if not np.array_equal(_current(h, w, shape), want[w]):
+                bad.append(w)
+    threads = [threading.Thread(target=work, args=(w,)) for w in range(7)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    lib.amb_integrator_destroy(h)
+    assert not bad
