@@ -404,9 +404,13 @@ class Integrator:
     # ------------------------------------------------------------- getters
     def _terms(self):
         """The ten FP64 term planes at the current timestep (device tensor), cached per timestep
-        like the reference's lazy current recompute (src/integrator.cu:477-495)."""
-        if self._terms_step != self._timestep:
-            torch = _torch()
+        like the reference's lazy current recompute (src/integrator.cu:477-495). They may be read on another
+        stream, or in another thread, than the one that queued them: that waits for them."""
+        torch = _torch()
+        stream = torch.cuda.current_stream(self._device)
+        if self._terms_step == self._timestep:
+            stream.wait_event(self._terms_done)
+        else:
             if self._terms_dev is None:
                 self._terms_dev = torch.empty((N.AMB_NTERMS, self._ny, self._nx), dtype=torch.float64,
                                               device=self._device)
@@ -414,7 +418,8 @@ class Integrator:
             fn = lib.amb_terms_f64 if self._precision == "f64" else lib.amb_terms_f32
             _check(fn(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
                       self._buf[self._cur].data_ptr(), self._timestep, None, self._terms_dev.data_ptr(),
-                      self._stream()))
+                      stream.cuda_stream))
+            self._terms_done = stream.record_event()
             self._terms_step = self._timestep
         return self._terms_dev
 
