@@ -4,12 +4,12 @@
 #include "amb_kernels.h"
 #include "amb_step_tile.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <vector>
 
 namespace
 {
@@ -415,8 +415,8 @@ struct amb_integrator
     void* buf[2] = {nullptr, nullptr};  // field ping-pong
     int cur = 0;
     uint16_t* residual = nullptr;
-    void* workspace = nullptr;  // step workspace, allocated at the first run if there is room
-    bool workspace_tried = false;
+    void* workspace = nullptr;  // step workspace where it is small, allocated at the first run
+    bool no_room = false;       // for a workspace: runs take the kernels that need none
     double* stage = nullptr;  // float64 staging plane for FP32 fields, allocated on first transfer
     double* terms = nullptr;  // AMB_NTERMS planes, allocated on first getter call
     int* flag = nullptr;
@@ -428,6 +428,114 @@ struct amb_integrator
 
 namespace
 {
+    // The largest workspace that a handle keeps. Larger ones (the planes of the FP64 step, four times the field) are
+    // leased for a run, which ends synchronised: idle ones, the latest eight of at most 256 MiB per device, wait for the
+    // next runs of any handle. An allocation that finds no room frees the idle ones first, and so does the
+    // last handle's end. (From a stream-ordered memory pool instead, ten steps of 2048^2 took 6060 us, 5946 so.)
+    constexpr size_t kKeptWorkspace = size_t(8) << 20, kIdleWorkspace = (size_t(256) << 20) + 4096;
+    constexpr int kDevices = 64, kIdle = 8;
+    struct Idle
+    {
+        void* p;
+        size_t bytes;
+    };
+    std::mutex g_idle_mutex;
+    Idle g_idle[kDevices][kIdle];
+    int g_handles = 0;
+
+    void free_idle()
+    {
+        std::lock_guard<std::mutex> lock(g_idle_mutex);
+        for (auto& device : g_idle)
+            for (Idle& i : device)
+            {
+                if (i.p) cudaFree(i.p);
+                i = Idle{};
+            }
+    }
+
+    template <typename T>
+    cudaError_t device_alloc(T** out, size_t bytes)
+    {
+        cudaError_t e = cudaMalloc(out, bytes);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        free_idle();
+        return cudaMalloc(out, bytes);
+    }
+
+    void count_handle(int by)
+    {
+        bool last;
+        {
+            std::lock_guard<std::mutex> lock(g_idle_mutex);
+            last = (g_handles += by) == 0;
+        }
+        if (last) free_idle();
+    }
+
+    // A workspace for the current device, given back at the end of the scope once the stream has drained.
+    struct Lease
+    {
+        void* p = nullptr;
+        size_t bytes = 0;
+        int dev = -1;
+        cudaStream_t stream;
+        explicit Lease(cudaStream_t s) : stream(s) {}
+        Lease(const Lease&) = delete;
+        Lease& operator=(const Lease&) = delete;
+        cudaError_t take(size_t need)
+        {
+            cudaError_t e = cudaGetDevice(&dev);
+            if (e != cudaSuccess) return e;
+            if (dev < kDevices)
+            {
+                std::lock_guard<std::mutex> lock(g_idle_mutex);
+                Idle* best = nullptr;  // the smallest that fits
+                for (Idle& i : g_idle[dev])
+                    if (i.p && i.bytes >= need && (!best || i.bytes < best->bytes)) best = &i;
+                if (best)
+                {
+                    p = best->p;
+                    bytes = best->bytes;
+                    *best = Idle{};
+                    return cudaSuccess;
+                }
+            }
+            bytes = need;
+            e = device_alloc(&p, need);
+            if (e != cudaSuccess) p = nullptr;
+            return e;
+        }
+        ~Lease()
+        {
+            if (!p) return;
+            cudaStreamSynchronize(stream);
+            if (dev >= kDevices || bytes > kIdleWorkspace)
+            {
+                cudaFree(p);
+                return;
+            }
+            // keep this one, at the expense of others where they are too many or too much
+            std::lock_guard<std::mutex> lock(g_idle_mutex);
+            Idle* slot = &g_idle[dev][0];
+            size_t held = bytes;
+            for (Idle& i : g_idle[dev])
+            {
+                held += i.bytes;
+                if (i.bytes < slot->bytes) slot = &i;
+            }
+            for (Idle& i : g_idle[dev])
+                if (i.p && (&i == slot || held > kIdleWorkspace))
+                {
+                    held -= i.bytes;
+                    cudaFree(i.p);
+                    i = Idle{};
+                }
+            *slot = Idle{p, bytes};
+        }
+    };
+
     void release(amb_integrator* h)
     {
         if (!h) return;
@@ -441,12 +549,13 @@ namespace
         cudaFree(h->flag);
         if (h->stream) cudaStreamDestroy(h->stream);
         delete h;
+        count_handle(-1);
     }
 
     cudaError_t ensure_stage(amb_integrator* h)
     {
         if (h->stage) return cudaSuccess;
-        return cudaMalloc(&h->stage, h->n() * sizeof(double));
+        return device_alloc(&h->stage, h->n() * sizeof(double));
     }
 
     // Host float64 -> device field (FP32 fields convert on the device).
@@ -474,7 +583,7 @@ namespace
         if (h->terms_timestep == h->timestep) return AMB_OK;
         if (!h->terms)
         {
-            cudaError_t e = cudaMalloc(&h->terms, h->n() * AMB_NTERMS * sizeof(double));
+            cudaError_t e = device_alloc(&h->terms, h->n() * AMB_NTERMS * sizeof(double));
             if (e != cudaSuccess) return fail(AMB_ERR_NOMEM, "terms buffer: " + std::string(cudaGetErrorString(e)));
         }
         int rc = h->precision == AMB_F64
@@ -520,6 +629,7 @@ extern "C" int amb_integrator_create(const double* host_field, int nrows, int nc
         return fail(AMB_ERR_INVALID, "precision must be AMB_F64, AMB_F32 or AMB_F32C");
     auto* h = new (std::nothrow) amb_integrator;
     if (!h) return fail(AMB_ERR_NOMEM, "host allocation failed");
+    count_handle(1);
     h->stencil = *stencil;
     h->model = *model;
     h->nrows = nrows;
@@ -527,9 +637,9 @@ extern "C" int amb_integrator_create(const double* host_field, int nrows, int nc
     h->precision = precision;
     h->seed = seed;
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&h->buf[i], h->n() * h->elem());
-    if (e == cudaSuccess && precision == AMB_F32C) e = cudaMalloc(&h->residual, h->n() * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->flag, sizeof(int));
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = device_alloc(&h->buf[i], h->n() * h->elem());
+    if (e == cudaSuccess && precision == AMB_F32C) e = device_alloc(&h->residual, h->n() * sizeof(uint16_t));
+    if (e == cudaSuccess) e = device_alloc(&h->flag, sizeof(int));
     if (e != cudaSuccess)
     {
         release(h);
@@ -550,32 +660,35 @@ extern "C" void amb_integrator_destroy(amb_integrator* h) { release(h); }
 extern "C" int amb_integrator_run(amb_integrator* h, int nsteps)
 {
     if (!h) return fail(AMB_ERR_INVALID, "NULL integrator");
+    Lease lease(h->stream);
     if (nsteps > 0)
     {
         int in_spare = 0;
         int rc;
         void* other = h->buf[1 - h->cur];
         const size_t ws_bytes = amb_step_workspace_bytes(h->precision, h->nrows, h->ncols);
-        if (ws_bytes && !h->workspace_tried)
+        if (!h->workspace && ws_bytes && !h->no_room)
         {
-            h->workspace_tried = true;
-            if (cudaMalloc(&h->workspace, ws_bytes) != cudaSuccess)
+            const bool keep = ws_bytes <= kKeptWorkspace;
+            if ((keep ? cudaMalloc(&h->workspace, ws_bytes) : lease.take(ws_bytes)) != cudaSuccess)
             {
-                h->workspace = nullptr;  // no room: the tile kernel needs none
+                if (keep) h->workspace = nullptr;
+                h->no_room = true;
                 cudaGetLastError();
             }
         }
-        if (h->precision == AMB_F64 && h->workspace)
+        void* ws = h->workspace ? h->workspace : lease.p;
+        if (h->precision == AMB_F64 && ws)
             rc = amb_step_f64_ws(&h->stencil, &h->model, h->seed, h->nrows, h->ncols,
                                  static_cast<double*>(h->buf[h->cur]), static_cast<double*>(other), h->timestep, nsteps,
-                                 nullptr, h->workspace, ws_bytes, h->stream, &in_spare);
+                                 nullptr, ws, ws_bytes, h->stream, &in_spare);
         else if (h->precision == AMB_F64)
             rc = amb_step_f64(&h->stencil, &h->model, h->seed, h->nrows, h->ncols, static_cast<double*>(h->buf[h->cur]),
                               static_cast<double*>(other), h->timestep, nsteps, nullptr, h->stream, &in_spare);
-        else if (h->workspace)
+        else if (ws)
             rc = amb_step_f32_ws(&h->stencil, &h->model, h->seed, h->nrows, h->ncols,
                                  static_cast<float*>(h->buf[h->cur]), static_cast<float*>(other), h->residual,
-                                 h->timestep, nsteps, nullptr, nullptr, h->workspace, ws_bytes, h->stream, &in_spare);
+                                 h->timestep, nsteps, nullptr, nullptr, ws, ws_bytes, h->stream, &in_spare);
         else
             rc = amb_step_f32(&h->stencil, &h->model, h->seed, h->nrows, h->ncols, static_cast<float*>(h->buf[h->cur]),
                               static_cast<float*>(other), h->residual, h->timestep, nsteps, nullptr, AMB_KERNEL_AUTO,

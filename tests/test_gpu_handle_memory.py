@@ -97,3 +97,54 @@ def test_threads_read_one_handle():
         t.join()
     lib.amb_integrator_destroy(h)
     assert not bad
+
+
+def test_runs_share_and_give_back_their_workspace():
+    """Four FP64 handles that have run hold their two planes each and one workspace of eight together; no handle, no
+    workspace."""
+    import torch
+    side = 2048
+    plane, field = side * side * 8, np.random.default_rng(4).normal(-0.4, 0.1, (side, side))
+    warm = _handle(field[:8, :8], N.AMB_F64)  # what the library holds with any handle
+    assert N.lib().amb_integrator_run(warm, 1) == 0
+    torch.cuda.empty_cache()
+    before = _used()
+    handles = [_handle(field, N.AMB_F64, seed=i) for i in range(4)]
+    for h in handles:
+        assert N.lib().amb_integrator_run(h, 2) == 0
+    assert _used() - before < (4 * 2 + 8 + 0.5) * plane
+    for h in handles + [warm]:
+        N.lib().amb_integrator_destroy(h)
+    assert _used() - before < 0.5 * plane
+
+
+def test_threads_run_handles_at_once():
+    """Handles of a size that leases its workspace, run by several threads: each the bits of a run alone."""
+    lib, shape, n = N.lib(), (700, 600), 4
+    rng = np.random.default_rng(5)
+    fields = [rng.normal(-0.4, 0.1, shape) for _ in range(n)]
+    out = []
+    for together in (True, False):
+        handles = [_handle(f, N.AMB_F64, seed=i) for i, f in enumerate(fields)]
+        rcs = []
+
+        def work(h):
+            for steps in (3, 1, 2, 5):
+                rcs.append(lib.amb_integrator_run(h, steps))
+        if together:
+            threads = [threading.Thread(target=work, args=(h,)) for h in handles]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+        else:
+            for h in handles:
+                work(h)
+        assert rcs == [0] * (4 * n)
+        out.append([])
+        for h in handles:
+            f = np.empty(shape)
+            assert lib.amb_integrator_get_field(h, f.ctypes.data) == 0
+            out[-1].append(f)
+            lib.amb_integrator_destroy(h)
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
