@@ -233,8 +233,8 @@ class Integrator:
         # 256 MiB: kept where small, else the bytes that each run takes and gives back; None: no room, tile kernel.
         self._workspace = None
         if precision != "f64" or kernel != "tile":
-            self._workspace = lib.amb_step_workspace_bytes(_PRECISIONS[precision], self._ny, self._nx)
-            if self._workspace <= _KEPT_WORKSPACE:
+            self._workspace = lib.amb_step_workspace_bytes(_PRECISIONS[precision], self._ny, self._nx) or None
+            if self._workspace is not None and self._workspace <= _KEPT_WORKSPACE:
                 self._workspace = self._lease()
         self._timestep = 0
         self._terms_step = None

@@ -208,10 +208,10 @@ extern "C" int amb_step_f64_ws(const amb_stencil* stencil, const amb_model* mode
     if (int rc = check_params(stencil, model)) return rc;
     if (!field || !spare || field == spare) return fail(AMB_ERR_INVALID, "field and spare must be distinct device buffers");
     if (nsteps < 0) return fail(AMB_ERR_INVALID, "nsteps must be >= 0");
-    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15)
-        || workspace_bytes < amb_step_workspace_bytes(AMB_F64, nrows, ncols))
+    const size_t need = amb_step_workspace_bytes(AMB_F64, nrows, ncols);
+    if (need && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15) || workspace_bytes < need))
         return fail(AMB_ERR_INVALID, "amb_step_f64_ws: workspace NULL, unaligned or smaller than amb_step_workspace_bytes");
-    if (nsteps == 0 || capturing(as_stream(stream)))
+    if (!need || nsteps == 0 || capturing(as_stream(stream)))
         return amb_step_f64(stencil, model, seed, nrows, ncols, field, spare, step0, nsteps, injected_noise, stream,
                             result_in_spare);
     const amb::StepParams p = make_params(stencil, model, seed, nrows, ncols, step0);

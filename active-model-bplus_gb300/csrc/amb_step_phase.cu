@@ -14,6 +14,9 @@ namespace amb
         // Largest planes workspace. A band of at most this many bytes keeps the recomputed rows of a
         // band boundary (16 of phase 1, 8 of phase 2) below 1 % of the band at 4096 columns.
         constexpr size_t kWorkspaceCap = size_t(256) << 20;
+        // A band has at least 48 rows, which for long rows are more than that; past this (700000 columns) the grid is
+        // left to the tile kernel.
+        constexpr size_t kWorkspaceMost = size_t(2) << 30;
         // Longest launch in seconds, and the steps that fit: a long run stays a queue of launches, between which
         // another stream's kernels find the SMs free (300000 steps of 64^2 in 180 launches: 6.0 us per step, as in
         // one). A step takes 6 us (tiles) or 12 us (phases) however small the grid, and 145 ps per site where the FP64
@@ -93,7 +96,8 @@ namespace amb
     size_t step_phase_workspace(int ny, int nx)
     {
         int band;
-        return workspace_bytes<double>(ny, nx, &band);
+        const size_t bytes = workspace_bytes<double>(ny, nx, &band);
+        return bytes <= kWorkspaceMost ? bytes : 0;
     }
 
     cudaError_t launch_steps_phase(double* a, double* b, const StepParams& p, int noise_mode, const double* injected,

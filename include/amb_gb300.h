@@ -174,8 +174,9 @@ int amb_step_f64_ex(const amb_stencil* stencil, const amb_model* model, uint64_t
  * (every step of the call in one cooperative launch, no FP64 operation recomputed in halos):
  * amb_step_workspace_bytes(AMB_F64, nrows, ncols) bytes of device memory, 16-byte aligned, whose
  * content need not be kept between calls but which calls that may overlap must not share. At most
- * 256 MiB (more only for rows of over 87000 columns). The results are bitwise those of
- * amb_step_f64. While the stream is being captured the call runs as amb_step_f64. */
+ * 256 MiB (up to 2 GiB for rows of over 87000 columns; 0, no workspace, where that is too little). The
+ * results are bitwise those of amb_step_f64. Without a workspace, and while the stream is being captured, the call
+ * runs as amb_step_f64. One launch takes at most some 10 ms of steps. */
 size_t amb_step_workspace_bytes(int precision, int nrows, int ncols);
 int amb_step_f64_ws(const amb_stencil* stencil, const amb_model* model, uint64_t seed, int nrows, int ncols,
                     double* field, double* spare, int64_t step0, int nsteps, const double* injected_noise,
