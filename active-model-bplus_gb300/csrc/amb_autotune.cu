@@ -7,8 +7,8 @@
 // kernel with 1, 2 or 4 pairs per CTA (or, fused, one single warp per CTA) and the row-segment
 // heights that put a whole number of tasks on each SM (plus the occupancy model's own choice). All candidates
 // give bitwise the same field. Each is timed with CUDA events over a few steps on
-// scratch buffers of the same shape; the fastest few are timed again and the best
-// is kept in a process-wide cache keyed by (device, nrows, ncols, compensated,
+// scratch buffers of the same shape; the fastest few are timed again and the best, or a nearly as fast one
+// that leaves more of the GPU to runs on other streams (kSparing), is kept in a process-wide cache keyed by (device, nrows, ncols, compensated,
 // noise), which AMB_KERNEL_AUTO consults. The kernels do the same work whatever the
 // field values, so zero-filled scratch fields time the real workload.
 #include "amb_gb300.h"
@@ -31,6 +31,12 @@ namespace
         amb_kernel_config config;
         double us_per_step;
     };
+    // A persistent launch on at most a quarter, or else half, of the GPU's threads is taken where it is at most this
+    // much slower than the fastest: runs of small grids on several streams then advance at once. us per step and run,
+    // one run and eight at once, f32c, T = 0.05: 128^2 3.0 and 0.85 (the fastest shape: 2.9 and 2.8), 64^2 2.95 and
+    // 0.47 (3.0 and 1.5), 256^2 3.7 and 2.1 (3.4 and 3.2); from 250 x 333 on no such shape comes near the fastest.
+    constexpr double kSparing = 1.08;
+
     std::map<Key, Entry> g_cache;
     std::mutex g_mutex;
 
@@ -124,6 +130,11 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
         for (int h : rows)
             for (int groups : {1, 2})
                 for (int flags : {0, AMB_FLAG_PERSISTENT}) cands.push_back({AMB_KERNEL_TILE, h, groups, flags | wide});
+        for (int part : {2, 4})  // on a half and a quarter of the SMs' threads
+        {
+            const int h = (nrows + std::max(1, 2 * sms / part / across) - 1) / std::max(1, 2 * sms / part / across);
+            if (h <= 64) cands.push_back({AMB_KERNEL_TILE, h, 1, AMB_FLAG_PERSISTENT | wide});
+        }
     }
     if (ncols >= 112 && ncols % 4 == 0)
     {
@@ -167,6 +178,14 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
 
     std::vector<std::pair<float, int>> times;
     int rc = AMB_OK;
+    std::pair<float, int> chosen{0.f, 0};
+    // How much of the GPU's threads (two CTAs of 256 per SM, by registers) a persistent launch holds on to.
+    const auto share = [&](const amb_kernel_config& c) {
+        if (c.kernel != AMB_KERNEL_TILE || !(c.flags & AMB_FLAG_PERSISTENT)) return 1.0;
+        const int cols = c.flags & AMB_FLAG_TILE_COLS_64 ? 64 : 32;
+        const double ctas = double((ncols + cols - 1) / cols) * ((nrows + c.seg_rows - 1) / c.seg_rows);
+        return std::min(1.0, ctas * c.pairs_per_cta / (2.0 * sms));
+    };
     for (size_t i = 0; i < cands.size() && rc == AMB_OK; ++i)
     {
         float ms = 0.f;
@@ -176,21 +195,47 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
     if (rc == AMB_OK)
     {
         std::sort(times.begin(), times.end());
-        // second round for the leaders: keep each one's faster time
-        const size_t lead = std::min<size_t>(4, times.size());
-        for (size_t j = 0; j < lead && rc == AMB_OK; ++j)
+        // second round for the leaders, over all and among those that leave half or three quarters of the GPU to
+        // others: keep each one's fastest time
+        std::vector<size_t> leaders;
+        for (double most : {1.0, 0.5, 0.25})
         {
-            float ms = 0.f;
-            rc = time_one(cands[times[j].second], &ms);
-            if (rc == AMB_OK) times[j].first = std::min(times[j].first, ms);
+            const size_t count = most == 1.0 ? 4 : 2;
+            for (size_t j = 0, taken = 0; j < times.size() && taken < count; ++j)
+                if (share(cands[times[j].second]) <= most)
+                {
+                    ++taken;
+                    if (std::find(leaders.begin(), leaders.end(), j) == leaders.end()) leaders.push_back(j);
+                }
         }
-        std::sort(times.begin(), times.begin() + lead);
+        for (int again = 0; again < 2; ++again)
+            for (size_t j : leaders)
+            {
+                float ms = 0.f;
+                if (rc == AMB_OK) rc = time_one(cands[times[j].second], &ms);
+                if (rc == AMB_OK) times[j].first = std::min(times[j].first, ms);
+            }
+        float fastest = times[leaders[0]].first;
+        for (size_t j : leaders) fastest = std::min(fastest, times[j].first);
+        const auto pick = [&](double most) {
+            const std::pair<float, int>* best = nullptr;
+            for (size_t j : leaders)
+                if (share(cands[times[j].second]) <= most && (!best || times[j].first < best->first)) best = &times[j];
+            return best;
+        };
+        for (double most : {0.25, 0.5, 1.0})
+        {
+            const auto* p = pick(most);
+            if (!p || p->first > kSparing * fastest) continue;
+            chosen = *p;
+            break;
+        }
     }
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     if (rc != AMB_OK) return rc;
-    *best = cands[times[0].second];
-    const double us = 1000.0 * times[0].first / probe_steps;
+    *best = cands[chosen.second];
+    const double us = 1000.0 * chosen.first / probe_steps;
     if (us_per_step) *us_per_step = us;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
