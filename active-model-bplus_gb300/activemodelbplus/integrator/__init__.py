@@ -409,7 +409,8 @@ class Integrator:
         torch = _torch()
         stream = torch.cuda.current_stream(self._device)
         if self._terms_step == self._timestep:
-            stream.wait_event(self._terms_done)
+            if stream != self._terms_stream:
+                self._terms_stream.synchronize()
         else:
             if self._terms_dev is None:
                 self._terms_dev = torch.empty((N.AMB_NTERMS, self._ny, self._nx), dtype=torch.float64,
@@ -419,7 +420,7 @@ class Integrator:
             _check(fn(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
                       self._buf[self._cur].data_ptr(), self._timestep, None, self._terms_dev.data_ptr(),
                       stream.cuda_stream))
-            self._terms_done = stream.record_event()
+            self._terms_stream = stream
             self._terms_step = self._timestep
         return self._terms_dev
 
