@@ -185,11 +185,12 @@ class Integrator:
         seed: 64-bit key of the Philox noise; ``None`` draws one from the OS,
             like the reference's non-deterministic seed.
         device: CUDA device (default: current).
-        kernel: "auto", "tile" or "sliding" (FP32 kernel choice; FP64 runs the three-phase kernel, or
-            the tile kernel with kernel="tile" or where its workspace does not fit).
+        kernel: "auto", "tile" or "sliding" (FP32 kernel choice; FP64 runs the three-phase kernel, on small
+            grids the one-tile-per-SM kernel, or the tile kernel with kernel="tile" or where the workspace, which
+            a run takes from torch's allocator and gives back, does not fit).
         autotune: with kernel="auto" and FP32 storage, time the candidate kernels and
             launch shapes for this grid once per process (``amb_autotune_f32``) and use
-            the fastest; otherwise a shape heuristic decides. The FP32 kernels give
+            the fastest, or one within 8 % of it that leaves half the GPU to others; otherwise a shape heuristic decides. The FP32 kernels give
             bitwise equal fields (the same arithmetic at every site), so the choice
             changes the time, never the result.
         launch: explicit launch shape: for kernel="sliding" (FP32 storage) {"seg_rows": h,

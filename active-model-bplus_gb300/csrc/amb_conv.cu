@@ -47,10 +47,10 @@
 // error over the largest gradient, values of mean 0.5, 32 x 32 channels, chains of 4 / 8 / 16 blocks / all blocks of
 // the CTA: 16 x 128^2 sites 0.6e-6 / 1.1e-6 / 2.0e-6 / 2.4e-6, 16 x 512^2 0.7e-6 / 1.2e-6 / 2.2e-6 / 45e-6 (partials of
 // eight rows, before the CTAs were persistent: 1.7e-6 and 3.9e-6).
-// Measured for 16 x 128^2 sites, 32 x 32 channels, with the reduction: 32.8 us (one chain 33.0; one 128 x 32
-// instruction per tap, 256 partials: 107); 16 x 512^2: 520 us (one chain 513). 9 us of the 32.8 are instructions, the
-// rest the copies, which the copy engine takes one by one (dZ rows that follow one another in memory go as
-// one), and the epilogue.
+// Measured for 16 x 128^2 sites, 32 x 32 channels: 26.7 us and 3.6 us for the reduction (one chain 26.0; one
+// 128 x 32 instruction per tap, 256 partials: 80 and 17); 16 x 512^2, both: 520 us (one chain 513). 9 us of the 26.7 are
+// instructions, the rest the copies, which the copy engine takes one by one (dZ rows that follow one another
+// in memory go as one), and the epilogue.
 #include "amb_gb300.h"
 #include "amb_kernels.h"
 #include "amb_tc.cuh"
@@ -1278,7 +1278,7 @@ namespace
 
     // The same on four columns per thread, for rows of whole aligned 16-byte quads and no per-site noise: a quarter of
     // the threads, 13 faces instead of 16 and wide accesses (a macro step at
-    // 512^2: 82.6 -> 80.0 us, at 768^2 156.4 -> 147.7).
+    // 512^2: 82.6 -> 79.2 us, at 768^2 156.4 -> 147.7).
     __global__ void learned_update_quad_kernel(const float* __restrict__ flux, const float* __restrict__ extra, int nrows,
                                                int ncols, float scale_y, float scale_x, int32_t* __restrict__ phi_q,
                                                float* __restrict__ phi_f, long long bound, int* __restrict__ flag,

@@ -1,4 +1,4 @@
-// FP64 steps of small grids: one tile per SM, all steps of a call in one cooperative launch.
+// FP64 steps of small grids: one tile per SM, many steps in one cooperative launch.
 //
 // The three-phase kernel (amb_step_phase.cuh) executes the fewest FP64 operations, but each of its
 // phases ends in a grid barrier and starts with L2 latency, about 4 us whatever the grid. Here a CTA
@@ -9,8 +9,8 @@
 // div J side by side. An item is a column and a run of rows whose row sums are carried. The noise is
 // drawn into the arrays that J1 replaces, for the next step while the barrier completes.
 //
-// us per step at T = 0.05, this kernel and the three-phase kernel: 64^2 6.1 (12.5), 48 x 100 6.7 (12.7),
-// 128^2 9.0 (13.2), 200 x 300 18.5 (20.1).
+// us per step at T = 0.05, this kernel and the three-phase kernel: 64^2 6.0 (12.5), 48 x 100 7.2 (12.7),
+// 128^2 9.3 (13.2), 200 x 300 18.4 (20.1).
 #pragma once
 
 #include "amb_step_phase.cuh"
@@ -20,10 +20,11 @@ namespace amb
     namespace dtile
     {
         // Threads per CTA. 512 for the lowest time of one run. A CTA of 256 leaves half an SM's registers to a CTA of
-        // another run, so that runs on several streams share the GPU, at the same time for one run where a tile has
-        // few sites. us per step of one run, and per step and run with 8 at once: 64^2 6.65 and 3.7 (512: 6.69 and
-        // 6.1), 128^2 9.8 and 6.9 (9.5 and 9.0), 200^2 16.8 and 12.9 (15.0 and 14.5). One launch per step of the tile
-        // kernel: 64^2 and 128^2 47.7 and 6.4, 200^2 47.7 and 13.7.
+        // another run, so that runs on several streams share the GPU, where a tile's lists are short enough for
+        // eight warps. us per step of one run, and per step and run with eight at once, 256 threads (512; one launch
+        // per step of the tile kernel): 64^2 6.0 and 3.7 (6.0 and 6.1; 47.7 and 6.4), 96^2 7.5 and 4.9 (7.1 and 7.1;
+        // 47.7 and 6.3), 128^2 9.3 and 6.9 (8.9 and 9.0; 47.7 and 6.4), 200^2 16.6 and 12.9 (14.5 and 14.5; 47.7 and
+        // 13.7). 512 threads on 64 registers each, two CTAs per SM: 128^2 9.4 and 7.3, 64^2 6.6 and 4.2.
         constexpr int kThreads = 512, kThreadsSmall = 256;
         constexpr double kSitesSmall = 110;  // most sites per SM for the small CTA
 

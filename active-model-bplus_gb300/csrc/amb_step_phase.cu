@@ -67,9 +67,9 @@ namespace amb
                    + list(tx, ty, 3, 0);
         }
 
-        // The tile shape that spreads a grid over the SMs, one tile each, at the least cost (64^2: 4 x 8, 6.1 us;
+        // The tile shape that spreads a grid over the SMs, one tile each, at the least cost (64^2: 4 x 8, 6.0 us;
         // 1 x 64 12.3). False above 400 sites per SM, where the halo costs more than two grid barriers (us per
-        // step, tiles and phases: 128^2 9.0 and 13.2, 200 x 300 18.5 and 20.1, 256^2 19.9 and 20.0, 350^2 35.8
+        // step, tiles and phases: 128^2 9.3 and 13.2, 200 x 300 18.4 and 20.1, 256^2 19.9 and 20.0, 350^2 35.8
         // and 29.5).
         bool tile_shape(int ny, int nx, int sms, dtile::Shape* best, int* threads)
         {

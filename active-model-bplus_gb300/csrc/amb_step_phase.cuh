@@ -1,4 +1,4 @@
-// Explicit-Euler step in three grid-wide phases, all steps of a call in one cooperative launch.
+// Explicit-Euler step in three grid-wide phases, many steps in one cooperative launch.
 //
 // The FP64 pipe is what binds the FP64 step on sm_103a: one warp instruction per 64 cycles and SM
 // sub-partition (2 lanes per clock and SM), issued back to back by a single warp, at the same cost
@@ -16,10 +16,10 @@
 // Work split: one warp marches down a run of rows of a 32-column block, keeping the row sums (and,
 // for the y derivatives, a ring of rows) in registers. The rows of all blocks form one list that is
 // cut evenly over all warps of the grid, so every sub-partition gets the same share to within one
-// row: a 64^2 grid occupies 128 SMs, where 32 x 32 tiles occupied 4.
+// row (grids too small for that run as one tile per SM, amb_step_dtile.cuh).
 //
-// Measured, us per step at T = 0.05 (tile kernel before): 64^2 12.5 (47.7), 256^2 20.0 (47.8),
-// 701 x 907 103 (222), 2048^2 598 (1177), 4096^2 2418 (4673), the last 6.9 Gsite/s or 88 % of the
+// Measured, us per step at T = 0.05 (tile kernel before): 256^2 19.9 (47.8), 350^2 30.0 (48.7), 512^2 52.5 (94.5),
+// 701 x 907 102 (222), 2048^2 597 (1177), 4096^2 2415 (4673), the last 6.9 Gsite/s or 88 % of the
 // FP64 pipe for the 80 operations. Small grids are bound by the three barriers and the L2 latency
 // behind each.
 //

@@ -11,9 +11,9 @@
 // block barriers, between stages of a few hundred issue slots. One tile per SM whose height makes the
 // tile count match the SMs is therefore best where it fits (256^2: 7 or 14 rows, 3.4 us per step;
 // two or three tiles per SM 4.8 and 6.6), several CTAs of 256 threads otherwise. us per step, f32c,
-// T = 0.05, autotuned, this kernel and the one-column-per-thread tile kernel before it: 256^2 3.4 (6.3),
-// 512^2 5.9 (8.7), 768^2 9.2 (15.4), 1024^2 16.2 (24.6), 250 x 333 4.6 (6.7); from 1536^2 on the sliding
-// kernel, with less halo work, is the faster (28.8 there).
+// T = 0.05, autotuned, this kernel and the one-column-per-thread tile kernel before it: 256^2 3.5 (6.3; 3.4 on
+// all SMs' threads), 512^2 5.8 (8.7), 768^2 9.1 (15.4), 1024^2 16.3 (24.6), 250 x 333 4.5 (6.7); from 1536^2 on the
+// sliding kernel, with less halo work, is the faster (28.7 there).
 //
 // The noise of a step depends on no field, so it is drawn into the arrays that J1 later replaces:
 // before the tile's halo has arrived, and in the persistent form while the grid barrier completes.

@@ -171,7 +171,7 @@ int amb_step_f64_ex(const amb_stencil* stencil, const amb_model* model, uint64_t
                     double* field, double* spare, int64_t step0, int nsteps, const double* injected_noise,
                     const amb_kernel_config* config, void* stream, int* result_in_spare);
 /* amb_step_f64 with a workspace for the planes of the three-phase kernel, the fastest FP64 form
- * (every step of the call in one cooperative launch, no FP64 operation recomputed in halos):
+ * (many steps in one cooperative launch, no FP64 operation recomputed in halos):
  * amb_step_workspace_bytes(AMB_F64, nrows, ncols) bytes of device memory, 16-byte aligned, whose
  * content need not be kept between calls but which calls that may overlap must not share. At most
  * 256 MiB (up to 2 GiB for rows of over 87000 columns; 0, no workspace, where that is too little). The
