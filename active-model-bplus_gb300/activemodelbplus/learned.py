@@ -221,19 +221,24 @@ class FluxNet:
             self._dimages = [None] + [dgrad_image(self.weights[l], self.cin[l], self.npad[l])
                                       for l in range(1, self.nlayers)]
             return
+        # of the shapes that the weights have now: narrower ones are padded with zeros, wider ones refused
+        ws = [w.detach().to(torch.float32).contiguous() for w in self.weights]
+        if any(w.ndim != 4 or tuple(w.shape[2:]) != (5, 5) for w in ws):
+            raise ValueError("weights must have shape [cout, cin, 5, 5]")
         # one kernel builds all images, in a buffer of their own (a captured macro step keeps reading the
         # images that it was captured with)
         L = self.nlayers
         sizes = [25 * self.cin[l] * self.npad[l] for l in range(L)]
         buf = torch.empty(2 * sum(sizes), dtype=torch.bfloat16, device=self.weights[0].device)
-        self._images, self._dimages, at = [], [], 0
+        images, dimages, at = [], [], 0
         for l, n in enumerate(sizes):
-            self._images.append(buf[at:at + n])
-            self._dimages.append(buf[at + n:at + 2 * n] if l else None)
+            images.append(buf[at:at + n])
+            dimages.append(buf[at + n:at + 2 * n] if l else None)
             at += 2 * n
-        ws = [w.detach().to(torch.float32).contiguous() for w in self.weights]
-        _check(N.lib().amb_conv5x5_stack_images(L, _ptrs(ws), _ints(self.cout), _ints(self.cin_used), _ints(self.cin),
-                                                _ints(self.npad), _ptrs(self._images), _ptrs(self._dimages), _stream()))
+        _check(N.lib().amb_conv5x5_stack_images(L, _ptrs(ws), _ints([w.shape[0] for w in ws]),
+                                                _ints([w.shape[1] for w in ws]), _ints(self.cin), _ints(self.npad),
+                                                _ptrs(images), _ptrs(dimages), _stream()))
+        self._images, self._dimages = images, dimages
 
     def state_dict(self) -> dict:
         d = {}
