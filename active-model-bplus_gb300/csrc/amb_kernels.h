@@ -22,7 +22,7 @@ namespace amb
                                              cudaStream_t stream);
 
     // FP32 steps of the quad tile kernel (amb_step_quad.cuh): one launch per step, or, with a barrier
-    // counter (one word of device memory), one cooperative launch. The result is in a when nsteps is even.
+    // counter (one word of device memory), cooperative launches of up to 10 ms. The result is in a when nsteps is even.
     struct QuadTile
     {
         int rows;      // output rows of a tile, 1 .. 64

@@ -1,8 +1,9 @@
-// Launchers of the FP32 quad tile kernel (amb_step_quad.cuh): one launch per step, or one
-// cooperative launch for all steps of a call.
+// Launchers of the FP32 quad tile kernel (amb_step_quad.cuh): one launch per step, or cooperative
+// launches of many steps.
 #include "amb_kernels.h"
 #include "amb_step_quad.cuh"
 
+#include <algorithm>
 #include <mutex>
 
 namespace amb
@@ -96,11 +97,16 @@ namespace amb
             return comp ? by_threads<32, COMP_BF16>(tile.threads, in, out, comp, l, step, inj, n, persistent, count, stream)
                         : by_threads<32, COMP_NONE>(tile.threads, in, out, comp, l, step, inj, n, persistent, count, stream);
         };
-        if (persistent) return go(a, b, p.step, injected, nsteps);
-        for (int s = 0; s < nsteps; ++s)
+        // A persistent launch takes at most some 10 ms of steps, so that a long run stays a queue of launches, between
+        // which other streams' kernels that need whole SMs get their turn. A step takes 2.5 us however small the grid,
+        // and 15.5 ps per site (1024^2).
+        const double step_seconds = std::max(2.5e-6, double(p.ny) * p.nx * 15.5e-12);
+        const int most = persistent ? int(std::max(1.0, 0.01 / step_seconds)) : 1;
+        for (int s = 0, n; s < nsteps; s += n)
         {
+            n = std::min(most, nsteps - s);
             const float* inj = injected ? injected + size_t(s) * 2 * p.ny * p.nx : nullptr;
-            cudaError_t e = go(s & 1 ? b : a, s & 1 ? a : b, p.step + s, inj, 1);
+            cudaError_t e = go(s & 1 ? b : a, s & 1 ? a : b, p.step + s, inj, n);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;

@@ -85,7 +85,8 @@ typedef struct amb_model
  *   kernel (1 to 64, more runs as 64; 0: 32, or 28 with AMB_FLAG_TILE_ROWS_28); not used by the FP64 tile kernel.
  * pairs_per_cta: sliding kernel: warp pairs per CTA (1, 2 or 4); tile kernel: groups of 256
  *   threads per CTA (1, 2 or 4; FP32: 4 runs as 2).
- * flags: AMB_FLAG_PERSISTENT (tile kernel): all nsteps of the call in one cooperative launch,
+ * flags: AMB_FLAG_PERSISTENT (tile kernel): all nsteps of the call in one cooperative launch (FP32:
+ *   launches of up to some 10 ms, so that other streams' kernels get their turn),
  *   a grid-wide barrier between the steps (for grids too small to fill the GPU, where a launch
  *   per step costs more than the step; ignored while the stream is being captured). The
  *   results are bitwise those of one launch per step.

@@ -71,3 +71,48 @@ def test_a_long_run_lets_others_through():
     total = time.perf_counter() - begin
     assert total > 1.0  # the long run was under way
     assert wait < 0.5, (wait, total)
+
+
+@pytest.mark.parametrize("shape,steps", [((810, 810), 2050), ((16, 20), 8100)])
+def test_same_bits_of_persistent_fp32_launches(shape, steps):
+    """Three launches of 983 (odd: the buffers swap) and of 4000 steps against one launch per step."""
+    st, m = Stencil(1e-3, 1, 1), Model(-0.25, 0, 0.25, 1, -1, -4, 0.05)
+    f = np.random.default_rng(6).normal(-0.4, 0.1, shape)
+    fields = []
+    for persistent in (True, False):
+        sim = Integrator(f, st, m, seed=4, precision="f32c", kernel="tile", launch={"persistent": persistent, "pairs_per_cta": 1})
+        sim.run(steps)
+        fields.append(sim.field)
+    assert np.array_equal(*fields)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32c"])
+def test_a_long_fp32_run_lets_others_through(precision):
+    """Ten steps of a 512^2 grid, whose CTAs fill the SMs, issued during a run of 600000 steps of a 64^2 FP32 grid
+    (almost two seconds) on another stream: done within half a second."""
+    import torch
+    st, m = Stencil(1e-3, 1, 1), Model(-0.25, 0, 0.25, 1, -1, -4, 0.05)
+    rng = np.random.default_rng(3)
+    long_ = Integrator(rng.normal(-0.4, 0.1, (64, 64)), st, m, seed=1, precision="f32c")
+    short = Integrator(rng.normal(-0.4, 0.1, (512, 512)), st, m, seed=1, precision=precision)
+    sl, ss = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(ss):
+        short.run(10)
+    long_.run(10)
+    torch.cuda.synchronize()
+
+    def work():
+        with torch.cuda.stream(sl):
+            long_.run(600000)
+    t = threading.Thread(target=work)
+    begin = time.perf_counter()
+    t.start()
+    time.sleep(0.1)
+    t0 = time.perf_counter()
+    with torch.cuda.stream(ss):
+        short.run(10)
+    wait = time.perf_counter() - t0
+    t.join()
+    total = time.perf_counter() - begin
+    assert total > 1.0  # the long run was under way
+    assert wait < 0.5, (wait, total)
