@@ -202,13 +202,15 @@ extern "C" int amb_autotune_f32(const amb_stencil* stencil, const amb_model* mod
         {
             const size_t count = most == 1.0 ? 4 : 2;
             for (size_t j = 0, taken = 0; j < times.size() && taken < count; ++j)
-                if (share(cands[times[j].second]) <= most)
+                if (times[j].first > 1.25f * times[0].first) break;  // out of reach, whatever the timing's noise
+                else if (share(cands[times[j].second]) <= most)
                 {
                     ++taken;
                     if (std::find(leaders.begin(), leaders.end(), j) == leaders.end()) leaders.push_back(j);
                 }
         }
-        for (int again = 0; again < 2; ++again)
+        const bool sparing = share(cands[times[leaders.back()].second]) <= 0.5;  // then twice: the choice is close
+        for (int again = 0; again < (sparing ? 2 : 1); ++again)
             for (size_t j : leaders)
             {
                 float ms = 0.f;
