@@ -163,8 +163,8 @@ def _random_seed() -> int:
     return int.from_bytes(os.urandom(8), "little")
 
 
-# Largest workspace that an FP64 integrator keeps between runs (362^2): a lease costs some 5 us per run.
-_KEPT_WORKSPACE = 8 << 20
+# Largest workspace that an FP64 integrator keeps between runs (724^2): a lease costs some 5 us per run.
+_KEPT_WORKSPACE = 32 << 20
 
 
 # Term planes (of the y component) that a current is the sum of, in the reference's order.

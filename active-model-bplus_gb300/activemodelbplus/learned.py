@@ -223,7 +223,8 @@ class FluxNet:
             return
         # of the shapes that the weights have now: narrower ones are padded with zeros, wider ones refused
         ws = [w.detach().to(torch.float32).contiguous() for w in self.weights]
-        if any(w.ndim != 4 or tuple(w.shape[2:]) != (5, 5) for w in ws):
+        shapes = [tuple(w.shape) for w in ws]
+        if any(len(s) != 4 or s[2:] != (5, 5) for s in shapes):
             raise ValueError("weights must have shape [cout, cin, 5, 5]")
         # one kernel builds all images, in a buffer of their own (a captured macro step keeps reading the
         # images that it was captured with)
@@ -235,9 +236,9 @@ class FluxNet:
             images.append(buf[at:at + n])
             dimages.append(buf[at + n:at + 2 * n] if l else None)
             at += 2 * n
-        _check(N.lib().amb_conv5x5_stack_images(L, _ptrs(ws), _ints([w.shape[0] for w in ws]),
-                                                _ints([w.shape[1] for w in ws]), _ints(self.cin), _ints(self.npad),
-                                                _ptrs(images), _ptrs(dimages), _stream()))
+        _check(N.lib().amb_conv5x5_stack_images(L, _ptrs(ws), _ints([s[0] for s in shapes]), _ints([s[1] for s in shapes]),
+                                                _ints(self.cin), _ints(self.npad), _ptrs(images), _ptrs(dimages),
+                                                _stream()))
         self._images, self._dimages = images, dimages
 
     def state_dict(self) -> dict:

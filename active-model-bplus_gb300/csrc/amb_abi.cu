@@ -432,7 +432,7 @@ namespace
     // leased for a run, which ends synchronised: idle ones, the latest eight of at most 256 MiB per device, wait for the
     // next runs of any handle. An allocation that finds no room frees the idle ones first, and so does the
     // last handle's end. (From a stream-ordered memory pool instead, ten steps of 2048^2 took 6060 us, 5946 so.)
-    constexpr size_t kKeptWorkspace = size_t(8) << 20, kIdleWorkspace = (size_t(256) << 20) + 4096;
+    constexpr size_t kKeptWorkspace = size_t(32) << 20, kIdleWorkspace = (size_t(256) << 20) + 4096;
     constexpr int kDevices = 64, kIdle = 8;
     struct Idle
     {

@@ -120,7 +120,7 @@ def test_runs_share_and_give_back_their_workspace():
 
 def test_threads_run_handles_at_once():
     """Handles of a size that leases its workspace, run by several threads: each the bits of a run alone."""
-    lib, shape, n = N.lib(), (700, 600), 4
+    lib, shape, n = N.lib(), (900, 800), 4
     rng = np.random.default_rng(5)
     fields = [rng.normal(-0.4, 0.1, shape) for _ in range(n)]
     out = []
