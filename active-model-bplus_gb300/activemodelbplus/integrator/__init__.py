@@ -403,16 +403,16 @@ class Integrator:
         self._raise_if_flagged()
 
     # ------------------------------------------------------------- getters
-    def _terms(self):
+    def _terms(self, stream: int | None = None):
         """The ten FP64 term planes at the current timestep (device tensor), cached per timestep
         like the reference's lazy current recompute (src/integrator.cu:477-495). They may be read on another
         stream, or in another thread, than the one that queued them: that waits for them."""
-        torch = _torch()
-        stream = torch.cuda.current_stream(self._device)
+        stream = self._stream() if stream is None else stream
         if self._terms_step == self._timestep:
-            if stream != self._terms_stream:
+            if stream != self._terms_stream.cuda_stream:
                 self._terms_stream.synchronize()
         else:
+            torch = _torch()
             if self._terms_dev is None:
                 self._terms_dev = torch.empty((N.AMB_NTERMS, self._ny, self._nx), dtype=torch.float64,
                                               device=self._device)
@@ -420,21 +420,22 @@ class Integrator:
             fn = lib.amb_terms_f64 if self._precision == "f64" else lib.amb_terms_f32
             _check(fn(ctypes.byref(self._s), ctypes.byref(self._m), self._seed, self._ny, self._nx,
                       self._buf[self._cur].data_ptr(), self._timestep, None, self._terms_dev.data_ptr(),
-                      stream.cuda_stream))
-            self._terms_stream = stream
+                      stream))
+            self._terms_stream = torch.cuda.current_stream(self._device)
             self._terms_step = self._timestep
         return self._terms_dev
 
     def _current(self, which: str):
         """Fresh host copies of both components, summed on the device in the reference's order
         (src/integrator.cu:406-465)."""
-        terms = self._terms()
+        stream = self._stream()
+        terms = self._terms(stream)
         try:
             out = _torch().empty((2, self._ny, self._nx), dtype=terms.dtype, device=terms.device)
         except _torch().cuda.OutOfMemoryError:
             return [self._sum_on_host([terms[k + c] for k in _CURRENT_TERMS[which]]) for c in range(2)]
         _check(N.lib().amb_current_from_terms(terms.data_ptr(), self._ny, self._nx, N.CURRENTS[which], out.data_ptr(),
-                                              self._stream()))
+                                              stream))
         return [v.cpu().numpy() for v in out]
 
     @staticmethod
